@@ -403,7 +403,10 @@ __device__ __forceinline__ double llh_poisson(double data, double pred) {
   return 2.0 * (pred - data + data * log(data / pred));
 }
 
-__device__ __forceinline__ double llh_bb_oa2021(double data, double pred, double mcuncert) {
+// log(data) as the Barlow-Beeston term uses it (bins with data only).
+__device__ __forceinline__ double log_data_of(double data) { return data > DBL_EPSILON ? log(data) : 0.0; }
+
+__device__ __forceinline__ double llh_bb_oa2021(double data, double log_data, double pred, double mcuncert) {
   // BarlowBeestonBanff2022.h:150-294 with its defaults (expectedValueMinimum
   // = -1, fractionalErrorLimit = 1e150, usePoissonLikelihood = false).
   if (pred <= -1.0) {
@@ -425,10 +428,10 @@ __device__ __forceinline__ double llh_bb_oa2021(double data, double pred, double
   if (data <= DBL_EPSILON) {
     stat = newmc;
   } else if (newmc > DBL_MIN) {
-    stat = newmc - data + data * (log(data) - log(newmc));
+    stat = newmc - data + data * (log_data - log(newmc));
   } else {
     const double mc = DBL_MIN;
-    stat = mc - data + data * (log(data) - log(mc));
+    stat = mc - data + data * (log_data - log(mc));
   }
   return 2.0 * stat + 2.0 * penalty;
 }
@@ -437,11 +440,11 @@ __device__ __forceinline__ double llh_bb_oa2021(double data, double pred, double
 // as BarlowBeestonBanff2022::eval(const SamplePair&, int) takes it
 // (BarlowBeestonBanff2022.h:92-148): the stored sqrt squared again, and +inf
 // for a non-finite value (the reference's throwIfInfLlh = false branch).
-__device__ __forceinline__ double llh_bb_bin(double data, double pred, double sqrt_sum_w2) {
+__device__ __forceinline__ double llh_bb_bin(double data, double log_data, double pred, double sqrt_sum_w2) {
   double mcuncert = sqrt_sum_w2;
   mcuncert *= mcuncert;
   if (!isfinite(mcuncert) || mcuncert < 0.0) return HUGE_VAL;
-  return llh_bb_oa2021(data, pred, mcuncert);
+  return llh_bb_oa2021(data, log_data, pred, mcuncert);
 }
 
 }  // namespace

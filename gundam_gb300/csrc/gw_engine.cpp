@@ -506,6 +506,7 @@ extern "C" int gw_set_data(gw_engine* e, const double* data, int32_t n_bins) {
     if (rc) return rc;
     GW_CUDA(e, cudaMemcpyAsync((void*)e->view.data, data, sizeof(double) * (size_t)n_bins, cudaMemcpyHostToDevice,
                                e->stream));
+    GW_CUDA(e, launch_log_data(e->view, e->stream));
     GW_CUDA(e, cudaStreamSynchronize(e->stream));
   }
   return GW_OK;
@@ -1264,6 +1265,9 @@ int build_and_upload(gw_engine* e) {
   }
   if ((rc = upload(e->data.data(), sizeof(double) * B, &p))) return rc;
   v.data = (const double*)p;
+  if ((rc = alloc(sizeof(double) * B, &p))) return rc;
+  v.log_data = (double*)p;
+  GW_CUDA(e, launch_log_data(v, nullptr));  // the stream of the uploads
   // tables
   {
     std::vector<TableDesc> td(e->tables.size());
@@ -1337,13 +1341,12 @@ int build_and_upload(gw_engine* e) {
   if ((rc = alloc((size_t)P * kpad * tsz, &p))) return rc;
   GW_CUDA(e, cudaMemset(p, 0, (size_t)P * kpad * tsz));
   v.x = p;
-  if ((rc = alloc(sizeof(double) * kpad, &p))) return rc;
-  GW_CUDA(e, cudaMemset(p, 0, sizeof(double) * kpad));
+  v.n_pen = e->has_prior ? (P + kPenRows - 1) / kPenRows : 0;
+  if ((rc = alloc(sizeof(double) * (size_t)v.n_pen * kpad, &p))) return rc;
   v.penalty = (double*)p;
   if ((rc = alloc(sizeof(double2) * (size_t)std::max(e->n_slots, 1) * kpad, &p))) return rc;
   v.partials = (double2*)p;
-  v.llh_nblk = (B + 255) / 256;
-  if ((rc = alloc(sizeof(double) * (size_t)kpad * v.llh_nblk, &p))) return rc;
+  if ((rc = alloc(sizeof(double) * (size_t)kpad * ((B + kLlhBins - 1) / kLlhBins), &p))) return rc;
   v.llh_blocks = (double*)p;
   if ((rc = alloc(sizeof(unsigned int) * kpad, &p))) return rc;
   GW_CUDA(e, cudaMemset(p, 0, sizeof(unsigned int) * kpad));

@@ -56,6 +56,7 @@ struct DevView {
   const int64_t* eig_off;
   const double* eig_V;
   const double* data;         // [n_bins]
+  double* log_data;           // [n_bins] log of the data (0 in bins without), see launch_log_data
   const TableDesc* tables;
   const TableFn* table_fns;
   const double* table_nodes;
@@ -66,11 +67,11 @@ struct DevView {
   void* grid_pts;             // GridPoint<T>[n_grids * kpad], formed by k_params
 
   void* x;                    // T[n_params * kpad], mirrored parameter values
-  double* penalty;            // [kpad]
+  int n_pen;                  // row blocks of the prior penalty (0: no prior)
+  double* penalty;            // [n_pen * kpad] parts of delta^T C^-1 delta, one row of points per block
   double2* partials;          // [n_slots * kpad]  (scratch)
-  double* llh_blocks;         // [kpad * llh_nblk] (scratch)
+  double* llh_blocks;         // [ceil(n_bins / kLlhBins) * kpad] (scratch)
   unsigned int* llh_counter;  // [kpad]           (scratch)
-  int llh_nblk;
   double* event_weights;      // [n_events] in result order, or nullptr
   uint32_t* status;
 };
@@ -111,6 +112,7 @@ cudaError_t launch_batched(const DevView& v, int K, const BatchedShape& b, int g
 // True when every pass of the shape over K points stays inside the kpad
 // columns of the parameter and partial-sum arrays.
 bool batched_shape_covers(const DevView& v, const BatchedShape& b, int K);
+cudaError_t launch_log_data(const DevView& v, cudaStream_t s);  // after every change of the data
 cudaError_t launch_bins_llh(const DevView& v, int K, double* sums, double* sums2, double* llh,
                             double* llh_stat, cudaStream_t s);
 
@@ -121,5 +123,7 @@ int plain_blocks_per_sm(const DevView& v);
 int batched_blocks_per_sm(const DevView& v, const BatchedShape& b);
 
 constexpr int kPlainThreads = 256;
+constexpr int kPenRows = 8;  // rows of C^-1 per penalty block of k_params
+constexpr int kLlhBins = 8;  // bins of k_bins_llh's smallest block
 
 }  // namespace gw

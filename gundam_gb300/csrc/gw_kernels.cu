@@ -26,11 +26,51 @@ namespace {
 // ---------------------------------------------------------------------------
 // Parameter update: mirror into the dial inputs, prior penalty.
 // ---------------------------------------------------------------------------
+// Grid (K, 1 + n_pen): block (k, 0) mirrors the parameters of point k and forms
+// its knot-grid intervals; block (k, 1 + q) forms the part of the penalty
+// delta^T C^-1 delta that rows [q, q + 1) * kPenRows of C^-1 give.
+//
+// The penalty is P^2 FP64 multiply-adds per point, and an SM issues two of them
+// per cycle: as one block (one thread per row, rows read with a stride of P)
+// it took 38 us at P = 200, a sixth of a K = 1 evaluation of 1M events.  Cut
+// over blocks of kPenRows rows, thread p taking column p (coalesced), the
+// launch takes 6.8 us at K = 1 and 15 us at K = 64.  The parts are added in
+// a fixed order by k_bins_llh.
 template <typename T>
 __global__ void __launch_bounds__(256) k_params(const DevView v, const double* __restrict__ params) {
   extern __shared__ double sp[];  // raw parameter vector of point k [, original values]
   const int k = blockIdx.x;
   const int P = v.n_params;
+  if (blockIdx.y > 0) {
+    // on the parameters as given (the eigen parameters of decomposed blocks,
+    // as the reference's penalty in eigen mode); u_p = sum_j C^-1[j][p] delta_j
+    for (int p = threadIdx.x; p < P; p += blockDim.x) sp[p] = params[(size_t)k * P + p] - v.prior_mean[p];
+    __syncthreads();
+    const int j0 = ((int)blockIdx.y - 1) * kPenRows, j1 = min(P, j0 + kPenRows);
+    double acc = 0;
+    for (int p = threadIdx.x; p < P; p += blockDim.x) {
+      const double* col = v.prior_icov + (size_t)j0 * P + p;
+      double c[kPenRows];
+#pragma unroll
+      for (int j = 0; j < kPenRows; ++j) c[j] = j0 + j < j1 ? col[(size_t)j * P] : 0.0;
+      double u = 0;
+#pragma unroll
+      for (int j = 0; j < kPenRows; ++j)
+        if (j0 + j < j1) u += c[j] * sp[j0 + j];
+      acc += sp[p] * u;
+    }
+    __shared__ double red[8];
+    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) red[warp] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0;
+      for (int w = 0; w < 8; ++w) t += red[w];
+      v.penalty[(size_t)(blockIdx.y - 1) * v.kpad + k] = t;
+    }
+    return;
+  }
   for (int p = threadIdx.x; p < P; p += blockDim.x) sp[p] = params[(size_t)k * P + p];
   __syncthreads();
   // eigen-decomposed blocks back to the original parameters
@@ -80,28 +120,6 @@ __global__ void __launch_bounds__(256) k_params(const DevView v, const double* _
       r.jb = 4 * coef_interval(xx, gd.n, gd.trunc != 0, r.u);
       gp[(size_t)g * v.kpad + k] = r;
     }
-  }
-  if (!v.has_prior) return;
-  // delta^T C^-1 delta on the parameters as given (the eigen parameters of
-  // decomposed blocks, as the reference's penalty in eigen mode), u = C^-1
-  // delta formed row by row.
-  double acc = 0;
-  for (int i = threadIdx.x; i < P; i += blockDim.x) {
-    const double* row = v.prior_icov + (size_t)i * P;
-    double u = 0;
-    for (int j = 0; j < P; ++j) u += row[j] * (sp[j] - v.prior_mean[j]);
-    acc += (sp[i] - v.prior_mean[i]) * u;
-  }
-  __shared__ double red[32];
-  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) red[warp] = acc;
-  __syncthreads();
-  if (warp == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    double t = lane < nw ? red[lane] : 0.0;
-    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0) v.penalty[k] = t;
   }
 }
 
@@ -432,59 +450,119 @@ __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_
 // ---------------------------------------------------------------------------
 // Bin sums and likelihood.
 // ---------------------------------------------------------------------------
+// One block covers BT bins of KT points, 256 threads:
+//   1. thread (point kk, slot lane sl, bin bb), points fastest so that the
+//      reads of a slot's row are contiguous, adds slots i0 + sl, + SL, ... of
+//      its bin in order; the SL lanes' sums are added in lane order;
+//   2. thread (bin, point), bins fastest, writes the sums and evaluates the
+//      likelihood term; the BT terms of a point are added by a shuffle tree;
+//   3. the last block of a point tile adds its blocks' parts and the penalty's
+//      in a fixed order.
+// A Barlow-Beeston term is ~150 FP64 instructions and an SM issues one warp of
+// them every 16 cycles, so the terms are cut into many small blocks with full
+// warps: 256 bins per block left 140 SMs idle at K = 1 (19.2 us for 3000 bins,
+// now 14.8 us; the launch alone is 5 us).  The small KT give their threads to the slots of a bin instead,
+// whose reads are a chain of L2 latencies.
+template <int KT, int BT>
 __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double* sums, double* sums2,
                                                   double* llh, double* llh_stat) {
-  const int k = blockIdx.y;
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  double term = 0.0;
-  if (b < v.n_bins) {
-    double s = 0.0, s2 = 0.0;
-    const int i0 = v.bin_slot[b], i1 = v.bin_slot[b + 1];
-    for (int i = i0; i < i1; ++i) {
-      const double2 p = v.partials[(size_t)i * v.kpad + k];
-      s += p.x;
-      s2 += p.y;
-    }
-    if (sums) sums[(size_t)k * v.n_bins + b] = s;
-    if (sums2) sums2[(size_t)k * v.n_bins + b] = s2;
-    if (v.llh_type == 1) {
-      term = llh_poisson(v.data[b], s);
-    } else if (v.llh_type == 2) {
-      term = llh_bb_bin(v.data[b], s, sqrt(s2));  // BinContent::sqrtSumSqWeights, squared again by the LLH
-    }
-  }
-  if (v.llh_type == 0 || (llh == nullptr && llh_stat == nullptr)) return;
-  __shared__ double red[32];
+  constexpr int NT = 256, SL = NT / (KT * BT);
+  static_assert(SL >= 1 && SL * KT * BT == NT && BT <= 32 && NT % KT == 0, "tile shape");
+  __shared__ double2 part[SL][BT][KT + (KT > 1 ? 1 : 0)];
+  __shared__ double red[NT];
   __shared__ bool last;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int o = 16; o; o >>= 1) term += __shfl_xor_sync(0xffffffffu, term, o);
-  if (lane == 0) red[warp] = term;
+  const int tid = threadIdx.x;
+  const int kb = blockIdx.y * KT, b0 = blockIdx.x * BT;
+  {
+    const int kk = tid % KT, sl = (tid / KT) % SL, bb = tid / (KT * SL);
+    const int b = b0 + bb, k = kb + kk;
+    double s = 0.0, s2 = 0.0;
+    if (b < v.n_bins && k < K) {
+      const int i1 = v.bin_slot[b + 1];
+      int i = v.bin_slot[b] + sl;
+      const double2* src = v.partials + k;
+      // four rows in flight, added in order
+      for (; i + 3 * SL < i1; i += 4 * SL) {
+        double2 p[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) p[q] = src[(size_t)(i + q * SL) * v.kpad];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          s += p[q].x;
+          s2 += p[q].y;
+        }
+      }
+      for (; i < i1; i += SL) {
+        const double2 p = src[(size_t)i * v.kpad];
+        s += p.x;
+        s2 += p.y;
+      }
+    }
+    part[sl][bb][kk] = make_double2(s, s2);
+  }
   __syncthreads();
-  if (warp == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    double t = lane < nw ? red[lane] : 0.0;
-    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0) {
-      v.llh_blocks[(size_t)k * v.llh_nblk + blockIdx.x] = t;
-      __threadfence();
-      const unsigned prev = atomicAdd(&v.llh_counter[k], 1u);
-      last = (prev == gridDim.x - 1);
+  const bool want_llh = v.llh_type != 0 && (llh != nullptr || llh_stat != nullptr);
+  if (tid < KT * BT) {
+    const int bb = tid % BT, kk = tid / BT;
+    const int b = b0 + bb, k = kb + kk;
+    const bool in = b < v.n_bins && k < K;
+    double term = 0.0;
+    if (in) {
+      double s = 0.0, s2 = 0.0;
+#pragma unroll
+      for (int q = 0; q < SL; ++q) {
+        const double2 p = part[q][bb][kk];
+        s = q ? s + p.x : p.x;
+        s2 = q ? s2 + p.y : p.y;
+      }
+      if (sums) sums[(size_t)k * v.n_bins + b] = s;
+      if (sums2) sums2[(size_t)k * v.n_bins + b] = s2;
+      if (want_llh) {
+        if (v.llh_type == 1)
+          term = llh_poisson(v.data[b], s);
+        else if (v.llh_type == 2)  // BinContent::sqrtSumSqWeights, squared again by the LLH
+          term = llh_bb_bin(v.data[b], v.log_data[b], s, sqrt(s2));
+      }
+    }
+    if (want_llh) {
+      // whole warps are in this branch (KT * BT is a multiple of 32)
+#pragma unroll
+      for (int o = BT / 2; o; o >>= 1) term += __shfl_xor_sync(0xffffffffu, term, o);
+      if (bb == 0 && k < K) v.llh_blocks[(size_t)blockIdx.x * v.kpad + k] = term;
     }
   }
+  if (!want_llh) return;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) last = atomicAdd(&v.llh_counter[blockIdx.y], 1u) == gridDim.x - 1;
   __syncthreads();
   if (!last) return;
-  if (warp == 0) {
-    __threadfence();
-    double t = 0.0;
-    for (int i = lane; i < (int)gridDim.x; i += 32) t += __ldcg(&v.llh_blocks[(size_t)k * v.llh_nblk + i]);
-    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0) {
-      const double pen = v.has_prior ? v.penalty[k] : 0.0;
-      if (llh_stat) llh_stat[k] = t;
-      if (llh) llh[k] = t + pen;
-      v.llh_counter[k] = 0u;
-    }
+  __threadfence();
+  constexpr int NL = NT / KT;
+  const int kk = tid % KT, l = tid / KT, k = kb + kk;
+  double t = 0.0;
+  if (k < K)
+    for (int i = l; i < (int)gridDim.x; i += NL) t += __ldcg(&v.llh_blocks[(size_t)i * v.kpad + k]);
+  red[tid] = t;
+  for (int h = NL / 2; h; h >>= 1) {
+    __syncthreads();
+    if (l < h) red[tid] += red[tid + h * KT];
   }
+  if (l == 0 && k < K) {
+    t = red[tid];
+    double pen = 0.0;
+    for (int q = 0; q < v.n_pen; ++q) pen += v.penalty[(size_t)q * v.kpad + k];
+    if (llh_stat) llh_stat[k] = t;
+    if (llh) llh[k] = t + pen;
+  }
+  if (tid == 0) v.llh_counter[blockIdx.y] = 0u;
+}
+
+// log(data) per bin, taken once when the data are set instead of per bin and
+// point in every evaluation.
+__global__ void k_log_data(const double* __restrict__ data, double* __restrict__ log_data, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) log_data[i] = log_data_of(data[i]);
 }
 
 }  // namespace
@@ -606,12 +684,13 @@ cudaError_t prepare_params(const DevView& v) {
 
 cudaError_t launch_params(const DevView& v, const double* params, int K, cudaStream_t s) {
   const size_t smem = params_smem_bytes(v);
+  const dim3 grid(K, 1 + v.n_pen);
   if (v.precision == 2)
-    k_params<dfloat><<<K, 256, smem, s>>>(v, params);
+    k_params<dfloat><<<grid, 256, smem, s>>>(v, params);
   else if (v.precision)
-    k_params<float><<<K, 256, smem, s>>>(v, params);
+    k_params<float><<<grid, 256, smem, s>>>(v, params);
   else
-    k_params<double><<<K, 256, smem, s>>>(v, params);
+    k_params<double><<<grid, 256, smem, s>>>(v, params);
   return cudaGetLastError();
 }
 
@@ -670,8 +749,23 @@ cudaError_t launch_batched(const DevView& v, int K, const BatchedShape& b, int g
 
 cudaError_t launch_bins_llh(const DevView& v, int K, double* sums, double* sums2, double* llh,
                             double* llh_stat, cudaStream_t s) {
-  dim3 grid(v.llh_nblk, K);
-  k_bins_llh<<<grid, 256, 0, s>>>(v, K, sums, sums2, llh, llh_stat);
+  // point tiles as wide as K allows, so that phase 2's warps are full
+  auto grid = [&](int kt, int bt) { return dim3((v.n_bins + bt - 1) / bt, (K + kt - 1) / kt); };
+  if (K == 1)
+    k_bins_llh<1, 32><<<grid(1, 32), 256, 0, s>>>(v, K, sums, sums2, llh, llh_stat);
+  else if (K <= 4)
+    k_bins_llh<4, 16><<<grid(4, 16), 256, 0, s>>>(v, K, sums, sums2, llh, llh_stat);
+  else if (K <= 8)
+    k_bins_llh<8, 16><<<grid(8, 16), 256, 0, s>>>(v, K, sums, sums2, llh, llh_stat);
+  else if (K <= 16)
+    k_bins_llh<16, 16><<<grid(16, 16), 256, 0, s>>>(v, K, sums, sums2, llh, llh_stat);
+  else
+    k_bins_llh<32, kLlhBins><<<grid(32, kLlhBins), 256, 0, s>>>(v, K, sums, sums2, llh, llh_stat);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_log_data(const DevView& v, cudaStream_t s) {
+  k_log_data<<<(v.n_bins + 255) / 256, 256, 0, s>>>(v.data, v.log_data, v.n_bins);
   return cudaGetLastError();
 }
 
@@ -687,7 +781,7 @@ __global__ void k_llh_bins(int type, const double* data, const double* pred, con
                            double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  out[i] = type == GW_LLH_POISSON ? llh_poisson(data[i], pred[i]) : llh_bb_bin(data[i], pred[i], sqrt_sum_w2[i]);
+  out[i] = type == GW_LLH_POISSON ? llh_poisson(data[i], pred[i]) : llh_bb_bin(data[i], log_data_of(data[i]), pred[i], sqrt_sum_w2[i]);
 }
 }  // namespace
 }  // namespace gw

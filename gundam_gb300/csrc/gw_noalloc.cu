@@ -3,8 +3,8 @@
 //
 // gw_llh_noalloc computes, for K parameter points, the summed per-bin
 // likelihood from bin sums the caller already holds on the device: the same
-// per-bin terms and the same fixed-order block / last-block reduction as the
-// engine's k_bins_llh.  That reduction needs scratch memory (one partial per
+// per-bin terms as the engine's k_bins_llh, and a fixed-order block /
+// last-block reduction.  That reduction needs scratch memory (one partial per
 // block and one arrival counter per point).  The engine allocates it with
 // cudaMalloc; here it is a fixed-size array in device global memory that the
 // library defines at file scope, so the call itself allocates nothing.
@@ -51,8 +51,8 @@ static __device__ __align__(256) unsigned char gw_noalloc_scratch[kNoAllocBytes]
 namespace gw {
 namespace {
 
-// Variant of k_bins_llh: per-bin terms from caller-provided sums, reduced per
-// point in the same fixed order; scratch = the file-scope array.
+// Per-bin terms of k_bins_llh from caller-provided sums, reduced per point in a
+// fixed order; scratch = the file-scope array.
 __global__ void __launch_bounds__(256) k_llh_noalloc(const double* __restrict__ sums,
                                                      const double* __restrict__ sums2,
                                                      const double* __restrict__ data, int n_bins, int llh_type,
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(256) k_llh_noalloc(const double* __restrict__ 
     if (llh_type == GW_LLH_POISSON) {
       term = llh_poisson(data[b], s);
     } else {
-      term = llh_bb_bin(data[b], s, sqrt(s2));
+      term = llh_bb_bin(data[b], log_data_of(data[b]), s, sqrt(s2));
     }
   }
   __shared__ double red[32];
