@@ -3,15 +3,14 @@
 //
 // Every GEMM is C[M x N] = A[M x K] * B[N x K]^T with both operands K-major
 // (contiguous along K) in BF16 and FP32 accumulation in tensor memory (TMEM):
-//   * one CTA (4 warps) owns a 128 x BN output tile;
-//   * the K loop stages 128 x 64 and BN x 64 BF16 tiles in shared memory in
-//     the canonical no-swizzle core-matrix layout (8 rows x 16 bytes per core
-//     matrix), double-buffered;
+//   * one CTA (4 or 8 warps) owns a 128 x BN output tile;
+//   * the K loop stages 128 x 64 and BN x 64 BF16 tiles in shared memory by TMA
+//     with the 128-byte swizzle, in a ring of S stages;
 //   * one elected thread issues tcgen05.mma (M = 128, N = BN, K = 16 each) and
 //     tcgen05.commit to an mbarrier per stage; every wait on it is bounded;
-//   * the epilogue reads the accumulator with tcgen05.ld (each warp its 32 TMEM
-//     lanes = rows) and fuses bias, SiLU, the SiLU derivative of the backward
-//     pass, and row-major / transposed BF16 or FP32 stores;
+//   * the epilogue reads the accumulator with tcgen05.ld (a thread: one row) and
+//     fuses bias, SiLU, the SiLU derivative of the backward pass, the training
+//     loss and its gradient, and row-major / transposed BF16 or FP32 stores;
 //   * TMEM is allocated once per CTA and freed on every exit path.
 // Forward: z = W x + b, h = silu(z); backward: dX = dY W (with the SiLU
 // derivative fused), dW = dY^T X; Adam on FP32 master weights refreshes the
@@ -37,7 +36,6 @@ typedef __nv_bfloat16 bf16;
 
 constexpr int kBM = 128;
 constexpr int kBK = 64;
-constexpr int kThreads = 128;
 constexpr uint64_t kWaitNs = 1000000000ull;  // 1 s per MMA commit
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -132,6 +130,13 @@ struct Epilogue {
   bf16* out_bf16;       // [M x N] after the activation, or null
   bf16* out_bf16_t;     // [N x M] after the activation, or null
   int ld_t;             // leading dimension of out_bf16_t (>= M)
+  // mean squared error against rows perm[r] (perm null: r) of target [. x N], or
+  // null: the BF16 outputs are then its gradient 2 e * inv, e = value - target,
+  // and *loss += scale * inv * sum e^2 (one atomic per tile)
+  const float* target;
+  const int32_t* perm;
+  float* loss;
+  float inv, scale;
 };
 
 // 2-D tiled TMA load of box {8 elements, R rows} at (k, row) into shared
@@ -163,6 +168,52 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// A thread's 32 consecutive values of one row of an FP32 matrix (p: the first,
+// 16-byte aligned when `vec`); only the first n are read or written.
+__device__ __forceinline__ void row_load(const float* __restrict__ p, int n, bool vec, float (&v)[32]) {
+  if (vec && n == 32) {
+#pragma unroll
+    for (int q = 0; q < 32; q += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(p + q);
+      v[q] = f.x;
+      v[q + 1] = f.y;
+      v[q + 2] = f.z;
+      v[q + 3] = f.w;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 32; ++q) v[q] = q < n ? p[q] : 0.f;
+  }
+}
+
+__device__ __forceinline__ void row_store(float* p, int n, bool vec, const float (&v)[32]) {
+  if (vec && n == 32) {
+#pragma unroll
+    for (int q = 0; q < 32; q += 4) *reinterpret_cast<float4*>(p + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 32; ++q)
+      if (q < n) p[q] = v[q];
+  }
+}
+
+__device__ __forceinline__ void row_store(bf16* p, int n, bool vec, const bf16 (&v)[32]) {
+  if (vec && n == 32) {
+#pragma unroll
+    for (int q = 0; q < 32; q += 8) {
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        w[i] = (uint32_t)__bfloat16_as_ushort(v[q + 2 * i]) | (uint32_t)__bfloat16_as_ushort(v[q + 2 * i + 1]) << 16;
+      *reinterpret_cast<uint4*>(p + q) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 32; ++q)
+      if (q < n) p[q] = v[q];
+  }
+}
+
 // Pipelined GEMM tile, C[128 x BN] = A[128 x K] * B[BN x K]^T.
 //   * thread 0 (warp 0) issues the TMA loads of each 64-wide K tile into one
 //     of S shared-memory stages (one box of 64 K-elements x rows per operand,
@@ -171,22 +222,31 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 //   * thread 32 (warp 1) waits for a stage, issues its four K = 16 MMAs and
 //     commits them to the stage's "empty" barrier, which lets the producer
 //     refill it; a final commit signals the epilogue;
-//   * all four warps read the accumulator from TMEM (warp w: rows 32w..32w+31)
-//     and store through a per-warp shared-memory transpose, so that row-major
-//     stores and gate loads are coalesced.
+//   * all NW warps read the accumulator from TMEM, warp w the rows
+//     32 (w % 4) .. + 31 and every (NW / 4)-th group of 32 columns, one row per
+//     thread, and load and store that row's 32 values as 16-byte vectors (128
+//     contiguous bytes per thread and matrix).  The gate or target values of a
+//     thread's first columns are loaded before it waits for the accumulator.
+//     A warp that went through 32 dependent loads per gate tile and a
+//     shared-memory transpose per output bound every backward product: 44 us
+//     (M = 2048, N = K = 512, against 17 us without a gate); now 11 us with or
+//     without one.
 // Every wait is bounded; on a timeout the tile records the failure in
 // *status, drains its own copies (bounded) and frees TMEM.
-template <int BN, int S>
-__global__ void __launch_bounds__(kThreads) k_gemm(const __grid_constant__ CUtensorMap tmA,
-                                                   const __grid_constant__ CUtensorMap tmB, int M, int N, int K,
-                                                   Epilogue ep, uint32_t* status) {
+template <int BN, int S, int NW>
+__global__ void __launch_bounds__(NW * 32) k_gemm(const __grid_constant__ CUtensorMap tmA,
+                                                  const __grid_constant__ CUtensorMap tmB, int M, int N, int K,
+                                                  Epilogue ep, uint32_t* status) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   constexpr int kA = kBM * kBK * 2;  // 16 KB
   constexpr int kB = BN * kBK * 2;
   constexpr int kStage = kA + kB;
+  constexpr int kGroups = NW / 4;  // column groups of the epilogue
+  static_assert(BN % (32 * kGroups) == 0, "every column group has whole 32-column chunks");
   __shared__ __align__(8) uint64_t full[S], empty[S], done;
   __shared__ float sbias[BN];  // the tile's bias columns, read by every row of the epilogue
+  __shared__ float sloss[NW];
   __shared__ uint32_t tmem_base;
   __shared__ volatile int failed;
 
@@ -196,7 +256,7 @@ __global__ void __launch_bounds__(kThreads) k_gemm(const __grid_constant__ CUten
   if (ep.bias) {
     // one coalesced load per column instead of one load per element in the
     // epilogue, where the dependent loads stalled the tile's four warps
-    for (int c = tid; c < BN; c += kThreads) sbias[c] = (n0 + c < N) ? ep.bias[n0 + c] : 0.f;
+    for (int c = tid; c < BN; c += NW * 32) sbias[c] = (n0 + c < N) ? ep.bias[n0 + c] : 0.f;
   }
   if (tid == 0) {
     for (int i = 0; i < S; ++i) {
@@ -255,6 +315,24 @@ __global__ void __launch_bounds__(kThreads) k_gemm(const __grid_constant__ CUten
     mma_commit(&done);
   }
   __syncwarp();
+
+  // this thread's row, and the gate / target values of its first columns
+  const int r = m0 + (warp & 3) * 32 + lane;
+  const bool row_ok = r < M;
+  const bool vec = (N & 7) == 0;  // rows of every operand stay 16-byte aligned
+  const float* pre_row = nullptr;
+  if (row_ok) {
+    if (ep.gate) pre_row = ep.gate + (size_t)r * N;
+    else if (ep.target) pre_row = ep.target + (size_t)(ep.perm ? ep.perm[r] : r) * N;
+  }
+  constexpr int kStep = 32 * kGroups;
+  const int cfirst = (warp >> 2) * 32;
+  float pre[32];
+  auto load_pre = [&](int c0) {
+    if (pre_row && n0 + c0 < N) row_load(pre_row + n0 + c0, min(32, N - (n0 + c0)), vec, pre);
+  };
+  load_pre(cfirst);
+
   const bool ok = mbar_wait_bounded(&done, 0);
   if (!ok) failed = 1;
   __syncthreads();
@@ -272,67 +350,63 @@ __global__ void __launch_bounds__(kThreads) k_gemm(const __grid_constant__ CUten
   }
   tc_fence_after();
 
-  // epilogue: the pipeline's shared memory is free now
-  float* tr = reinterpret_cast<float*>(smem) + warp * (32 * 33);
-  const int rbase = m0 + warp * 32;
-  const int r = rbase + lane;
-  const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-  for (int c0 = 0; c0 < BN; c0 += 32) {
+  const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  float e2 = 0.f;
+  for (int c0 = cfirst; c0 < BN; c0 += kStep) {
     if (n0 + c0 >= N) break;
     float v[32];
     tmem_ld32(lane_addr + (uint32_t)c0, v);
-    const int ncol = min(32, N - (n0 + c0));
-    if (ep.gate) {
-      // coalesced load of the gate tile [32 rows x 32 cols] -> transpose
-      __syncwarp();
-      for (int i = 0; i < 32; ++i) {
-        const int rr = rbase + i;
-        tr[i * 33 + lane] = (rr < M && lane < ncol) ? ep.gate[(size_t)rr * N + n0 + c0 + lane] : 0.f;
+    if (row_ok) {
+      const int ncol = min(32, N - (n0 + c0));
+      const size_t o = (size_t)r * N + n0 + c0;
+      if (ep.gate) {
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+          const float g = pre[q];
+          const float sg = sigmoidf_(g);
+          v[q] *= sg * (1.f + g * (1.f - sg));
+        }
       }
-      __syncwarp();
+      if (ep.bias) {
 #pragma unroll
-      for (int q = 0; q < 32; ++q) {
-        const float g = tr[lane * 33 + q];
-        const float sg = sigmoidf_(g);
-        v[q] *= sg * (1.f + g * (1.f - sg));
+        for (int q = 0; q < 32; ++q) v[q] += sbias[c0 + q];
       }
-    }
+      if (ep.out_f32) row_store(ep.out_f32 + o, ncol, vec, v);
+      if (ep.target) {
 #pragma unroll
-    for (int q = 0; q < 32; ++q)
-      if (ep.bias && q < ncol) v[q] += sbias[c0 + q];
-    if (ep.out_f32) {
-      __syncwarp();
-#pragma unroll
-      for (int q = 0; q < 32; ++q) tr[lane * 33 + q] = v[q];
-      __syncwarp();
-      for (int i = 0; i < 32; ++i) {
-        const int rr = rbase + i;
-        if (rr < M && lane < ncol) ep.out_f32[(size_t)rr * N + n0 + c0 + lane] = tr[i * 33 + lane];
+        for (int q = 0; q < 32; ++q) {
+          const float e = v[q] - pre[q];
+          if (q < ncol) e2 += e * e;
+          v[q] = 2.f * e * ep.inv;
+        }
       }
-    }
-    if (ep.out_bf16 || ep.out_bf16_t) {
+      load_pre(c0 + kStep);
+      if (ep.out_bf16 || ep.out_bf16_t) {
+        bf16 h[32];
 #pragma unroll
-      for (int q = 0; q < 32; ++q) v[q] = (ep.act == 1) ? v[q] * sigmoidf_(v[q]) : v[q];
-      if (ep.out_bf16_t && r < M) {
+        for (int q = 0; q < 32; ++q) h[q] = __float2bfloat16((ep.act == 1) ? v[q] * sigmoidf_(v[q]) : v[q]);
+        if (ep.out_bf16) row_store(ep.out_bf16 + o, ncol, vec, h);
+        if (ep.out_bf16_t) {
 #pragma unroll
-        for (int q = 0; q < 32; ++q)
-          if (q < ncol) ep.out_bf16_t[(size_t)(n0 + c0 + q) * ep.ld_t + r] = __float2bfloat16(v[q]);
-      }
-      if (ep.out_bf16) {
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < 32; ++q) tr[lane * 33 + q] = v[q];
-        __syncwarp();
-        for (int i = 0; i < 32; ++i) {
-          const int rr = rbase + i;
-          if (rr < M && lane < ncol) ep.out_bf16[(size_t)rr * N + n0 + c0 + lane] = __float2bfloat16(tr[i * 33 + lane]);
+          for (int q = 0; q < 32; ++q)
+            if (q < ncol) ep.out_bf16_t[(size_t)(n0 + c0 + q) * ep.ld_t + r] = h[q];
         }
       }
     }
+    __syncwarp();
+  }
+  if (ep.target) {
+    for (int o = 16; o; o >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, o);
+    if (lane == 0) sloss[warp] = e2;
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, BN);
+  if (ep.target && tid == 0) {
+    float t = 0.f;
+    for (int w = 0; w < NW; ++w) t += sloss[w];
+    atomicAdd(ep.loss, t * ep.inv * ep.scale);
+  }
 }
 
 // ---- small kernels ----
@@ -362,82 +436,121 @@ __global__ void k_rows_to_bf16(const float* __restrict__ x, const int32_t* __res
   }
 }
 
-// Mean squared error against target rows perm[r] of t (perm null: row r) and
-// its gradient dy = 2 (y - t) / (rows * cols), row-major and transposed
-// (tiled as k_rows_to_bf16).  loss += scale * sum e^2 / (rows * cols), one
-// atomic per block.
-__global__ void k_mse(const float* __restrict__ y, const float* __restrict__ t, const int32_t* __restrict__ perm,
-                      int rows, int cols, bf16* dy, bf16* dyt, int ld_t, float* loss, float scale) {
-  __shared__ bf16 tile[32][34];
-  __shared__ float red[8];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const float inv = 1.f / ((float)rows * (float)cols);
-  float e2 = 0.f;
-  for (int i = ty; i < 32; i += 8) {
-    const int r = r0 + i, c = c0 + tx;
-    bf16 g = __float2bfloat16(0.f);
-    if (r < rows && c < cols) {
-      const size_t tr = perm ? (size_t)perm[r] : (size_t)r;
-      const float e = y[(size_t)r * cols + c] - t[tr * cols + c];
-      e2 += e * e;
-      g = __float2bfloat16(2.f * e * inv);
-      dy[(size_t)r * cols + c] = g;
-    }
-    tile[i][tx] = g;
-  }
-  __syncthreads();
-  for (int i = ty; i < 32; i += 8) {
-    const int c = c0 + i, r = r0 + tx;
-    if (c < cols && r < rows) dyt[(size_t)c * ld_t + r] = tile[tx][i];
-  }
-  for (int o = 16; o; o >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, o);
-  if (tx == 0) red[ty] = e2;
-  __syncthreads();
-  if (ty == 0 && tx == 0) {
-    float b = 0.f;
-    for (int i = 0; i < 8; ++i) b += red[i];
-    atomicAdd(loss, b * inv * scale);
-  }
-}
-
-// Column sums of a row-major BF16 matrix (bias gradients): block (32, 16),
-// 32 columns per block, a fixed-order reduction over the 16 row strides.
-__global__ void k_colsum(const bf16* __restrict__ g, int rows, int cols, float* out) {
-  __shared__ float part[16][33];
-  const int c = blockIdx.x * 32 + threadIdx.x;
+// Bias gradient of one output unit by 16 lanes: the FP32 sum of its BF16 row
+// dzt [B].  Lane q adds the elements q, q + 16, ... in order, then the 16 parts
+// are added in lane order; the sum on every lane of the half-warp.
+__device__ __forceinline__ float bias_grad(const bf16* __restrict__ dzt, int B) {
+  const int q = threadIdx.x & 15;
   float s = 0.f;
-  if (c < cols)
-    for (int r = threadIdx.y; r < rows; r += 16) s += __bfloat162float(g[(size_t)r * cols + c]);
-  part[threadIdx.y][threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.y == 0 && c < cols) {
-    float t = 0.f;
-    for (int i = 0; i < 16; ++i) t += part[i][threadIdx.x];
-    out[c] = t;
+  int i = q;
+  for (; i + 15 * 16 < B; i += 256) {
+    bf16 u[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) u[j] = dzt[i + 16 * j];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) s += __bfloat162float(u[j]);
   }
+  for (; i < B; i += 16) s += __bfloat162float(dzt[i]);
+  __syncwarp();
+  float t = 0.f;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) t += __shfl_sync(0xffffffffu, s, j, 16);
+  return t;
 }
 
-// Adam on FP32 master weights; refreshes the BF16 copy and its transpose.
-__global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                       int n, int rows, int cols, float lr, float b1, float b2, float eps, float c1, float c2,
-                       bf16* wb, bf16* wt) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gi;
-  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-  w[i] = wi;
-  if (wb) {
-    const bf16 b = __float2bfloat16(wi);
-    wb[i] = b;
-    if (wt && rows > 0) {
-      const int r = i / cols, c = i % cols;
-      wt[(size_t)c * rows + r] = b;
+// Bias gradients of one layer, a half-warp per unit (gwm_gradients).
+__global__ void __launch_bounds__(256) k_bias_grad(const bf16* __restrict__ dzt, int rows, int B, float* out) {
+  const int r = blockIdx.x * 16 + (threadIdx.x >> 4);
+  const float g = bias_grad(dzt + (size_t)min(r, rows - 1) * B, B);  // whole warps stay in the shuffles
+  if (r < rows && (threadIdx.x & 15) == 0) out[r] = g;
+}
+
+__device__ __forceinline__ float adam_value(float w, float g, float& m, float& v, float lr, float c1, float c2) {
+  constexpr float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  m = b1 * m + (1.f - b1) * g;
+  v = b2 * v + (1.f - b2) * g * g;
+  return w - lr * (m / c1) / (sqrtf(v / c2) + eps);
+}
+
+constexpr int kMaxLayers = 16;
+struct AdamLayer {
+  float *w, *m, *v, *b, *mb, *vb;
+  const float* g;
+  bf16 *wb, *wt;
+  const bf16* dzt;  // [rows x batch] output gradients, for the biases (null: biases stay)
+  int rows, cols;
+  int tile0, bias0;  // first weight tile and first bias block of the layer
+};
+struct AdamArgs {
+  AdamLayer l[kMaxLayers];
+  int n_layers, n_tiles, batch;
+  float lr, c1, c2;
+};
+
+// Adam on the FP32 master weights and biases of every layer in one launch.
+// Blocks [0, n_tiles): 32 x 32 weight tiles, whose BF16 copy and its
+// transpose are both stored coalesced (the transpose through shared memory);
+// the blocks after them: 16 biases each, whose gradient is formed here from
+// the layer's transposed output gradients.  A launch per weight and bias array
+// with a scattered transpose, and a column-sum launch per layer, took 99 us of a
+// 440 us step at 200 -> 512 -> 512 -> 512 -> 3000 and batch 2048; this launch
+// takes 24 us.  The bound is the 32 bytes per weight that w, g, m, v and the BF16
+// copies move (69 MB, mostly from L2).
+__global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamArgs a) {
+  const int tid = threadIdx.x;
+  int blk = blockIdx.x, li = 0;
+  if (blk < a.n_tiles) {
+    while (li + 1 < a.n_layers && blk >= a.l[li + 1].tile0) ++li;
+    const AdamLayer& L = a.l[li];
+    const int t = blk - L.tile0, tc = (L.cols + 31) / 32;
+    const int r0 = (t / tc) * 32, c0 = (t % tc) * 32;
+    const int tx = tid & 31, ty = tid >> 5;
+    __shared__ bf16 tile[32][34];
+    const int c = c0 + tx;
+    float w[4], g[4], m[4], v[4];
+    size_t at[4];
+    bool in[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int r = r0 + ty + 8 * j;
+      in[j] = r < L.rows && c < L.cols;
+      at[j] = (size_t)r * L.cols + c;
+      if (in[j]) {
+        w[j] = L.w[at[j]];
+        g[j] = L.g[at[j]];
+        m[j] = L.m[at[j]];
+        v[j] = L.v[at[j]];
+      }
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (!in[j]) continue;
+      w[j] = adam_value(w[j], g[j], m[j], v[j], a.lr, a.c1, a.c2);
+      L.w[at[j]] = w[j];
+      L.m[at[j]] = m[j];
+      L.v[at[j]] = v[j];
+      const bf16 b = __float2bfloat16(w[j]);
+      L.wb[at[j]] = b;
+      tile[ty + 8 * j][tx] = b;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int cc = c0 + ty + 8 * j, r = r0 + tx;
+      if (cc < L.cols && r < L.rows) L.wt[(size_t)cc * L.rows + r] = tile[tx][ty + 8 * j];
+    }
+    return;
+  }
+  blk -= a.n_tiles;
+  while (li + 1 < a.n_layers && blk >= a.l[li + 1].bias0) ++li;
+  const AdamLayer& L = a.l[li];
+  const int r = (blk - L.bias0) * 16 + (tid >> 4);
+  const float g = bias_grad(L.dzt + (size_t)min(r, L.rows - 1) * a.batch, a.batch);
+  if (r < L.rows && (tid & 15) == 0) {
+    float m = L.mb[r], v = L.vb[r];
+    L.b[r] = adam_value(L.b[r], g, m, v, a.lr, a.c1, a.c2);
+    L.mb[r] = m;
+    L.vb[r] = v;
   }
 }
 
@@ -915,7 +1028,7 @@ static int make_map(gwm_net* n, CUtensorMap* map, const bf16* p, int rows, int K
   return GW_OK;
 }
 
-template <int BN, int S>
+template <int BN, int S, int NW>
 static int launch_gemm(gwm_net* n, const bf16* A, const bf16* B, int M, int N, int K, const gwm::Epilogue& ep) {
   CUtensorMap ma, mb;
   int rc = make_map(n, &ma, A, M, K, gwm::kBM);
@@ -924,30 +1037,34 @@ static int launch_gemm(gwm_net* n, const bf16* A, const bf16* B, int M, int N, i
   const size_t smem = gemm_smem(BN, S);
   static std::once_flag once;
   std::call_once(once, [smem]() {
-    cudaFuncSetAttribute(gwm::k_gemm<BN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(gwm::k_gemm<BN, S, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   dim3 grid((N + BN - 1) / BN, (M + gwm::kBM - 1) / gwm::kBM);
-  gwm::k_gemm<BN, S><<<grid, gwm::kThreads, smem, n->stream>>>(ma, mb, M, N, K, ep, n->status);
+  gwm::k_gemm<BN, S, NW><<<grid, NW * 32, smem, n->stream>>>(ma, mb, M, N, K, ep, n->status);
   GWM_CUDA(n, cudaGetLastError());
   return GW_OK;
 }
 
 // C[M x N] = A[M x K] * B[N x K]^T with the given epilogue.  The widest tile
-// that still gives one CTA per SM or more (148 of GB300's 152), else the
-// narrowest (64 columns): at the network's sizes a launch is one wave, and
-// a tile runs few K steps, so more CTAs, not wider tiles, keep the tensor
-// pipe busy (hidden layers, M = 2048, N = 512: 64 CTAs of 128 columns left
-// 88 SMs idle).  Ring depth: 128 x 256 tiles take two stages, so that two CTAs
-// (and their accumulators, 256 TMEM columns each) share an SM and one's
-// epilogue overlaps the other's MMAs; 64- and 128-column tiles take four.
+// that still gives one CTA per SM or more (148 of GB300's 152): at the
+// network's sizes a launch is one wave, and a tile runs few K steps, so more
+// CTAs, not wider tiles, keep the chip busy.  128 x 256 tiles take a ring of
+// two stages, so that two CTAs (and their accumulators, 256 TMEM columns each)
+// share an SM and one's epilogue overlaps the other's MMAs.  Where even
+// 64-column tiles leave half of the SMs idle (few rows, or the weight
+// gradients of the hidden layers), 32-column tiles with a ring of eight
+// stages: a product is then one latency chain per CTA, and eight stages put
+// the whole of K = 512 in flight at once (64 rows, N = K = 512: 17 us with
+// 64-column tiles and four stages, 9 us now; 3000 columns: 10.4 -> 8 us).
 // The tile shape does not change the order of any accumulation.
 static int gemm(gwm_net* n, const bf16* A, const bf16* B, int M, int N, int K, const gwm::Epilogue& ep) {
   if (K % 8 != 0) return gwm_fail(n, GW_ERR_ARG, "GEMM K must be a multiple of 8");
   const int tiles_m = (M + gwm::kBM - 1) / gwm::kBM;
   constexpr int kWave = 148;
-  if (N > 128 && tiles_m * ((N + 255) / 256) >= kWave) return launch_gemm<256, 2>(n, A, B, M, N, K, ep);
-  if (N > 64 && tiles_m * ((N + 127) / 128) >= kWave) return launch_gemm<128, 4>(n, A, B, M, N, K, ep);
-  return launch_gemm<64, 4>(n, A, B, M, N, K, ep);
+  if (N > 128 && tiles_m * ((N + 255) / 256) >= kWave) return launch_gemm<256, 2, 8>(n, A, B, M, N, K, ep);
+  if (N > 64 && tiles_m * ((N + 127) / 128) >= kWave) return launch_gemm<128, 4, 8>(n, A, B, M, N, K, ep);
+  if (N > 32 && tiles_m * ((N + 63) / 64) >= kWave / 2) return launch_gemm<64, 4, 8>(n, A, B, M, N, K, ep);
+  return launch_gemm<32, 8, 4>(n, A, B, M, N, K, ep);
 }
 
 static int check_status(gwm_net* n) {
@@ -1023,6 +1140,29 @@ extern "C" int gwm_last_error(const gwm_net* n, char* buf, size_t len) {
   return GW_OK;
 }
 
+// Appends layer l to the arguments of k_adam; batch: the rows of the layer's
+// transposed output gradients (biases).  Returns the bias blocks so far.
+static int adam_layer(gwm_net* n, int l, gwm::AdamArgs* a, int batch, int bias_blocks = 0) {
+  gwm::AdamLayer& L = a->l[a->n_layers++];
+  L.w = n->w[l];
+  L.m = n->mw[l];
+  L.v = n->vw[l];
+  L.b = n->b[l];
+  L.mb = n->mb[l];
+  L.vb = n->vb[l];
+  L.g = n->gw_[l];
+  L.wb = n->wb[l];
+  L.wt = n->wt[l];
+  L.dzt = n->dzt[l];
+  L.rows = n->dims[l + 1];
+  L.cols = n->dims[l];
+  L.tile0 = a->n_tiles;
+  L.bias0 = bias_blocks;
+  a->n_tiles += ((L.rows + 31) / 32) * ((L.cols + 31) / 32);
+  a->batch = batch;
+  return bias_blocks + (L.rows + 15) / 16;
+}
+
 // Weights of layer l: w [dims[l+1] x dims[l]] row-major, b [dims[l+1]] (host, FP32).
 extern "C" int gwm_set_layer(gwm_net* n, int32_t l, const float* w, const float* b) {
   if (!n || !w || !b || l < 0 || l >= n->n_layers) return GW_ERR_ARG;
@@ -1037,9 +1177,11 @@ extern "C" int gwm_set_layer(gwm_net* n, int32_t l, const float* w, const float*
   GWM_CUDA(n, cudaMemset(n->vw[l], 0, sizeof(float) * nw));
   GWM_CUDA(n, cudaMemset(n->mb[l], 0, sizeof(float) * rows));
   GWM_CUDA(n, cudaMemset(n->vb[l], 0, sizeof(float) * rows));
-  gwm::k_adam<<<(unsigned)((nw + 255) / 256), 256, 0, n->stream>>>(n->w[l], n->gw_[l], n->mw[l], n->vw[l], (int)nw,
-                                                                   rows, cols, 0.f, 0.9f, 0.999f, 1e-8f, 1.f, 1.f,
-                                                                   n->wb[l], n->wt[l]);
+  gwm::AdamArgs aa{};
+  adam_layer(n, l, &aa, 1);
+  aa.lr = 0.f;
+  aa.c1 = aa.c2 = 1.f;
+  gwm::k_adam<<<aa.n_tiles, 256, 0, n->stream>>>(aa);
   GWM_CUDA(n, cudaGetLastError());
   GWM_CUDA(n, cudaStreamSynchronize(n->stream));
   n->step = 0;
@@ -1056,17 +1198,47 @@ extern "C" int gwm_get_layer(gwm_net* n, int32_t l, float* w, float* b) {
   return GW_OK;
 }
 
-static int forward(gwm_net* n, int B) {
+// What a forward pass leaves behind besides the output z[L-1].
+enum Keep : int {
+  kKeepNone = 0,  // inference
+  kKeepZ = 1,     // the hidden pre-activations, for the input gradient
+  kKeepAll = 2    // and the transposed activations, for the weight gradients
+};
+
+// The training loss at the output: targets (rows perm[r] when perm is set),
+// *loss += scale * mean squared error.  The output z[L-1] itself is not stored.
+struct Loss {
+  const float* target;
+  const int32_t* perm;
+  float* loss;
+  float scale;
+};
+
+// Forward pass of the B rows in h[0].  With a loss, the output layer's tiles
+// form its gradient dz[L-1] (and the transpose) in their epilogue, so that the
+// B x dims[L] output is neither written nor read back.
+static int forward(gwm_net* n, int B, Keep keep, const Loss* loss = nullptr) {
   const int L = n->n_layers;
   for (int l = 0; l < L; ++l) {
     gwm::Epilogue ep{};
     ep.bias = n->b[l];
-    ep.act = (l + 1 < L) ? 1 : 0;
-    ep.out_f32 = n->z[l];
     if (l + 1 < L) {
+      ep.act = 1;
+      if (keep != kKeepNone) ep.out_f32 = n->z[l];
       ep.out_bf16 = n->h[l + 1];
-      ep.out_bf16_t = n->ht[l + 1];
+      if (keep == kKeepAll) ep.out_bf16_t = n->ht[l + 1];
       ep.ld_t = B;
+    } else if (loss) {
+      ep.target = loss->target;
+      ep.perm = loss->perm;
+      ep.loss = loss->loss;
+      ep.inv = 1.f / ((float)B * (float)n->dims[L]);
+      ep.scale = loss->scale;
+      ep.out_bf16 = n->dz[l];
+      ep.out_bf16_t = n->dzt[l];
+      ep.ld_t = B;
+    } else {
+      ep.out_f32 = n->z[l];
     }
     int rc = gemm(n, n->h[l], n->wb[l], B, n->dims[l + 1], n->dims[l], ep);
     if (rc) return rc;
@@ -1098,7 +1270,7 @@ extern "C" int gwm_forward(gwm_net* n, const float* x, int32_t B, float* y, int3
   if (!n || !x || !y || B < 1 || B > n->batch_max || B % 8) return gwm_fail(n, GW_ERR_ARG, "gwm_forward: bad batch");
   GWM_CUDA(n, cudaSetDevice(n->device));
   int rc = load_input(n, x, B, device_ptrs != 0);
-  if (!rc) rc = forward(n, B);
+  if (!rc) rc = forward(n, B, kKeepNone);
   if (rc) return rc;
   const int L = n->n_layers;
   GWM_CUDA(n, cudaMemcpyAsync(y, n->z[L - 1], sizeof(float) * (size_t)B * n->dims[L],
@@ -1108,15 +1280,14 @@ extern "C" int gwm_forward(gwm_net* n, const float* x, int32_t B, float* y, int3
 
 static int backward(gwm_net* n, int B) {
   const int L = n->n_layers;
-  // dz[L-1] (and its transpose) was written by the loss kernel
+  // dz[L-1] (and its transpose) was written by the forward pass's loss epilogue;
+  // the bias gradients follow from the dzt (k_adam, k_bias_grad)
   for (int l = L - 1; l >= 0; --l) {
     // dW_l = dz_l^T h_l : [dims[l+1] x dims[l]], K = B
     gwm::Epilogue e1{};
     e1.out_f32 = n->gw_[l];
     int rc = gemm(n, n->dzt[l], n->ht[l], n->dims[l + 1], n->dims[l], B, e1);
     if (rc) return rc;
-    gwm::k_colsum<<<(n->dims[l + 1] + 31) / 32, dim3(32, 16), 0, n->stream>>>(n->dz[l], B, n->dims[l + 1], n->gb[l]);
-    GWM_CUDA(n, cudaGetLastError());
     if (l > 0) {
       // dz_{l-1} = (dz_l W_l) * silu'(z_{l-1}) : [B x dims[l]], K = dims[l+1]
       gwm::Epilogue e2{};
@@ -1131,39 +1302,27 @@ static int backward(gwm_net* n, int B) {
   return GW_OK;
 }
 
-// Loss and output gradient against targets t (rows perm[r] when perm is set);
-// adds scale * loss into *loss.
-static int mse(gwm_net* n, const float* t, const int32_t* perm, int B, float* loss, float scale) {
-  const int L = n->n_layers, C = n->dims[L];
-  gwm::k_mse<<<tiles32(B, C), dim3(32, 8), 0, n->stream>>>(n->z[L - 1], t, perm, B, C, n->dz[L - 1], n->dzt[L - 1],
-                                                            B, loss, scale);
-  GWM_CUDA(n, cudaGetLastError());
-  return GW_OK;
-}
-
-static int loss_and_grad(gwm_net* n, const float* t, int B, bool device_ptr) {
-  const int L = n->n_layers, C = n->dims[L];
-  const size_t cnt = (size_t)B * C;
+// Forward pass with the loss against host or device targets t [B x dims[L]] in *n->loss.
+static int forward_loss(gwm_net* n, const float* t, int B, bool device_ptr) {
+  const size_t cnt = (size_t)B * n->dims[n->n_layers];
   GWM_CUDA(n, cudaMemcpyAsync(n->target, t, sizeof(float) * cnt,
                               device_ptr ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, n->stream));
   GWM_CUDA(n, cudaMemsetAsync(n->loss, 0, sizeof(float), n->stream));
-  return mse(n, n->target, nullptr, B, n->loss, 1.f);
+  const Loss ls{n->target, nullptr, n->loss, 1.f};
+  return forward(n, B, kKeepAll, &ls);
 }
 
-// One Adam update of every layer with learning rate lr.
-static int adam_all(gwm_net* n, float lr) {
+// One Adam update of every layer with learning rate lr after a backward pass of B rows.
+static int adam_all(gwm_net* n, int B, float lr) {
   n->step += 1;
-  const float b1 = 0.9f, b2 = 0.999f;
-  const float c1 = 1.f - powf(b1, (float)n->step), c2 = 1.f - powf(b2, (float)n->step);
-  for (int l = 0; l < n->n_layers; ++l) {
-    const int rows = n->dims[l + 1], cols = n->dims[l];
-    const int nw = rows * cols;
-    gwm::k_adam<<<(nw + 255) / 256, 256, 0, n->stream>>>(n->w[l], n->gw_[l], n->mw[l], n->vw[l], nw, rows, cols, lr,
-                                                         b1, b2, 1e-8f, c1, c2, n->wb[l], n->wt[l]);
-    gwm::k_adam<<<(rows + 255) / 256, 256, 0, n->stream>>>(n->b[l], n->gb[l], n->mb[l], n->vb[l], rows, 0, 1, lr,
-                                                           b1, b2, 1e-8f, c1, c2, nullptr, nullptr);
-    GWM_CUDA(n, cudaGetLastError());
-  }
+  gwm::AdamArgs a{};
+  int bias_blocks = 0;
+  for (int l = 0; l < n->n_layers; ++l) bias_blocks = adam_layer(n, l, &a, B, bias_blocks);
+  a.lr = lr;
+  a.c1 = 1.f - powf(0.9f, (float)n->step);
+  a.c2 = 1.f - powf(0.999f, (float)n->step);
+  gwm::k_adam<<<a.n_tiles + bias_blocks, 256, 0, n->stream>>>(a);
+  GWM_CUDA(n, cudaGetLastError());
   return GW_OK;
 }
 
@@ -1175,10 +1334,12 @@ extern "C" int gwm_gradients(gwm_net* n, const float* x, const float* t, int32_t
     return gwm_fail(n, GW_ERR_ARG, "gwm_gradients: bad batch");
   GWM_CUDA(n, cudaSetDevice(n->device));
   int rc = load_input(n, x, B, false);
-  if (!rc) rc = forward(n, B);
-  if (!rc) rc = loss_and_grad(n, t, B, false);
+  if (!rc) rc = forward_loss(n, t, B, false);
   if (!rc) rc = backward(n, B);
   if (rc) return rc;
+  for (int l = 0; l < n->n_layers; ++l)
+    gwm::k_bias_grad<<<(n->dims[l + 1] + 15) / 16, 256, 0, n->stream>>>(n->dzt[l], n->dims[l + 1], B, n->gb[l]);
+  GWM_CUDA(n, cudaGetLastError());
   rc = check_status(n);
   if (rc) return rc;
   for (int l = 0; l < n->n_layers; ++l) {
@@ -1196,10 +1357,9 @@ extern "C" int gwm_train_step(gwm_net* n, const float* x, const float* t, int32_
   if (!n || !x || !t || B < 8 || B > n->batch_max || B % 8) return gwm_fail(n, GW_ERR_ARG, "gwm_train_step: bad batch");
   GWM_CUDA(n, cudaSetDevice(n->device));
   int rc = load_input(n, x, B, device_ptrs != 0);
-  if (!rc) rc = forward(n, B);
-  if (!rc) rc = loss_and_grad(n, t, B, device_ptrs != 0);
+  if (!rc) rc = forward_loss(n, t, B, device_ptrs != 0);
   if (!rc) rc = backward(n, B);
-  if (!rc) rc = adam_all(n, lr);
+  if (!rc) rc = adam_all(n, B, lr);
   if (rc) return rc;
   if (loss) {
     GWM_CUDA(n, cudaMemcpyAsync(loss, n->loss, sizeof(float), cudaMemcpyDeviceToHost, n->stream));
@@ -1380,7 +1540,7 @@ extern "C" int gwm_predict(gwm_net* n, const double* theta, int32_t B, int32_t l
   int rc = stage_input(n, n->xin, nullptr, Bp, false);
   if (rc) return rc;
   GWM_CUDA(n, cudaGetLastError());
-  rc = forward(n, Bp);
+  rc = forward(n, Bp, kKeepNone);
   if (rc) return rc;
   rc = head_llh(n, B, llh_type, log_rates != nullptr);
   if (rc) return rc;
@@ -1530,10 +1690,10 @@ extern "C" int gwm_train_epochs(gwm_net* n, int32_t epochs, int32_t batch, float
     const double c = std::cos(M_PI * (double)s / (double)total);
     const float lr = (float)(lr_min + 0.5 * (lr0 - lr_min) * (1.0 + c));
     rc = stage_input(n, n->train_x, p, batch);
-    if (!rc) rc = forward(n, batch);
-    if (!rc) rc = mse(n, n->train_t, p, batch, d_loss + e, inv_spe);
+    const Loss ls{n->train_t, p, d_loss + e, inv_spe};
+    if (!rc) rc = forward(n, batch, kKeepAll, &ls);
     if (!rc) rc = backward(n, batch);
-    if (!rc) rc = adam_all(n, lr);
+    if (!rc) rc = adam_all(n, batch, lr);
   }
   (void)din;
   (void)nb;
@@ -1755,7 +1915,7 @@ static int surrogate_llh_device(gwm_net* n, int C, int llh_type) {
   gwm::k_standardize<<<(unsigned)(((size_t)Bp * din + 255) / 256), 256, 0, n->stream>>>(n->h_theta, Bp, din,
                                                                                      n->h_mean, n->h_scale, n->xin);
   int rc = stage_input(n, n->xin, nullptr, Bp, false);
-  if (!rc) rc = forward(n, Bp);
+  if (!rc) rc = forward(n, Bp, kKeepNone);
   if (rc) return rc;
   return head_llh(n, C, llh_type, false, false);
 }
@@ -1852,7 +2012,7 @@ extern "C" int gwm_substeps(gwm_net* n, const double* theta0, const double* f0, 
     gwm::k_propose_stage<<<C, thr, sh_prop, n->stream>>>(s->phi, P, s->Lt, seed, (uint64_t)st + 1, n->h_theta,
                                                         n->h_mean, n->h_scale, n->xin, n->h[0]);
     GWM_CUDA(n, cudaGetLastError());
-    rc = forward(n, Bp);
+    rc = forward(n, Bp, kKeepNone);
     if (!rc) rc = head_llh(n, C, llh_type, false, false);
     if (rc) break;
     gwm::k_finish_accept<<<C, thr, sh_fin, n->stream>>>(n->h_part, nbx, n->h_theta, P, prior ? s->m : nullptr,
@@ -1905,7 +2065,7 @@ extern "C" int gwm_value_grad(gwm_net* n, const double* theta, int32_t C, int32_
   gwm::k_standardize<<<(unsigned)(((size_t)Bp * din + 255) / 256), 256, 0, n->stream>>>(n->h_theta, Bp, din,
                                                                                      n->h_mean, n->h_scale, n->xin);
   int rc = stage_input(n, n->xin, nullptr, Bp, false);
-  if (!rc) rc = forward(n, Bp);
+  if (!rc) rc = forward(n, Bp, kKeepZ);
   if (rc) return rc;
   // the head: likelihood partials, G, S and dY (rows C..Bp of dY stay zero)
   GWM_CUDA(n, cudaMemsetAsync(n->dz[L - 1], 0, sizeof(bf16) * (size_t)Bp * nb, n->stream));
