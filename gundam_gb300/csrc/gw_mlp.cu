@@ -424,11 +424,10 @@ __global__ void k_rows_to_bf16(const float* __restrict__ x, const int32_t* __res
     if (r < rows && c < cols) {
       const size_t src = perm ? (size_t)perm[r] : (size_t)r;
       v = __float2bfloat16(x[src * cols + c]);
-      if (y) y[(size_t)r * cols + c] = v;
+      y[(size_t)r * cols + c] = v;
     }
     tile[i][tx] = v;
   }
-  if (!yt) return;
   __syncthreads();
   for (int i = ty; i < 32; i += 8) {
     const int c = c0 + i, r = r0 + tx;
@@ -554,13 +553,16 @@ __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamArgs a
   }
 }
 
-// Standardised inputs: x = (theta - mean) / scale, FP32.
+// Standardised inputs: x = (theta - mean) / scale, FP32, and (h0 set) the BF16
+// rows of the first GEMM.
 __global__ void k_standardize(const double* __restrict__ theta, int rows, int cols, const float* __restrict__ mean,
-                              const float* __restrict__ scale, float* x) {
+                              const float* __restrict__ scale, float* x, bf16* h0) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)rows * cols) return;
   const int c = (int)(i % cols);
-  x[i] = (float)((theta[i] - (double)mean[c]) / (double)scale[c]);
+  const float z = (float)((theta[i] - (double)mean[c]) / (double)scale[c]);
+  x[i] = z;
+  if (h0) h0[i] = __float2bfloat16(z);
 }
 
 // Surrogate head (device pointers).  The predicted log rate of a bin is
@@ -612,6 +614,8 @@ __device__ __forceinline__ float log_ratio_f(float data, float mc) {
 // engine keeps its FP64 path).  Same formulas as the engine's FP64 ones:
 // Poisson (PoissonLogLikelihood.h:19-53) and Barlow-Beeston OA2021
 // (BarlowBeestonBanff2022.h:150-294), with log(data / mc) from log_ratio_f.
+// The one sum of two products that the compiler could fuse either way is fused
+// explicitly, so that every kernel gives a point the same value.
 __device__ __forceinline__ float llh_term_f(int type, float data, float pred, float sumw2) {
   if (type == GW_LLH_POISSON) {
     if (pred <= 0.f) return INFINITY;
@@ -624,7 +628,7 @@ __device__ __forceinline__ float llh_term_f(int type, float data, float pred, fl
   if (sumw2 > 0.f) {
     const float f2 = sumw2 / (pred * pred);
     const float temp = sumw2 / pred - 1.f;
-    const float temp2 = temp * temp + 4.f * data * f2;
+    const float temp2 = __fmaf_rn(__fmul_rn(4.f, data), f2, __fmul_rn(temp, temp));
     if (temp2 < 0.f) return INFINITY;
     const float beta = 0.5f * (sqrtf(temp2) - temp);
     newmc = fmaxf(pred * beta, FLT_MIN);
@@ -658,7 +662,7 @@ __device__ __forceinline__ void llh_term_grad_f(int type, float data, float pred
   if (sumw2 > 0.f) {
     const float f2 = sumw2 / (pred * pred);
     const float temp = sumw2 / pred - 1.f;
-    const float temp2 = temp * temp + 4.f * data * f2;
+    const float temp2 = __fmaf_rn(temp, temp, __fmul_rn(__fmul_rn(4.f, data), f2));
     if (temp2 < 0.f) return;
     const float beta = 0.5f * (sqrtf(temp2) - temp);
     const float pen = (beta - 1.f) * (beta - 1.f) / f2;
@@ -669,25 +673,203 @@ __device__ __forceinline__ void llh_term_grad_f(int type, float data, float pred
   }
 }
 
-// Head and likelihood terms, fused.  Block (32 bins, 8 point rows); thread
-// (x, y) of block (bx, by) handles bin 32 bx + x and the PPT points
-// by * 8 PPT + y + 8 j.  The block first stages, for each of its points and
-// parameters, the input x and (additive base) the table offset of the
-// interpolation interval and its weight in shared memory; the inner loop is
-// then two coalesced table loads and two FMAs per point and parameter, with
-// the table lines of a bin shared through L1 across the block's points.
-// Per point and block, the 32 bins' terms are summed by a fixed shuffle tree
-// into part[point][bx] (FP64); optional outputs: sums, sums2 (FP64), log rates.
-// GRAD: also, per (point, bin), G = dL/dlog mu + dL/dlog s2 (the derivative
-// with respect to the log rate, the modelled sum of w^2 moving with it) and
-// S = dL/dlog s2 into gbuf / sbuf, and dY = G * sd (the derivative with
-// respect to the network output) as BF16 into dy.
-template <int PPT, bool GRAD = false>
+// Where the head's results go.  sums, sums2 (FP64) and logr are optional.  With
+// G set (value and gradient): per (point, bin), G = dL/dlog mu + dL/dlog s2
+// (the derivative with respect to the log rate, the modelled sum of w^2 moving
+// with it), S = dL/dlog s2, and dY = G * sd (the derivative with respect to the
+// network output) as BF16.
+struct HeadOut {
+  double *part, *sums, *sums2, *logr;
+  float *G, *S;
+  bf16* dy;
+};
+
+// Likelihood term of one (point m, bin) from the base `acc` and the log ratio
+// `racc`, with its optional outputs.
+template <bool GRAD>
+__device__ __forceinline__ double head_term(const Head& h, const float* __restrict__ mlp, int C, int m, int bin,
+                                            const double* __restrict__ data, int llh_type, float acc, float racc,
+                                            const HeadOut& out) {
+  if (bin >= h.nb || m >= C) return 0.0;
+  const size_t o = (size_t)m * h.nb + bin;
+  const float lr = acc + h.mu[bin] + h.sd[bin] * mlp[o];
+  const float mu = expf(lr), s2 = expf(lr + racc);
+  if (out.sums) out.sums[o] = (double)mu;
+  if (out.sums2) out.sums2[o] = (double)s2;
+  if (out.logr) out.logr[o] = (double)lr;
+  if constexpr (GRAD) {
+    float gmu, gs2;
+    llh_term_grad_f(llh_type, (float)data[bin], mu, s2, gmu, gs2);
+    const float G = gmu + gs2;
+    out.G[o] = G;
+    out.S[o] = gs2;
+    out.dy[o] = __float2bfloat16(G * h.sd[bin]);
+  }
+  return (double)llh_term_f(llh_type, (float)data[bin], mu, s2);
+}
+
+// The warp's sum of t by a fixed shuffle tree, into part[m][blockIdx.x] (FP64).
+__device__ __forceinline__ void head_part(double t, int C, int m, double* __restrict__ part) {
+  for (int off = 16; off; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+  if ((threadIdx.x & 31) == 0 && m < C) part[(size_t)m * gridDim.x + blockIdx.x] = t;
+}
+
+// Head and likelihood terms, fused, for a base of few nodes: block of 128
+// threads, 64 bins (a lane: two neighbours, in packed FP32) x 8 points (warp v
+// the points v and v + 4).  The parameters go by in chunks of kHeadK: one TMA
+// box brings the chunk's table rows (every node) and one its r_w rows into a
+// ring of kHeadStages stages (zeros beyond the bins and the parameters); 64
+// threads form the interval and weight of each point and parameter one chunk
+// ahead.  A (point, parameter) step of 64 bins is then three shared-memory loads
+// (five wavefronts, which is what bounds it) and four packed operations.  Reading the table from L1 / L2 in the loop made
+// it a chain of L2 latencies: 67 us for 64 points, 200 parameters and 3000 bins.
+// Staging through registers (32 bins per warp) took 51 us, 27 instructions per
+// step of 32 bins, issue 62 %; this form takes 31 us (256-thread blocks of 16
+// points: 40 us, two of 188 blocks on 36 of the SMs).
+// The base is summed over the parameters in order, as k_head_llh does.
+constexpr int kHeadK = 8;       // parameters per chunk (network widths are multiples of 8)
+constexpr int kHeadNodes = 8;   // nodes a chunk has room for
+constexpr int kHeadStages = 3;
+constexpr int kHeadBins = 64, kHeadPts = 8, kHeadThreads = 128;
+constexpr int kHeadStage = kHeadK * (kHeadNodes + 1) * kHeadBins;  // floats
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void upk2(f32x2 r, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+template <bool GRAD>
+__global__ void __launch_bounds__(kHeadThreads, 3) k_head_staged(const __grid_constant__ CUtensorMap tm_tab,
+                                                        const __grid_constant__ CUtensorMap tm_rw, Head h,
+                                                        const float* __restrict__ x, const float* __restrict__ mlp,
+                                                        int C, const double* __restrict__ data, int llh_type,
+                                                        HeadOut out, uint32_t* status) {
+  extern __shared__ __align__(128) float sh_h[];  // [kHeadStages][kHeadStage]
+  __shared__ float4 s_pt[2][kHeadK][kHeadPts];  // (weight, input, staged row of the interval * kHeadBins, 0)
+  __shared__ __align__(8) uint64_t bar[kHeadStages];
+  const int din = h.din, nb = h.nb, nodes = h.nodes;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int mb = blockIdx.y * kHeadPts, b0 = blockIdx.x * kHeadBins;
+  const float inv_w = (float)(nodes - 1) / (2.f * h.lim);
+  const int nchunk = din / kHeadK;
+  const bool has_rw = h.r_w != nullptr;
+  const uint32_t bytes = (uint32_t)(kHeadK * nodes + (has_rw ? kHeadK : 0)) * kHeadBins * 4u;
+  auto issue = [&](int c) {
+    float* st = sh_h + (c % kHeadStages) * kHeadStage;
+    mbar_arrive_expect(&bar[c % kHeadStages], bytes);
+    tma_load_2d(st, &tm_tab, b0, c * kHeadK * nodes, &bar[c % kHeadStages]);
+    if (has_rw) tma_load_2d(st + kHeadK * kHeadNodes * kHeadBins, &tm_rw, b0, c * kHeadK, &bar[c % kHeadStages]);
+  };
+  if (tid == 0) {
+    for (int i = 0; i < kHeadStages; ++i) mbar_init(&bar[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int c = 0; c < min(nchunk, kHeadStages); ++c) issue(c);
+  }
+  // one (parameter, point) of each chunk per thread of the first two warps
+  const int sk = tid / kHeadPts, sm = tid % kHeadPts;
+  float z = 0.f;
+  auto fetch = [&](int c) {
+    if (sk < kHeadK) {
+      const int k = c * kHeadK + sk;
+      z = mb + sm < C ? x[(size_t)(mb + sm) * din + k] : 0.f;
+    }
+  };
+  auto store = [&](int buf) {
+    if (sk < kHeadK) {
+      const float xc = fminf(fmaxf(z, -h.lim), h.lim);
+      const float u = (xc + h.lim) * inv_w;
+      const int i = min((int)u, nodes - 2);
+      const float t = u - (float)i;
+      s_pt[buf][sk][sm] = make_float4(t, z, __int_as_float((sk * nodes + i) * kHeadBins), 0.f);
+    }
+  };
+  const int bin = b0 + 2 * lane;
+  f32x2 acc[2], racc[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    acc[j] = pk2(bin < nb ? h.b0[bin] : 0.f, bin + 1 < nb ? h.b0[bin + 1] : 0.f);
+    racc[j] = pk2(bin < nb ? h.r_b[bin] : 0.f, bin + 1 < nb ? h.r_b[bin + 1] : 0.f);
+  }
+  fetch(0);
+  store(0);
+  if (nchunk > 1) fetch(1);
+  __syncthreads();
+  for (int c = 0; c < nchunk; ++c) {
+    const int buf = c & 1, st = c % kHeadStages;
+    const bool ok = mbar_wait_bounded(&bar[st], (uint32_t)((c / kHeadStages) & 1));
+    if (c + 1 < nchunk) store(buf ^ 1);  // its readers passed the barrier at the end of chunk c - 1
+    if (c + 2 < nchunk) fetch(c + 2);
+    const float* tab = sh_h + st * kHeadStage + 2 * lane;
+    if (ok) {
+      auto step = [&](int kk) {
+        const f32x2 w = has_rw ? *reinterpret_cast<const f32x2*>(tab + (kHeadK * kHeadNodes + kk) * kHeadBins) : 0ull;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float4 pt = s_pt[buf][kk][warp + 4 * j];
+          const float* row = tab + __float_as_int(pt.z);
+          const f32x2 lo = *reinterpret_cast<const f32x2*>(row);
+          const f32x2 hi = *reinterpret_cast<const f32x2*>(row + kHeadBins);
+          acc[j] = add2(acc[j], fma2(pk2(pt.x, pt.x), sub2(hi, lo), lo));
+          racc[j] = fma2(pk2(pt.y, pt.y), w, racc[j]);
+        }
+      };
+#pragma unroll
+      for (int kk = 0; kk < kHeadK; ++kk) step(kk);  // din is a multiple of kHeadK (gwm_create)
+    }
+    if (__syncthreads_or(!ok)) {
+      if (tid == 0) {
+        atomicOr(status, 1u);
+        // the copies still in flight land before the block exits (bounded)
+        for (int i = c; i < min(nchunk, c + kHeadStages); ++i)
+          mbar_wait_bounded(&bar[i % kHeadStages], (uint32_t)((i / kHeadStages) & 1));
+      }
+      return;
+    }
+    if (tid == 0 && c + kHeadStages < nchunk) issue(c + kHeadStages);
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    float a0, a1, r0, r1;
+    upk2(acc[j], a0, a1);
+    upk2(racc[j], r0, r1);
+    const int m = mb + warp + 4 * j;
+    const double t0 = head_term<GRAD>(h, mlp, C, m, bin, data, llh_type, a0, r0, out);
+    const double t1 = head_term<GRAD>(h, mlp, C, m, bin + 1, data, llh_type, a1, r1, out);
+    head_part(t0 + t1, C, m, out.part);
+  }
+}
+
+// The same for an affine base or one of more nodes than k_head_staged holds.
+// Block (32 bins, 8 point rows); thread (x, y) of block (bx, by) handles bin
+// 32 bx + x and the PPT points by * 8 PPT + y + 8 j.  The block first stages,
+// for each of its points and parameters, the input x and (additive base) the
+// table offset of the interpolation interval and its weight in shared memory;
+// the inner loop is then two coalesced table loads and two FMAs per point and
+// parameter, with the table lines of a bin shared through L1 across the
+// block's points.
+template <int PPT, bool GRAD>
 __global__ void __launch_bounds__(256) k_head_llh(Head h, const float* __restrict__ x, const float* __restrict__ mlp,
-                                                  int C, const double* __restrict__ data, int llh_type,
-                                                  double* __restrict__ part, double* sums, double* sums2,
-                                                  double* logr, float* gbuf = nullptr, float* sbuf = nullptr,
-                                                  bf16* dy = nullptr) {
+                                                  int C, const double* __restrict__ data, int llh_type, HeadOut out) {
   extern __shared__ unsigned char sh_raw[];
   constexpr int NP = 8 * PPT;  // points per block
   const int din = h.din;
@@ -747,27 +929,7 @@ __global__ void __launch_bounds__(256) k_head_llh(Head h, const float* __restric
 #pragma unroll
   for (int j = 0; j < PPT; ++j) {
     const int m = mb + threadIdx.y + 8 * j;
-    float term = 0.f;
-    if (bin_ok && m < C) {
-      const size_t o = (size_t)m * h.nb + bin;
-      const float lr = acc[j] + h.mu[bin] + h.sd[bin] * mlp[o];
-      const float mu = expf(lr), s2 = expf(lr + racc[j]);
-      term = llh_term_f(llh_type, (float)data[bin], mu, s2);
-      if (sums) sums[o] = (double)mu;
-      if (sums2) sums2[o] = (double)s2;
-      if (logr) logr[o] = (double)lr;
-      if constexpr (GRAD) {
-        float gmu, gs2;
-        llh_term_grad_f(llh_type, (float)data[bin], mu, s2, gmu, gs2);
-        const float G = gmu + gs2;
-        gbuf[o] = G;
-        sbuf[o] = gs2;
-        dy[o] = __float2bfloat16(G * h.sd[bin]);
-      }
-    }
-    double t = (double)term;
-    for (int off = 16; off; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
-    if (threadIdx.x == 0 && m < C) part[(size_t)m * gridDim.x + blockIdx.x] = t;
+    head_part(head_term<GRAD>(h, mlp, C, m, bin, data, llh_type, acc[j], racc[j], out), C, m, out.part);
   }
 }
 
@@ -787,13 +949,15 @@ __global__ void k_llh_finish(const double* __restrict__ part, int nblk, int C, d
 //   gz[m][k] = sum_b G[m][b] * d base_b / d x_k + S[m][b] * r_w[k][b]
 // (d base / d x_k: the slope of the interpolation interval of x_k, zero
 // outside [-lim, lim]; affine base: tab[k][b]).  The point's G and S rows are
-// staged in shared memory; fixed-order block reduction.
+// staged in shared memory; fixed-order block reduction: the 8 warps' parts of a
+// (point, parameter) go to gz[m][k][0..7], which k_grad_finish adds in order.
+// The general form, for an affine base or one of more nodes than
+// k_base_grad_staged holds.
 __global__ void __launch_bounds__(256) k_base_grad(Head h, const float* __restrict__ x, const float* __restrict__ G,
                                                    const float* __restrict__ S, float* __restrict__ gz) {
   extern __shared__ float shg[];
   float* g = shg;            // [nb]
   float* sg = shg + h.nb;    // [nb]
-  __shared__ float red[8][8];
   const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int b = tid; b < h.nb; b += 256) {
     g[b] = G[(size_t)m * h.nb + b];
@@ -825,17 +989,159 @@ __global__ void __launch_bounds__(256) k_base_grad(Head h, const float* __restri
       if (rw) acc = fmaf(sg[b], rw[b], acc);
     }
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) red[q][warp] = acc;
+    if (lane == 0) gz[((size_t)m * h.din + k) * 8 + warp] = acc;
   }
-  __syncthreads();
-  if (tid < 8) {
-    const int k = blockIdx.y * 8 + tid;
-    if (k < h.din) {
-      float t = 0.f;
-      for (int w = 0; w < 8; ++w) t += red[tid][w];
-      gz[(size_t)m * h.din + k] = t;
+}
+
+// The same for a base of few nodes, all points of a tile sharing the table.
+// Block (w, bk): the bins 32 w + lane + 256 j (j = 0, 1, ...), those of warp w
+// of k_base_grad, and the parameters [bk, bk + 1) * kGradK; warp v the points
+// 8 v .. 8 v + 7 of each 64-point tile.  Per j, one TMA box brings the kGradK * nodes
+// table rows of the 32 bins and one the r_w rows (zeros beyond the bins and the
+// parameters), kGradStages j ahead, so that the table is read once per 64 points
+// instead of twice per (point, parameter), and no load of it is waited for:
+// 64 points, 200 parameters and 3000 bins took 108 us, bound by the latency of
+// the 460 MB that went through L2; this form takes 33 us (39 us with
+// kGradK = 4).  Each lane's sum over j and the shuffle tree
+// are those of k_base_grad.
+constexpr int kGradK = 8, kGradM = 8, kGradStages = 8;
+constexpr int kGradRows = kGradK * kHeadNodes;
+__global__ void __launch_bounds__(256, 2) k_base_grad_staged(const __grid_constant__ CUtensorMap tm_tab,
+                                                             const __grid_constant__ CUtensorMap tm_rw, Head h,
+                                                             const float* __restrict__ x,
+                                                             const float* __restrict__ G,
+                                                             const float* __restrict__ S, int C,
+                                                             float* __restrict__ gz, uint32_t* status) {
+  extern __shared__ __align__(128) float sh_g[];  // [kGradStages][kGradRows + kGradK][32]
+  constexpr int kStage = (kGradRows + kGradK) * 32;
+  __shared__ int2 s_iv[kGradK][8 * kGradM];  // (staged row of the interval * 32, slope scale)
+  __shared__ __align__(8) uint64_t bar[kGradStages];
+  const int w = blockIdx.x, k0 = blockIdx.y * kGradK, m0 = blockIdx.z * 8 * kGradM;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nb = h.nb, nodes = h.nodes;
+  const int b0 = 32 * w;
+  const int nj = b0 < nb ? (nb - b0 + 255) / 256 : 0;
+  const bool has_rw = h.r_w != nullptr;
+  const uint32_t bytes = (uint32_t)(kGradK * nodes + (has_rw ? kGradK : 0)) * 128u;
+  auto issue = [&](int j) {
+    float* st = sh_g + (j % kGradStages) * kStage;
+    mbar_arrive_expect(&bar[j % kGradStages], bytes);
+    tma_load_2d(st, &tm_tab, b0 + 256 * j, k0 * nodes, &bar[j % kGradStages]);
+    if (has_rw) tma_load_2d(st + kGradRows * 32, &tm_rw, b0 + 256 * j, k0, &bar[j % kGradStages]);
+  };
+  if (tid == 0) {
+    for (int i = 0; i < kGradStages; ++i) mbar_init(&bar[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int j = 0; j < min(nj, kGradStages); ++j) issue(j);
+  }
+  const float inv_w = (float)(nodes - 1) / (2.f * h.lim);
+  for (int e = tid; e < kGradK * 8 * kGradM; e += 256) {
+    const int q = e / (8 * kGradM), mm = e % (8 * kGradM);
+    const int k = min(k0 + q, h.din - 1), m = min(m0 + mm, C - 1);
+    const float z = x[(size_t)m * h.din + k];
+    const float xc = fminf(fmaxf(z, -h.lim), h.lim);
+    const float u = (xc + h.lim) * inv_w;
+    const int i = min((int)u, nodes - 2);
+    s_iv[q][mm] = make_int2((q * nodes + i) * 32, __float_as_int((z > -h.lim && z < h.lim) ? inv_w : 0.f));
+  }
+  float acc[kGradK][kGradM];
+#pragma unroll
+  for (int q = 0; q < kGradK; ++q)
+#pragma unroll
+    for (int j = 0; j < kGradM; ++j) acc[q][j] = 0.f;
+  const int mw = m0 + warp * kGradM;  // this warp's first point
+  float g[kGradM], sg[kGradM];
+  auto load_gs = [&](int j) {
+    const int b = b0 + 256 * j + lane;
+#pragma unroll
+    for (int i = 0; i < kGradM; ++i) {
+      const bool in = b < nb && mw + i < C;
+      const size_t o = (size_t)(mw + i) * nb + b;
+      g[i] = in ? G[o] : 0.f;
+      sg[i] = in ? S[o] : 0.f;
     }
+  };
+  if (nj > 0) load_gs(0);
+  bool failed = false;
+  __syncthreads();
+  for (int j = 0; j < nj; ++j) {
+    const int st = j % kGradStages;
+    const bool ok = mbar_wait_bounded(&bar[st], (uint32_t)((j / kGradStages) & 1));
+    if (__syncthreads_or(!ok)) {
+      failed = true;
+      if (tid == 0) {
+        atomicOr(status, 1u);
+        // the copies still in flight land before the block exits (bounded)
+        for (int i = j; i < min(nj, j + kGradStages); ++i)
+          mbar_wait_bounded(&bar[i % kGradStages], (uint32_t)((i / kGradStages) & 1));
+      }
+      break;
+    }
+    const float* tab = sh_g + st * kStage + lane;
+    float cg[kGradM], cs[kGradM];
+#pragma unroll
+    for (int i = 0; i < kGradM; ++i) {
+      cg[i] = g[i];
+      cs[i] = sg[i];
+    }
+    if (j + 1 < nj) load_gs(j + 1);
+    if (b0 + 256 * j + lane < nb) {
+#pragma unroll
+      for (int q = 0; q < kGradK; ++q) {
+        const float rw = has_rw ? tab[(kGradRows + q) * 32] : 0.f;
+#pragma unroll
+        for (int i = 0; i < kGradM; ++i) {
+          const int2 iv = s_iv[q][warp * kGradM + i];
+          const float lo = tab[iv.x], hi = tab[iv.x + 32];
+          const float slope = (hi - lo) * __int_as_float(iv.y);
+          acc[q][i] = fmaf(cg[i], slope, acc[q][i]);
+          if (has_rw) acc[q][i] = fmaf(cs[i], rw, acc[q][i]);
+        }
+      }
+    }
+    __syncthreads();
+    if (tid == 0 && j + kGradStages < nj) issue(j + kGradStages);
   }
+  if (failed) return;
+#pragma unroll
+  for (int q = 0; q < kGradK; ++q)
+#pragma unroll
+    for (int i = 0; i < kGradM; ++i) {
+      float t = acc[q][i];
+      for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0 && k0 + q < h.din && mw + i < C) gz[((size_t)(mw + i) * h.din + k0 + q) * 8 + w] = t;
+    }
+}
+
+// Columns [k0, k1) of a mat-vec by one thread: sum_k A[k][p] d[k] with A
+// [. x P] row-major, N partial sums in turn, sixteen loads in flight (a load at
+// a time made the penalty and the proposal chains of L2 latencies: 27 us per
+// launch at P = 200, now 10-14 us).
+template <int N>
+__device__ __forceinline__ void column_sum(const float* __restrict__ A, int P, int p, const float* __restrict__ d,
+                                           int k0, int k1, float (&u)[N]) {
+#pragma unroll
+  for (int q = 0; q < N; ++q) u[q] = 0.f;
+  int k = k0;
+  for (; k + 16 <= k1; k += 16) {
+    float c[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) c[q] = __ldg(A + (size_t)(k + q) * P + p);
+#pragma unroll
+    for (int q = 0; q < 16; ++q) u[q % N] = fmaf(c[q], d[k + q], u[q % N]);
+  }
+  for (; k + N <= k1; k += N)
+#pragma unroll
+    for (int q = 0; q < N; ++q) u[q] = fmaf(__ldg(A + (size_t)(k + q) * P + p), d[k + q], u[q]);
+  for (; k < k1; ++k) u[0] = fmaf(__ldg(A + (size_t)k * P + p), d[k], u[0]);
+}
+
+// Sum of red [n] in FP64 by one warp, a fixed order; the result on every lane.
+__device__ __forceinline__ double warp_sum(const float* red, int n) {
+  double t = 0.0;
+  for (int i = threadIdx.x & 31; i < n; i += 32) t += (double)red[i];
+  for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
 }
 
 // Per point (block), G groups of P32 threads as k_finish_accept: the value
@@ -864,15 +1170,9 @@ __global__ void k_grad_finish(const double* __restrict__ part, int nblk, const d
     __syncthreads();
     const int ks = (P + Gn - 1) / Gn;
     if (p < P) {
-      const int k0 = g * ks, k1 = min(P, (g + 1) * ks);
-      float u0 = 0.f, u1 = 0.f;
-      int k = k0;
-      for (; k + 2 <= k1; k += 2) {
-        u0 = fmaf(icov[(size_t)k * P + p], d[k], u0);
-        u1 = fmaf(icov[(size_t)(k + 1) * P + p], d[k + 1], u1);
-      }
-      for (; k < k1; ++k) u0 = fmaf(icov[(size_t)k * P + p], d[k], u0);
-      up[g * P32 + p] = u0 + u1;
+      float u[2];
+      column_sum<2>(icov, P, p, d, g * ks, min(P, (g + 1) * ks), u);
+      up[g * P32 + p] = u[0] + u[1];
     }
     __syncthreads();
   }
@@ -883,15 +1183,16 @@ __global__ void k_grad_finish(const double* __restrict__ part, int nblk, const d
     red[p] = m ? d[p] * u : 0.f;
     if (p < P) {
       const size_t o = (size_t)c * P + p;
-      grad[o] = (double)((gz[o] + dx[o]) / scale[p]) + (m ? 2.0 * (double)u : 0.0);
+      float gs = 0.f;  // the parts of k_base_grad, in order
+#pragma unroll
+      for (int w = 0; w < 8; ++w) gs += gz[o * 8 + w];
+      grad[o] = (double)((gs + dx[o]) / scale[p]) + (m ? 2.0 * (double)u : 0.0);
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double pen = 0.0;
-    if (m)
-      for (int i = 0; i < P32; ++i) pen += (double)red[i];
-    f[c] = s_llh + pen;
+  if (threadIdx.x < 32) {
+    const double pen = m ? warp_sum(red, P32) : 0.0;
+    if (lane == 0) f[c] = s_llh + pen;
   }
 }
 
@@ -1023,6 +1324,22 @@ static int make_map(gwm_net* n, CUtensorMap* map, const bf16* p, int rows, int K
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)p, dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return gwm_fail(n, GW_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+  return GW_OK;
+}
+
+// Tensor map of a row-major FP32 matrix [rows x cols] (cols % 4 == 0) read in
+// boxes of box_cols x box_rows, zero fill.
+static int make_map_f32(gwm_net* n, CUtensorMap* map, const float* p, int rows, int cols, int box_cols, int box_rows) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) return gwm_fail(n, GW_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)cols * 4};
+  const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)p, dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return gwm_fail(n, GW_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   return GW_OK;
@@ -1249,10 +1566,10 @@ static int forward(gwm_net* n, int B, Keep keep, const Loss* loss = nullptr) {
 static dim3 tiles32(int rows, int cols) { return dim3((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32)); }
 
 // Input rows to BF16 (and transposed) for the first GEMM; row r is perm[r] of x (perm null: r).
-// The transposed copy feeds the weight gradient of the first layer only.
-static int stage_input(gwm_net* n, const float* x, const int32_t* perm, int B, bool transposed = true) {
+// The transposed copy feeds the weight gradient of the first layer.
+static int stage_input(gwm_net* n, const float* x, const int32_t* perm, int B) {
   gwm::k_rows_to_bf16<<<tiles32(B, n->dims[0]), dim3(32, 8), 0, n->stream>>>(
-      x, perm, B, n->dims[0], n->h[0], transposed ? n->ht[0] : nullptr, B);
+      x, perm, B, n->dims[0], n->h[0], n->ht[0], B);
   GWM_CUDA(n, cudaGetLastError());
   return GW_OK;
 }
@@ -1499,25 +1816,101 @@ extern "C" int gwm_set_head_additive(gwm_net* n, const float* in_mean, const flo
   return head_common(n, in_mean, in_scale, base_b, out_mu, out_sd, ratio_w, data);
 }
 
+// Tensor maps of the base table and of r_w in boxes of box_cols bins x
+// box_params parameters.
+static int head_maps(gwm_net* n, CUtensorMap* tab, CUtensorMap* rw, int box_cols, int box_params) {
+  const int din = n->dims[0], nb = n->dims[n->n_layers];
+  const int rc = make_map_f32(n, tab, n->h_tab, din * n->h_nodes, nb, box_cols, box_params * n->h_nodes);
+  return rc ? rc : make_map_f32(n, rw, n->h_rw, din, nb, box_cols, box_params);
+}
+
+// A base whose tables the staged kernels hold (k_head_staged, k_base_grad_staged).
+static bool head_staged(const gwm_net* n) { return n->h_nodes >= 2 && n->h_nodes <= gwm::kHeadNodes; }
+
+// Likelihood partials per point: one per block of bins.
+static int head_parts(const gwm_net* n) {
+  const int nb = n->dims[n->n_layers], w = head_staged(n) ? gwm::kHeadBins : 32;
+  return (nb + w - 1) / w;
+}
+
+template <bool GRAD>
+static int launch_head(gwm_net* n, int C, int llh_type, const gwm::HeadOut& out) {
+  const int L = n->n_layers;
+  constexpr int kPPT = 2;
+  const size_t shm = (size_t)8 * kPPT * n->dims[0] * 12;
+  if (shm > 200 * 1024) return gwm_fail(n, GW_ERR_LIMIT, "surrogate head: too many inputs");
+  if (head_staged(n)) {
+    CUtensorMap tab, rw;
+    const int rc = head_maps(n, &tab, &rw, gwm::kHeadBins, gwm::kHeadK);
+    if (rc) return rc;
+    constexpr int kShm = gwm::kHeadStages * gwm::kHeadStage * 4;
+    static std::once_flag once;
+    std::call_once(once, []() {
+      cudaFuncSetAttribute(gwm::k_head_staged<GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kShm);
+    });
+    const dim3 grid(head_parts(n), (C + gwm::kHeadPts - 1) / gwm::kHeadPts);
+    gwm::k_head_staged<GRAD><<<grid, gwm::kHeadThreads, kShm, n->stream>>>(
+        tab, rw, head_view(n), n->xin, n->z[L - 1], C, n->h_data, llh_type, out, n->status);
+  } else {
+    if (shm > 48 * 1024) {
+      static std::once_flag once;
+      std::call_once(once, []() {
+        cudaFuncSetAttribute(gwm::k_head_llh<kPPT, GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      });
+    }
+    const dim3 grid(head_parts(n), (C + 8 * kPPT - 1) / (8 * kPPT));
+    gwm::k_head_llh<kPPT, GRAD><<<grid, dim3(32, 8), shm, n->stream>>>(head_view(n), n->xin, n->z[L - 1], C,
+                                                                       n->h_data, llh_type, out);
+  }
+  GWM_CUDA(n, cudaGetLastError());
+  return GW_OK;
+}
+
+// The base's part of the input gradient, eight parts per (point, parameter) in g_gz.
+static int launch_base_grad(gwm_net* n, int C) {
+  const int din = n->dims[0], nb = n->dims[n->n_layers];
+  const size_t shb = sizeof(float) * 2 * (size_t)nb;
+  if (shb > 200 * 1024) return gwm_fail(n, GW_ERR_LIMIT, "gwm_value_grad: too many bins");
+  if (head_staged(n)) {
+    CUtensorMap tab, rw;
+    const int rc = head_maps(n, &tab, &rw, 32, gwm::kGradK);
+    if (rc) return rc;
+    constexpr int kShm = gwm::kGradStages * (gwm::kGradRows + gwm::kGradK) * 32 * 4;
+    static std::once_flag once;
+    std::call_once(once, []() {
+      cudaFuncSetAttribute(gwm::k_base_grad_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, kShm);
+    });
+    constexpr int kTile = 8 * gwm::kGradM;
+    const dim3 grid(8, (din + gwm::kGradK - 1) / gwm::kGradK, (C + kTile - 1) / kTile);
+    gwm::k_base_grad_staged<<<grid, 256, kShm, n->stream>>>(tab, rw, head_view(n), n->xin, n->g_G, n->g_S, C,
+                                                            n->g_gz, n->status);
+  } else {
+    if (shb > 48 * 1024) {
+      static std::once_flag once;
+      std::call_once(once, []() {
+        cudaFuncSetAttribute(gwm::k_base_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      });
+    }
+    gwm::k_base_grad<<<dim3(C, (din + 7) / 8), 256, shb, n->stream>>>(head_view(n), n->xin, n->g_G, n->g_S, n->g_gz);
+  }
+  GWM_CUDA(n, cudaGetLastError());
+  return GW_OK;
+}
+
 // Fused head + likelihood of the first C rows of the network's output (xin
 // holds their standardised inputs): h_llh [C]; with `outputs`, h_sums,
 // h_sums2 and h_logr too.
 static int head_llh(gwm_net* n, int C, int llh_type, bool outputs, bool finish = true) {
-  const int nb = n->dims[n->n_layers], L = n->n_layers;
-  constexpr int kPPT = 2;
-  const int nbx = (nb + 31) / 32;
-  dim3 grid(nbx, (C + 8 * kPPT - 1) / (8 * kPPT));
-  const size_t shm = (size_t)8 * kPPT * n->dims[0] * 12;
-  if (shm > 48 * 1024) {
-    static std::once_flag once;
-    std::call_once(once, []() {
-      cudaFuncSetAttribute(gwm::k_head_llh<kPPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    });
-    if (shm > 200 * 1024) return gwm_fail(n, GW_ERR_LIMIT, "surrogate head: too many inputs");
+  gwm::HeadOut out{};
+  out.part = n->h_part;
+  if (outputs) {
+    out.sums = n->h_sums;
+    out.sums2 = n->h_sums2;
+    out.logr = n->h_logr;
   }
-  gwm::k_head_llh<kPPT><<<grid, dim3(32, 8), shm, n->stream>>>(
-      head_view(n), n->xin, n->z[L - 1], C, n->h_data, llh_type, n->h_part, outputs ? n->h_sums : nullptr,
-      outputs ? n->h_sums2 : nullptr, outputs ? n->h_logr : nullptr);
+  const int rc = launch_head<false>(n, C, llh_type, out);
+  if (rc) return rc;
+  const int nbx = head_parts(n);
   if (finish) gwm::k_llh_finish<<<(C + 7) / 8, 256, 0, n->stream>>>(n->h_part, nbx, C, n->h_llh);
   GWM_CUDA(n, cudaGetLastError());
   return GW_OK;
@@ -1535,12 +1928,10 @@ extern "C" int gwm_predict(gwm_net* n, const double* theta, int32_t B, int32_t l
   if (Bp > n->batch_max) return gwm_fail(n, GW_ERR_ARG, "gwm_predict: batch above batch_max after padding");
   if (Bp > B) GWM_CUDA(n, cudaMemsetAsync(n->h_theta, 0, sizeof(double) * (size_t)Bp * din, n->stream));
   GWM_CUDA(n, cudaMemcpyAsync(n->h_theta, theta, sizeof(double) * (size_t)B * din, cudaMemcpyHostToDevice, n->stream));
-  gwm::k_standardize<<<(unsigned)(((size_t)Bp * din + 255) / 256), 256, 0, n->stream>>>(n->h_theta, Bp, din,
-                                                                                     n->h_mean, n->h_scale, n->xin);
-  int rc = stage_input(n, n->xin, nullptr, Bp, false);
-  if (rc) return rc;
+  gwm::k_standardize<<<(unsigned)(((size_t)Bp * din + 255) / 256), 256, 0, n->stream>>>(
+      n->h_theta, Bp, din, n->h_mean, n->h_scale, n->xin, n->h[0]);
   GWM_CUDA(n, cudaGetLastError());
-  rc = forward(n, Bp, kKeepNone);
+  int rc = forward(n, Bp, kKeepNone);
   if (rc) return rc;
   rc = head_llh(n, B, llh_type, log_rates != nullptr);
   if (rc) return rc;
@@ -1586,8 +1977,8 @@ extern "C" int gwm_train_size(gwm_net* n, int64_t* count) {
 static int append_rows(gwm_net* n, int K) {
   const int din = n->dims[0], nb = n->dims[n->n_layers];
   float* x = n->train_x + (size_t)n->train_n * din;
-  gwm::k_standardize<<<(unsigned)(((size_t)K * din + 255) / 256), 256, 0, n->stream>>>(n->h_theta, K, din, n->h_mean,
-                                                                                    n->h_scale, x);
+  gwm::k_standardize<<<(unsigned)(((size_t)K * din + 255) / 256), 256, 0, n->stream>>>(
+      n->h_theta, K, din, n->h_mean, n->h_scale, x, nullptr);
   gwm::k_target<<<dim3((nb + 255) / 256, K), 256, 0, n->stream>>>(head_view(n), x, n->h_sums,
                                                                   n->train_t + (size_t)n->train_n * nb);
   GWM_CUDA(n, cudaGetLastError());
@@ -1781,17 +2172,9 @@ __global__ void k_propose_stage(const double* __restrict__ phi, int P, const flo
   const int g = threadIdx.x / P32, p = threadIdx.x - g * P32;
   const int ks = (P + G - 1) / G;
   if (p < P) {
-    const int k0 = g * ks, k1 = min(min(P, (g + 1) * ks), p + 1);
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-    int k = k0;
-    for (; k + 4 <= k1; k += 4) {
-      a0 = fmaf(Lt[(size_t)k * P + p], nrm[k], a0);
-      a1 = fmaf(Lt[(size_t)(k + 1) * P + p], nrm[k + 1], a1);
-      a2 = fmaf(Lt[(size_t)(k + 2) * P + p], nrm[k + 2], a2);
-      a3 = fmaf(Lt[(size_t)(k + 3) * P + p], nrm[k + 3], a3);
-    }
-    for (; k < k1; ++k) a0 = fmaf(Lt[(size_t)k * P + p], nrm[k], a0);
-    part[g * P32 + p] = (a0 + a1) + (a2 + a3);
+    float a[4];
+    column_sum<4>(Lt, P, p, nrm, g * ks, min(min(P, (g + 1) * ks), p + 1), a);
+    part[g * P32 + p] = (a[0] + a[1]) + (a[2] + a[3]);
   }
   __syncthreads();
   if (g == 0 && p < P) {
@@ -1838,17 +2221,9 @@ __global__ void k_finish_accept(const double* __restrict__ part, int nblk, const
     __syncthreads();
     const int ks = (P + G - 1) / G;
     if (p < P) {
-      const int k0 = g * ks, k1 = min(P, (g + 1) * ks);
-      float u0 = 0.f, u1 = 0.f, u2 = 0.f, u3 = 0.f;
-      int k = k0;
-      for (; k + 4 <= k1; k += 4) {
-        u0 = fmaf(icov[(size_t)k * P + p], d[k], u0);
-        u1 = fmaf(icov[(size_t)(k + 1) * P + p], d[k + 1], u1);
-        u2 = fmaf(icov[(size_t)(k + 2) * P + p], d[k + 2], u2);
-        u3 = fmaf(icov[(size_t)(k + 3) * P + p], d[k + 3], u3);
-      }
-      for (; k < k1; ++k) u0 = fmaf(icov[(size_t)k * P + p], d[k], u0);
-      up[g * P32 + p] = (u0 + u1) + (u2 + u3);
+      float u[4];
+      column_sum<4>(icov, P, p, d, g * ks, min(P, (g + 1) * ks), u);
+      up[g * P32 + p] = (u[0] + u[1]) + (u[2] + u[3]);
     }
     __syncthreads();
     if (g == 0) {
@@ -1858,10 +2233,9 @@ __global__ void k_finish_accept(const double* __restrict__ part, int nblk, const
     }
   }
   __syncthreads();
+  double pen = 0.0;
+  if (m && threadIdx.x < 32) pen = warp_sum(red, P32);
   if (threadIdx.x == 0) {
-    double pen = 0.0;
-    if (m)
-      for (int i = 0; i < P32; ++i) pen += (double)red[i];
     const double fn = s_llh + pen;
     int take;
     if (first) {
@@ -1912,10 +2286,10 @@ static void chain_free(gwm_chain_state* s) {
 static int surrogate_llh_device(gwm_net* n, int C, int llh_type) {
   const int din = n->dims[0];
   const int Bp = ((C + 7) / 8) * 8;
-  gwm::k_standardize<<<(unsigned)(((size_t)Bp * din + 255) / 256), 256, 0, n->stream>>>(n->h_theta, Bp, din,
-                                                                                     n->h_mean, n->h_scale, n->xin);
-  int rc = stage_input(n, n->xin, nullptr, Bp, false);
-  if (!rc) rc = forward(n, Bp, kKeepNone);
+  gwm::k_standardize<<<(unsigned)(((size_t)Bp * din + 255) / 256), 256, 0, n->stream>>>(
+      n->h_theta, Bp, din, n->h_mean, n->h_scale, n->xin, n->h[0]);
+  GWM_CUDA(n, cudaGetLastError());
+  const int rc = forward(n, Bp, kKeepNone);
   if (rc) return rc;
   return head_llh(n, C, llh_type, false, false);
 }
@@ -1993,7 +2367,7 @@ extern "C" int gwm_substeps(gwm_net* n, const double* theta0, const double* f0, 
   if (Bp > C)
     GWM_CUDA(n, cudaMemsetAsync(n->h_theta + (size_t)C * P, 0, sizeof(double) * (size_t)(Bp - C) * P, n->stream));
   int rc = GW_OK;
-  const int nbx = (n->dims[n->n_layers] + 31) / 32;
+  const int nbx = head_parts(n);
   const size_t sh_fin = sizeof(float) * ((size_t)P32 * (G + 2));
   if (f0) {
     GWM_CUDA(n, cudaMemcpyAsync(s->f, f0, sizeof(double) * C, cudaMemcpyHostToDevice, n->stream));
@@ -2056,45 +2430,31 @@ extern "C" int gwm_value_grad(gwm_net* n, const double* theta, int32_t C, int32_
   if (Bp > Bm) return gwm_fail(n, GW_ERR_ARG, "gwm_value_grad: batch above batch_max after padding");
   if (!n->g_G) {
     int rc = gwm_alloc(n, &n->g_G, (size_t)Bm * nb) | gwm_alloc(n, &n->g_S, (size_t)Bm * nb) |
-             gwm_alloc(n, &n->g_gz, (size_t)Bm * din) | gwm_alloc(n, &n->g_dx, (size_t)Bm * din) |
+             gwm_alloc(n, &n->g_gz, (size_t)Bm * din * 8) | gwm_alloc(n, &n->g_dx, (size_t)Bm * din) |
              gwm_alloc(n, &n->g_f, Bm) | gwm_alloc(n, &n->g_grad, (size_t)Bm * din);
     if (rc) return rc;
   }
   if (Bp > C) GWM_CUDA(n, cudaMemsetAsync(n->h_theta, 0, sizeof(double) * (size_t)Bp * din, n->stream));
   GWM_CUDA(n, cudaMemcpyAsync(n->h_theta, theta, sizeof(double) * (size_t)C * din, cudaMemcpyHostToDevice, n->stream));
-  gwm::k_standardize<<<(unsigned)(((size_t)Bp * din + 255) / 256), 256, 0, n->stream>>>(n->h_theta, Bp, din,
-                                                                                     n->h_mean, n->h_scale, n->xin);
-  int rc = stage_input(n, n->xin, nullptr, Bp, false);
-  if (!rc) rc = forward(n, Bp, kKeepZ);
-  if (rc) return rc;
-  // the head: likelihood partials, G, S and dY (rows C..Bp of dY stay zero)
-  GWM_CUDA(n, cudaMemsetAsync(n->dz[L - 1], 0, sizeof(bf16) * (size_t)Bp * nb, n->stream));
-  constexpr int kPPT = 2;
-  const int nbx = (nb + 31) / 32;
-  const size_t shm = (size_t)8 * kPPT * din * 12;
-  if (shm > 48 * 1024) {
-    static std::once_flag once;
-    std::call_once(once, []() {
-      cudaFuncSetAttribute(gwm::k_head_llh<kPPT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    });
-    if (shm > 200 * 1024) return gwm_fail(n, GW_ERR_LIMIT, "surrogate head: too many inputs");
-  }
-  gwm::k_head_llh<kPPT, true><<<dim3(nbx, (C + 8 * kPPT - 1) / (8 * kPPT)), dim3(32, 8), shm, n->stream>>>(
-      head_view(n), n->xin, n->z[L - 1], C, n->h_data, llh_type, n->h_part, nullptr, nullptr, nullptr, n->g_G,
-      n->g_S, n->dz[L - 1]);
+  gwm::k_standardize<<<(unsigned)(((size_t)Bp * din + 255) / 256), 256, 0, n->stream>>>(
+      n->h_theta, Bp, din, n->h_mean, n->h_scale, n->xin, n->h[0]);
   GWM_CUDA(n, cudaGetLastError());
-  rc = backward_dx(n, Bp);
+  int rc = forward(n, Bp, kKeepZ);
   if (rc) return rc;
-  const size_t shb = sizeof(float) * 2 * (size_t)nb;
-  if (shb > 48 * 1024) {
-    if (shb > 200 * 1024) return gwm_fail(n, GW_ERR_LIMIT, "gwm_value_grad: too many bins");
-    static std::once_flag once2;
-    std::call_once(once2, []() {
-      cudaFuncSetAttribute(gwm::k_base_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    });
-  }
-  gwm::k_base_grad<<<dim3(C, (din + 7) / 8), 256, shb, n->stream>>>(head_view(n), n->xin, n->g_G, n->g_S, n->g_gz);
-  GWM_CUDA(n, cudaGetLastError());
+  // the head: likelihood partials, G, S and dY (rows C..Bp of dY are zero)
+  if (Bp > C)
+    GWM_CUDA(n, cudaMemsetAsync(n->dz[L - 1] + (size_t)C * nb, 0, sizeof(bf16) * (size_t)(Bp - C) * nb, n->stream));
+  const int nbx = head_parts(n);
+  gwm::HeadOut out{};
+  out.part = n->h_part;
+  out.G = n->g_G;
+  out.S = n->g_S;
+  out.dy = n->dz[L - 1];
+  rc = launch_head<true>(n, C, llh_type, out);
+  if (!rc) rc = backward_dx(n, Bp);
+  if (rc) return rc;
+  rc = launch_base_grad(n, C);
+  if (rc) return rc;
   const int P32 = (din + 31) & ~31;
   const int Gn = std::max(1, std::min(4, 1024 / P32));
   const bool prior = n->chain && n->chain->prior;
