@@ -123,9 +123,15 @@ __global__ void __launch_bounds__(256) k_params(const DevView v, const double* _
   }
 }
 
-// Device table functions: one thread per (entry, point).
+// Device table functions: one thread per (entry, kTabPts points), the points on
+// grid.z.  The FP64 sine and divisions are what it costs, and an SM issues a
+// warp of them every 16 cycles: with one thread per entry for all points, the
+// 4096 entries of a kriging table kept 16 SMs busy (511 us at 100 points); the
+// points spread them over the chip, and the logarithm of the entry's node is
+// taken once per kTabPts points.
+constexpr int kTabPts = 4;
 template <typename T>
-__global__ void k_table_fn(const DevView v, int K) {
+__global__ void __launch_bounds__(128) k_table_fn(const DevView v, int K) {
   const TableFn fn = v.table_fns[blockIdx.y];
   const TableDesc td = v.tables[fn.table];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -133,14 +139,16 @@ __global__ void k_table_fn(const DevView v, int K) {
   const T* xs = (const T*)v.x;
   const double E = v.table_nodes[fn.nodes + j];
   T* arena = (T*)v.table_arena;
-  for (int k = 0; k < K; ++k) {
+  const double logE = fn.kind == 1 ? log(E) : 0.0;
+  const int k0 = blockIdx.z * kTabPts, k1 = min(K, k0 + kTabPts);
+  for (int k = k0; k < k1; ++k) {
     double q[6];
 #pragma unroll
     for (int i = 0; i < 6; ++i) q[i] = (double)xs[(size_t)fn.par[i] * v.kpad + k];
     double val = 1.0;
     if (fn.kind == 1) {
       const double s = sin(q[1] * 1.267 / E + q[2]);
-      val = 1.0 - q[0] * s * s * (1.0 + q[3] * (log(E) - q[4])) * q[5];
+      val = 1.0 - q[0] * s * s * (1.0 + q[3] * (logE - q[4])) * q[5];
     }
     arena[td.offset + (int64_t)j * v.kpad + k] = (T)val;
   }
@@ -696,13 +704,13 @@ cudaError_t launch_params(const DevView& v, const double* params, int K, cudaStr
 
 cudaError_t launch_table_fns(const DevView& v, int K, int max_size, cudaStream_t s) {
   if (v.n_table_fns == 0) return cudaSuccess;
-  dim3 grid((max_size + 255) / 256, v.n_table_fns);
+  const dim3 grid((max_size + 127) / 128, v.n_table_fns, (K + kTabPts - 1) / kTabPts);
   if (v.precision == 2)
-    k_table_fn<dfloat><<<grid, 256, 0, s>>>(v, K);
+    k_table_fn<dfloat><<<grid, 128, 0, s>>>(v, K);
   else if (v.precision)
-    k_table_fn<float><<<grid, 256, 0, s>>>(v, K);
+    k_table_fn<float><<<grid, 128, 0, s>>>(v, K);
   else
-    k_table_fn<double><<<grid, 256, 0, s>>>(v, K);
+    k_table_fn<double><<<grid, 128, 0, s>>>(v, K);
   return cudaGetLastError();
 }
 
