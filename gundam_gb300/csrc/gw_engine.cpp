@@ -105,12 +105,13 @@ struct gw_engine {
   int max_fn_table = 0;
   std::vector<void*> dev_allocs;  // owned device allocations
   void* d_params = nullptr;
-  void* d_sums = nullptr;
-  void* d_sums2 = nullptr;
-  void* d_llh = nullptr;
-  void* d_llh_stat = nullptr;
+  // one evaluation's results in one block, so that they travel in one copy: the
+  // status word (kOutHead bytes), then FP64 llh [K], statistical llh [K], sums
+  // [K x B], sums of squares [K x B]
+  void* d_out = nullptr;
   void* d_evw = nullptr;
-  PinnedBuf h_params, h_sums, h_sums2, h_llh, h_llh_stat, h_status;
+  PinnedBuf h_params, h_out, h_status;
+  cudaEvent_t out_part[4] = {nullptr, nullptr, nullptr, nullptr};
   bool copy_weights = false;
   bool weights_valid = false;
   bool use_graph = false;
@@ -146,6 +147,8 @@ struct gw_engine {
       cudaEventDestroy(pe.second);
     }
     if (chain_done) cudaEventDestroy(chain_done);
+    for (cudaEvent_t ev : out_part)
+      if (ev) cudaEventDestroy(ev);
     for (void* p : dev_allocs) cudaFree(p);
     if (stream) cudaStreamDestroy(stream);
   }
@@ -204,6 +207,15 @@ static int chain_end(gw_engine* e, cudaStream_t s) {
   e->chain_any = true;
   return GW_OK;
 }
+
+// Byte offsets of a K-point evaluation's results in the result block.
+constexpr size_t kOutHead = 64;
+struct OutLayout {
+  size_t llh, stat, sums, sums2, end;
+  OutLayout(size_t K, size_t B)
+      : llh(kOutHead), stat(llh + 8 * K), sums(stat + 8 * K), sums2(sums + 8 * K * B), end(sums2 + 8 * K * B) {}
+  double* at(void* block, size_t off) const { return (double*)((char*)block + off); }
+};
 
 static bool par_ok(const gw_engine* e, int32_t p) { return p >= 0 && p < e->cfg.n_params; }
 static bool res_ok(const gw_engine* e, int32_t r) { return r >= 0 && r < e->cfg.n_results; }
@@ -1351,20 +1363,15 @@ int build_and_upload(gw_engine* e) {
   if ((rc = alloc(sizeof(unsigned int) * kpad, &p))) return rc;
   GW_CUDA(e, cudaMemset(p, 0, sizeof(unsigned int) * kpad));
   v.llh_counter = (unsigned int*)p;
-  if ((rc = alloc(sizeof(uint32_t), &p))) return rc;
-  GW_CUDA(e, cudaMemset(p, 0, sizeof(uint32_t)));
-  v.status = (uint32_t*)p;
   // evaluation I/O buffers
   if ((rc = alloc(sizeof(double) * (size_t)kpad * P, &e->d_params))) return rc;
-  if ((rc = alloc(sizeof(double) * (size_t)kpad * B, &e->d_sums))) return rc;
-  if ((rc = alloc(sizeof(double) * (size_t)kpad * B, &e->d_sums2))) return rc;
-  if ((rc = alloc(sizeof(double) * (size_t)kpad, &e->d_llh))) return rc;
-  if ((rc = alloc(sizeof(double) * (size_t)kpad, &e->d_llh_stat))) return rc;
+  const size_t out_bytes = kOutHead + sizeof(double) * 2 * (size_t)kpad * ((size_t)B + 1);
+  if ((rc = alloc(out_bytes, &e->d_out))) return rc;
+  GW_CUDA(e, cudaMemset(e->d_out, 0, kOutHead));
+  v.status = (uint32_t*)e->d_out;
+  for (cudaEvent_t& ev : e->out_part) GW_CUDA(e, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   GW_CUDA(e, cudaMallocHost(&e->h_params.p, sizeof(double) * (size_t)kpad * P));
-  GW_CUDA(e, cudaMallocHost(&e->h_sums.p, sizeof(double) * (size_t)kpad * B));
-  GW_CUDA(e, cudaMallocHost(&e->h_sums2.p, sizeof(double) * (size_t)kpad * B));
-  GW_CUDA(e, cudaMallocHost(&e->h_llh.p, sizeof(double) * (size_t)kpad));
-  GW_CUDA(e, cudaMallocHost(&e->h_llh_stat.p, sizeof(double) * (size_t)kpad));
+  GW_CUDA(e, cudaMallocHost(&e->h_out.p, out_bytes));
   GW_CUDA(e, cudaMallocHost(&e->h_status.p, sizeof(uint32_t)));
 
   // layout facts
@@ -1495,10 +1502,8 @@ static int launch_chain(gw_engine* e, const double* d_params, int K, double* d_s
   return GW_OK;
 }
 
-static int check_status(gw_engine* e) {
-  GW_CUDA(e, cudaMemcpyAsync(e->h_status.p, e->view.status, sizeof(uint32_t), cudaMemcpyDeviceToHost, e->stream));
-  GW_CUDA(e, cudaStreamSynchronize(e->stream));
-  const uint32_t st = *(uint32_t*)e->h_status.p;
+// The status word of finished work: clears it and reports the error it names.
+static int report_status(gw_engine* e, uint32_t st) {
   if (st) {
     GW_CUDA(e, cudaMemsetAsync(e->view.status, 0, sizeof(uint32_t), e->stream));
     GW_CUDA(e, cudaStreamSynchronize(e->stream));
@@ -1506,6 +1511,17 @@ static int check_status(gw_engine* e) {
   }
   return GW_OK;
 }
+
+static int check_status(gw_engine* e) {
+  GW_CUDA(e, cudaMemcpyAsync(e->h_status.p, e->view.status, sizeof(uint32_t), cudaMemcpyDeviceToHost, e->stream));
+  GW_CUDA(e, cudaStreamSynchronize(e->stream));
+  return report_status(e, *(uint32_t*)e->h_status.p);
+}
+
+// Results of this size and more are copied out by four threads: starting them
+// takes about 50 us, the time one thread takes for some hundred KB into fresh
+// pages.
+constexpr size_t kLargeOut = (size_t)4 << 20;
 
 extern "C" int gw_eval(gw_engine* e, const double* params, int32_t K, double* sums, double* sums2, double* llh,
                        double* llh_stat) {
@@ -1518,24 +1534,27 @@ extern "C" int gw_eval(gw_engine* e, const double* params, int32_t K, double* su
   if (rc) return rc;
   std::memcpy(e->h_params.p, params, sizeof(double) * (size_t)K * P);
   cudaStream_t s = e->stream;
+  const OutLayout o((size_t)K, (size_t)B);
+  // the results up to the last one asked for, in one copy (five copies of the status and the results
+  // cost 8 us more a call); large blocks in four, which are copied out while the
+  // later ones arrive (100 points x 10,000 bins: 2.56 -> 1.87 ms a call)
+  const size_t bytes = sums2 ? o.end : sums ? o.sums2 : o.sums;
+  const bool large = bytes >= kLargeOut;
+  char* const h_out = (char*)e->h_out.p;
   auto run = [&]() -> int {
     GW_CUDA(e, cudaMemcpyAsync(e->d_params, e->h_params.p, sizeof(double) * (size_t)K * P,
                                cudaMemcpyHostToDevice, s));
-    int r = launch_chain(e, (const double*)e->d_params, K, (double*)e->d_sums, (double*)e->d_sums2,
-                         (double*)e->d_llh, (double*)e->d_llh_stat, s);
+    int r = launch_chain(e, (const double*)e->d_params, K, o.at(e->d_out, o.sums), o.at(e->d_out, o.sums2),
+                         o.at(e->d_out, o.llh), o.at(e->d_out, o.stat), s);
     if (r) return r;
-    GW_CUDA(e, cudaMemcpyAsync(e->h_sums.p, e->d_sums, sizeof(double) * (size_t)K * B, cudaMemcpyDeviceToHost, s));
-    GW_CUDA(e, cudaMemcpyAsync(e->h_sums2.p, e->d_sums2, sizeof(double) * (size_t)K * B, cudaMemcpyDeviceToHost,
-                               s));
-    GW_CUDA(e, cudaMemcpyAsync(e->h_llh.p, e->d_llh, sizeof(double) * (size_t)K, cudaMemcpyDeviceToHost, s));
-    GW_CUDA(e, cudaMemcpyAsync(e->h_llh_stat.p, e->d_llh_stat, sizeof(double) * (size_t)K, cudaMemcpyDeviceToHost,
-                               s));
+    if (!large) GW_CUDA(e, cudaMemcpyAsync(h_out, e->d_out, bytes, cudaMemcpyDeviceToHost, s));
     return GW_OK;
   };
   rc = chain_begin(e, s);
   if (rc) return rc;
   if (e->use_graph) {
-    auto it = e->graphs.find(K);
+    const int key = 4 * K + (sums2 ? 2 : sums ? 1 : 0);  // the copy's size is part of the graph
+    auto it = e->graphs.find(key);
     if (it == e->graphs.end()) {
       GW_CUDA(e, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
       int r = run();
@@ -1550,7 +1569,7 @@ extern "C" int gw_eval(gw_engine* e, const double* params, int32_t K, double* su
       ce = cudaGraphInstantiate(&ex, g, 0);
       cudaGraphDestroy(g);
       if (ce != cudaSuccess) return fail(e, GW_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(ce));
-      it = e->graphs.emplace(K, ex).first;
+      it = e->graphs.emplace(key, ex).first;
     }
     GW_CUDA(e, cudaGraphLaunch(it->second, s));
   } else {
@@ -1559,12 +1578,56 @@ extern "C" int gw_eval(gw_engine* e, const double* params, int32_t K, double* su
   }
   rc = chain_end(e, s);
   if (rc) return rc;
-  rc = check_status(e);  // synchronizes the stream
+  // byte range [lo, hi) of the block to the caller's arrays
+  auto copy_out = [&](size_t lo, size_t hi) {
+    const size_t from[4] = {o.llh, o.stat, o.sums, o.sums2}, to[4] = {o.stat, o.sums, o.sums2, o.end};
+    double* const dst[4] = {llh, llh_stat, sums, sums2};
+    for (int i = 0; i < 4; ++i) {
+      const size_t x = std::max(lo, from[i]), y = std::min(hi, to[i]);
+      if (dst[i] && x < y) std::memcpy((char*)dst[i] + (x - from[i]), h_out + x, y - x);
+    }
+  };
+  constexpr int kParts = 4;
+  size_t edge[kParts + 1] = {0, bytes, bytes, bytes, bytes};
+  if (large) {
+    for (int i = 1; i < kParts; ++i) edge[i] = bytes / kParts * i & ~(size_t)63;
+    for (int i = 0; i < kParts; ++i) {
+      GW_CUDA(e, cudaMemcpyAsync(h_out + edge[i], (char*)e->d_out + edge[i], edge[i + 1] - edge[i],
+                                 cudaMemcpyDeviceToHost, s));
+      GW_CUDA(e, cudaEventRecord(e->out_part[i], s));
+    }
+    GW_CUDA(e, cudaEventSynchronize(e->out_part[0]));
+  } else {
+    GW_CUDA(e, cudaStreamSynchronize(s));
+  }
+  rc = report_status(e, *(const uint32_t*)h_out);  // the first part holds the status word
   if (rc) return rc;
-  if (sums) std::memcpy(sums, e->h_sums.p, sizeof(double) * (size_t)K * B);
-  if (sums2) std::memcpy(sums2, e->h_sums2.p, sizeof(double) * (size_t)K * B);
-  if (llh) std::memcpy(llh, e->h_llh.p, sizeof(double) * (size_t)K);
-  if (llh_stat) std::memcpy(llh_stat, e->h_llh_stat.p, sizeof(double) * (size_t)K);
+  if (large) {
+    // a thread per part: the caller's arrays are often fresh, and copying into
+    // pages touched for the first time runs at a few GB/s per thread
+    std::vector<std::thread> th;
+    cudaError_t st[kParts] = {cudaSuccess, cudaSuccess, cudaSuccess, cudaSuccess};
+    auto part = [&](int i) {
+      st[i] = cudaSetDevice(e->device);
+      if (st[i] == cudaSuccess) st[i] = cudaEventSynchronize(e->out_part[i]);
+      if (st[i] == cudaSuccess) copy_out(edge[i], edge[i + 1]);
+    };
+    int own = kParts;  // parts [own, kParts) went to threads
+    try {
+      th.reserve(kParts);
+      while (own > 1) {
+        th.emplace_back(part, own - 1);
+        --own;
+      }
+    } catch (const std::exception&) {
+      // no thread to be had: this one copies the rest
+    }
+    for (int i = 0; i < own; ++i) part(i);
+    for (auto& x : th) x.join();
+    for (const cudaError_t r : st) GW_CUDA(e, r);
+  } else {
+    copy_out(0, bytes);
+  }
   e->weights_valid = e->copy_weights && K == 1;
   return GW_OK;
 }
@@ -1634,17 +1697,18 @@ static int autotune_plain(gw_engine* e) {
   cudaEvent_t a, b;
   GW_CUDA(e, cudaEventCreate(&a));
   GW_CUDA(e, cudaEventCreate(&b));
+  const OutLayout o(1, (size_t)e->cfg.n_bins);
   float best = 1e30f;
   int best_kind = e->view.plain_kind;
   for (int kind = 0; kind < 3; ++kind) {
     if (gw_set_plain_kernel(e, kind) != GW_OK) continue;
-    int rc = launch_chain(e, (const double*)e->d_params, 1, (double*)e->d_sums, (double*)e->d_sums2,
-                          (double*)e->d_llh, (double*)e->d_llh_stat, e->stream);
+    int rc = launch_chain(e, (const double*)e->d_params, 1, o.at(e->d_out, o.sums), o.at(e->d_out, o.sums2),
+                          o.at(e->d_out, o.llh), o.at(e->d_out, o.stat), e->stream);
     if (rc) return rc;
     GW_CUDA(e, cudaEventRecord(a, e->stream));
     for (int rep = 0; rep < 5; ++rep) {
-      rc = launch_chain(e, (const double*)e->d_params, 1, (double*)e->d_sums, (double*)e->d_sums2,
-                        (double*)e->d_llh, (double*)e->d_llh_stat, e->stream);
+      rc = launch_chain(e, (const double*)e->d_params, 1, o.at(e->d_out, o.sums), o.at(e->d_out, o.sums2),
+                        o.at(e->d_out, o.llh), o.at(e->d_out, o.stat), e->stream);
       if (rc) return rc;
     }
     GW_CUDA(e, cudaEventRecord(b, e->stream));
@@ -1680,6 +1744,7 @@ extern "C" int gw_autotune(gw_engine* e, int32_t K) {
   cudaEvent_t a, b_ev;
   GW_CUDA(e, cudaEventCreate(&a));
   GW_CUDA(e, cudaEventCreate(&b_ev));
+  const OutLayout o((size_t)K, (size_t)e->cfg.n_bins);
   float best = 1e30f;
   BatchedShape best_shape = e->shape;
   int best_grid = e->batched_grid;
@@ -1696,13 +1761,13 @@ extern "C" int gw_autotune(gw_engine* e, int32_t K) {
     if (bps < 1) continue;
     e->shape = b;
     e->batched_grid = (int)std::max<int64_t>(1, std::min<int64_t>(e->view.n_tiles, (int64_t)bps * e->num_sms));
-    int rc = launch_chain(e, (const double*)e->d_params, K, (double*)e->d_sums, (double*)e->d_sums2,
-                          (double*)e->d_llh, (double*)e->d_llh_stat, e->stream);
+    int rc = launch_chain(e, (const double*)e->d_params, K, o.at(e->d_out, o.sums), o.at(e->d_out, o.sums2),
+                          o.at(e->d_out, o.llh), o.at(e->d_out, o.stat), e->stream);
     if (rc) return rc;
     GW_CUDA(e, cudaEventRecord(a, e->stream));
     for (int rep = 0; rep < 3; ++rep) {
-      rc = launch_chain(e, (const double*)e->d_params, K, (double*)e->d_sums, (double*)e->d_sums2,
-                        (double*)e->d_llh, (double*)e->d_llh_stat, e->stream);
+      rc = launch_chain(e, (const double*)e->d_params, K, o.at(e->d_out, o.sums), o.at(e->d_out, o.sums2),
+                        o.at(e->d_out, o.llh), o.at(e->d_out, o.stat), e->stream);
       if (rc) return rc;
     }
     GW_CUDA(e, cudaEventRecord(b_ev, e->stream));
