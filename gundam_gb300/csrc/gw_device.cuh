@@ -8,6 +8,7 @@
 
 #include "gw_dials.cuh"
 #include "gw_internal.h"
+#include "gw_launch.h"
 
 namespace gw {
 namespace {

@@ -39,6 +39,7 @@ namespace {
 template <typename T>
 __global__ void __launch_bounds__(256) k_params(const DevView v, const double* __restrict__ params) {
   extern __shared__ double sp[];  // raw parameter vector of point k [, original values]
+  dep_launch();  // not itself a dependent launch: what it reads was complete before it started
   const int k = blockIdx.x;
   const int P = v.n_params;
   if (blockIdx.y > 0) {
@@ -132,6 +133,8 @@ __global__ void __launch_bounds__(256) k_params(const DevView v, const double* _
 constexpr int kTabPts = 4;
 template <typename T>
 __global__ void __launch_bounds__(128) k_table_fn(const DevView v, int K) {
+  dep_launch();
+  dep_wait();
   const TableFn fn = v.table_fns[blockIdx.y];
   const TableDesc td = v.tables[fn.table];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -179,6 +182,8 @@ __global__ void __launch_bounds__(kPlainThreads) k_plain(const DevView v) {
 
   int tile = blockIdx.x;
   if (tid == 0 && tile < v.n_tiles) issue_tile(v, tile, stage0, &bar[0]);
+  dep_launch();
+  dep_wait();  // the points (k_params, k_table_fn); the first tile's copy travels meanwhile
   for (int it = 0; tile < v.n_tiles; ++it, tile += gridDim.x) {
     const int st = it & 1;
     const uint32_t parity = (uint32_t)((it >> 1) & 1);
@@ -310,6 +315,8 @@ __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_
     if (ntile > 0) issue_tile_hdr(v, blockIdx.x, smem, shdr, &bar[0]);
     if (ntile > 1) issue_tile_hdr(v, blockIdx.x + gridDim.x, smem + TB, shdr + hstride, &bar[1]);
   }
+  dep_launch();
+  dep_wait();  // the points (k_params, k_table_fn); the first tiles' copies travel meanwhile
   __syncthreads();
 
   if (tid < kWsEval) {
@@ -481,6 +488,7 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
   __shared__ bool last;
   const int tid = threadIdx.x;
   const int kb = blockIdx.y * KT, b0 = blockIdx.x * BT;
+  dep_wait();
   {
     const int kk = tid % KT, sl = (tid / KT) % SL, bb = tid / (KT * SL);
     const int b = b0 + bb, k = kb + kk;
@@ -706,39 +714,45 @@ cudaError_t launch_table_fns(const DevView& v, int K, int max_size, cudaStream_t
   if (v.n_table_fns == 0) return cudaSuccess;
   const dim3 grid((max_size + 127) / 128, v.n_table_fns, (K + kTabPts - 1) / kTabPts);
   if (v.precision == 2)
-    k_table_fn<dfloat><<<grid, 128, 0, s>>>(v, K);
+    launch_dependent(k_table_fn<dfloat>, grid, 128, 0, s, v, K);
   else if (v.precision)
-    k_table_fn<float><<<grid, 128, 0, s>>>(v, K);
+    launch_dependent(k_table_fn<float>, grid, 128, 0, s, v, K);
   else
-    k_table_fn<double><<<grid, 128, 0, s>>>(v, K);
+    launch_dependent(k_table_fn<double>, grid, 128, 0, s, v, K);
   return cudaGetLastError();
 }
 
+// The K = 1 chain is dependent launches (gw_launch.h): parameter update, weights
+// and bins are short, and the weights kernel's first tiles travel while the
+// parameters are updated (100k events, FP64: 81 -> 71 us an evaluation).  The
+// batched chain is not: a batched kernel fills the SMs for a millisecond, and
+// launched that way it ran slower (64 points of 1M events 1.17 -> 1.26 ms, in
+// FP64 2.04 -> 2.45 ms).
 cudaError_t launch_plain(const DevView& v, int grid, cudaStream_t s) {
   const size_t smem = plain_smem_bytes(v);
   if (v.plain_kind == 2) {
     const int nt = plain_threads(2);
     if (v.precision == 2)
-      k_plain_ws<dfloat, 256><<<grid, nt, smem, s>>>(v);
+      launch_dependent(k_plain_ws<dfloat, 256>, grid, nt, smem, s, v);
     else if (v.precision)
-      k_plain_ws<float, 256><<<grid, nt, smem, s>>>(v);
+      launch_dependent(k_plain_ws<float, 256>, grid, nt, smem, s, v);
     else
-      k_plain_ws<double, 256><<<grid, nt, smem, s>>>(v);
+      launch_dependent(k_plain_ws<double, 256>, grid, nt, smem, s, v);
   } else if (v.plain_kind == 1) {
     const int nt = plain_threads(1);
     if (v.precision == 2)
-      k_plain_ws<dfloat, 192><<<grid, nt, smem, s>>>(v);
+      launch_dependent(k_plain_ws<dfloat, 192>, grid, nt, smem, s, v);
     else if (v.precision)
-      k_plain_ws<float, 192><<<grid, nt, smem, s>>>(v);
+      launch_dependent(k_plain_ws<float, 192>, grid, nt, smem, s, v);
     else
-      k_plain_ws<double, 192><<<grid, nt, smem, s>>>(v);
+      launch_dependent(k_plain_ws<double, 192>, grid, nt, smem, s, v);
   } else {
     if (v.precision == 2)
-      k_plain<dfloat><<<grid, kPlainThreads, smem, s>>>(v);
+      launch_dependent(k_plain<dfloat>, grid, kPlainThreads, smem, s, v);
     else if (v.precision)
-      k_plain<float><<<grid, kPlainThreads, smem, s>>>(v);
+      launch_dependent(k_plain<float>, grid, kPlainThreads, smem, s, v);
     else
-      k_plain<double><<<grid, kPlainThreads, smem, s>>>(v);
+      launch_dependent(k_plain<double>, grid, kPlainThreads, smem, s, v);
   }
   return cudaGetLastError();
 }
@@ -760,8 +774,8 @@ cudaError_t launch_bins_llh(const DevView& v, int K, double* sums, double* sums2
   // point tiles as wide as K allows, so that phase 2's warps are full
   auto grid = [&](int kt, int bt) { return dim3((v.n_bins + bt - 1) / bt, (K + kt - 1) / kt); };
   if (K == 1)
-    k_bins_llh<1, 32><<<grid(1, 32), 256, 0, s>>>(v, K, sums, sums2, llh, llh_stat);
-  else if (K <= 4)
+    return launch_dependent(k_bins_llh<1, 32>, grid(1, 32), 256, 0, s, v, K, sums, sums2, llh, llh_stat);
+  if (K <= 4)
     k_bins_llh<4, 16><<<grid(4, 16), 256, 0, s>>>(v, K, sums, sums2, llh, llh_stat);
   else if (K <= 8)
     k_bins_llh<8, 16><<<grid(8, 16), 256, 0, s>>>(v, K, sums, sums2, llh, llh_stat);

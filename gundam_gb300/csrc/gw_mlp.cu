@@ -28,11 +28,14 @@
 #include <vector>
 
 #include "gw.h"
+#include "gw_launch.h"
 
 namespace gwm {
 namespace {
 
 typedef __nv_bfloat16 bf16;
+using gw::dep_launch;
+using gw::dep_wait;
 
 constexpr int kBM = 128;
 constexpr int kBK = 64;
@@ -137,6 +140,7 @@ struct Epilogue {
   const int32_t* perm;
   float* loss;
   float inv, scale;
+  int b_ready;          // 1: B was written before the launch chain began (weights, outside training)
 };
 
 // 2-D tiled TMA load of box {8 elements, R rows} at (k, row) into shared
@@ -253,11 +257,6 @@ __global__ void __launch_bounds__(NW * 32) k_gemm(const __grid_constant__ CUtens
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * BN;
   if (warp == 0) tmem_alloc(&tmem_base, BN);
-  if (ep.bias) {
-    // one coalesced load per column instead of one load per element in the
-    // epilogue, where the dependent loads stalled the tile's four warps
-    for (int c = tid; c < BN; c += NW * 32) sbias[c] = (n0 + c < N) ? ep.bias[n0 + c] : 0.f;
-  }
   if (tid == 0) {
     for (int i = 0; i < S; ++i) {
       mbar_init(&full[i], 1);
@@ -273,6 +272,24 @@ __global__ void __launch_bounds__(NW * 32) k_gemm(const __grid_constant__ CUtens
   const uint32_t tmem = tmem_base;
   const int nk = (K + kBK - 1) / kBK;
   int produced = 0;
+  // the kernel before this one may still run: until dep_wait only what it does
+  // not write is read, the weights' tiles of the first stages when they are
+  // known to be ready
+  dep_launch();
+  const int early = ep.b_ready ? min(nk, S) : 0;
+  if (tid == 0) {
+    for (int kt = 0; kt < early; ++kt) {
+      mbar_arrive_expect(&full[kt], (uint32_t)kStage);
+      tma_load_2d(smem + kt * kStage + kA, &tmB, kt * kBK, n0, &full[kt]);
+    }
+  }
+  dep_wait();
+  if (ep.bias) {
+    // one coalesced load per column instead of one load per element in the
+    // epilogue, where the dependent loads stalled the tile's four warps (read
+    // after the barrier that follows the accumulator's completion)
+    for (int c = tid; c < BN; c += NW * 32) sbias[c] = (n0 + c < N) ? ep.bias[n0 + c] : 0.f;
+  }
 
   if (tid == 0) {
     // producer
@@ -282,12 +299,14 @@ __global__ void __launch_bounds__(NW * 32) k_gemm(const __grid_constant__ CUtens
         failed = 1;
         break;
       }
-      if (failed) break;
+      if (failed && kt >= early) break;  // a stage whose weights are on the way is completed, so that it can be drained
       unsigned char* a = smem + st * kStage;
       unsigned char* b = a + kA;
-      mbar_arrive_expect(&full[st], (uint32_t)kStage);
+      if (kt >= early) {
+        mbar_arrive_expect(&full[st], (uint32_t)kStage);
+        tma_load_2d(b, &tmB, kt * kBK, n0, &full[st]);
+      }
       tma_load_2d(a, &tmA, kt * kBK, m0, &full[st]);
-      tma_load_2d(b, &tmB, kt * kBK, n0, &full[st]);
       produced = kt + 1;
     }
   } else if (tid == 32) {
@@ -415,6 +434,8 @@ __global__ void __launch_bounds__(NW * 32) k_gemm(const __grid_constant__ CUtens
 // through shared memory so both stores are coalesced; block (32, 8).
 __global__ void k_rows_to_bf16(const float* __restrict__ x, const int32_t* __restrict__ perm, int rows, int cols,
                                bf16* y, bf16* yt, int ld_t) {
+  dep_launch();
+  dep_wait();
   __shared__ bf16 tile[32][34];
   const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;
@@ -459,6 +480,8 @@ __device__ __forceinline__ float bias_grad(const bf16* __restrict__ dzt, int B) 
 
 // Bias gradients of one layer, a half-warp per unit (gwm_gradients).
 __global__ void __launch_bounds__(256) k_bias_grad(const bf16* __restrict__ dzt, int rows, int B, float* out) {
+  dep_launch();
+  dep_wait();
   const int r = blockIdx.x * 16 + (threadIdx.x >> 4);
   const float g = bias_grad(dzt + (size_t)min(r, rows - 1) * B, B);  // whole warps stay in the shuffles
   if (r < rows && (threadIdx.x & 15) == 0) out[r] = g;
@@ -496,6 +519,8 @@ struct AdamArgs {
 // takes 24 us.  The bound is the 32 bytes per weight that w, g, m, v and the BF16
 // copies move (69 MB, mostly from L2).
 __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamArgs a) {
+  dep_launch();
+  dep_wait();
   const int tid = threadIdx.x;
   int blk = blockIdx.x, li = 0;
   if (blk < a.n_tiles) {
@@ -557,6 +582,7 @@ __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamArgs a
 // rows of the first GEMM.
 __global__ void k_standardize(const double* __restrict__ theta, int rows, int cols, const float* __restrict__ mean,
                               const float* __restrict__ scale, float* x, bf16* h0) {
+  dep_launch();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)rows * cols) return;
   const int c = (int)(i % cols);
@@ -764,6 +790,7 @@ __global__ void __launch_bounds__(kHeadThreads, 3) k_head_staged(const __grid_co
                                                         const float* __restrict__ x, const float* __restrict__ mlp,
                                                         int C, const double* __restrict__ data, int llh_type,
                                                         HeadOut out, uint32_t* status) {
+  dep_launch();
   extern __shared__ __align__(128) float sh_h[];  // [kHeadStages][kHeadStage]
   __shared__ float4 s_pt[2][kHeadK][kHeadPts];  // (weight, input, staged row of the interval * kHeadBins, 0)
   __shared__ __align__(8) uint64_t bar[kHeadStages];
@@ -783,8 +810,9 @@ __global__ void __launch_bounds__(kHeadThreads, 3) k_head_staged(const __grid_co
   if (tid == 0) {
     for (int i = 0; i < kHeadStages; ++i) mbar_init(&bar[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    for (int c = 0; c < min(nchunk, kHeadStages); ++c) issue(c);
+    for (int c = 0; c < min(nchunk, kHeadStages); ++c) issue(c);  // the tables: constant
   }
+  dep_wait();
   // one (parameter, point) of each chunk per thread of the first two warps
   const int sk = tid / kHeadPts, sm = tid % kHeadPts;
   float z = 0.f;
@@ -870,6 +898,8 @@ __global__ void __launch_bounds__(kHeadThreads, 3) k_head_staged(const __grid_co
 template <int PPT, bool GRAD>
 __global__ void __launch_bounds__(256) k_head_llh(Head h, const float* __restrict__ x, const float* __restrict__ mlp,
                                                   int C, const double* __restrict__ data, int llh_type, HeadOut out) {
+  dep_launch();
+  dep_wait();
   extern __shared__ unsigned char sh_raw[];
   constexpr int NP = 8 * PPT;  // points per block
   const int din = h.din;
@@ -935,6 +965,8 @@ __global__ void __launch_bounds__(256) k_head_llh(Head h, const float* __restric
 
 // llh[m] = sum over blocks of part[m][*], one warp per point, fixed order.
 __global__ void k_llh_finish(const double* __restrict__ part, int nblk, int C, double* __restrict__ llh) {
+  dep_launch();
+  dep_wait();
   const int m = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (m >= C) return;
@@ -955,6 +987,8 @@ __global__ void k_llh_finish(const double* __restrict__ part, int nblk, int C, d
 // k_base_grad_staged holds.
 __global__ void __launch_bounds__(256) k_base_grad(Head h, const float* __restrict__ x, const float* __restrict__ G,
                                                    const float* __restrict__ S, float* __restrict__ gz) {
+  dep_launch();
+  dep_wait();
   extern __shared__ float shg[];
   float* g = shg;            // [nb]
   float* sg = shg + h.nb;    // [nb]
@@ -1012,6 +1046,7 @@ __global__ void __launch_bounds__(256, 2) k_base_grad_staged(const __grid_consta
                                                              const float* __restrict__ G,
                                                              const float* __restrict__ S, int C,
                                                              float* __restrict__ gz, uint32_t* status) {
+  dep_launch();
   extern __shared__ __align__(128) float sh_g[];  // [kGradStages][kGradRows + kGradK][32]
   constexpr int kStage = (kGradRows + kGradK) * 32;
   __shared__ int2 s_iv[kGradK][8 * kGradM];  // (staged row of the interval * 32, slope scale)
@@ -1032,8 +1067,9 @@ __global__ void __launch_bounds__(256, 2) k_base_grad_staged(const __grid_consta
   if (tid == 0) {
     for (int i = 0; i < kGradStages; ++i) mbar_init(&bar[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    for (int j = 0; j < min(nj, kGradStages); ++j) issue(j);
+    for (int j = 0; j < min(nj, kGradStages); ++j) issue(j);  // the tables: constant
   }
+  dep_wait();
   const float inv_w = (float)(nodes - 1) / (2.f * h.lim);
   for (int e = tid; e < kGradK * 8 * kGradM; e += 256) {
     const int q = e / (8 * kGradM), mm = e % (8 * kGradM);
@@ -1151,6 +1187,8 @@ __global__ void k_grad_finish(const double* __restrict__ part, int nblk, const d
                               const float* __restrict__ scale, const float* __restrict__ gz,
                               const float* __restrict__ dx, const double* __restrict__ m,
                               const float* __restrict__ icov, double* __restrict__ f, double* __restrict__ grad) {
+  dep_launch();
+  dep_wait();
   extern __shared__ float shf2[];
   const int P32 = (P + 31) & ~31, Gn = blockDim.x / P32;
   float* d = shf2;              // [P32]
@@ -1216,6 +1254,7 @@ __global__ void k_target(Head h, const float* __restrict__ x, const double* __re
 // ---------------------------------------------------------------------------
 // Host side: the network object and the C ABI.
 // ---------------------------------------------------------------------------
+using gw::launch_dependent;
 using gwm::bf16;
 
 struct gwm_chain_state;
@@ -1357,7 +1396,8 @@ static int launch_gemm(gwm_net* n, const bf16* A, const bf16* B, int M, int N, i
     cudaFuncSetAttribute(gwm::k_gemm<BN, S, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   dim3 grid((N + BN - 1) / BN, (M + gwm::kBM - 1) / gwm::kBM);
-  gwm::k_gemm<BN, S, NW><<<grid, NW * 32, smem, n->stream>>>(ma, mb, M, N, K, ep, n->status);
+  launch_dependent(gwm::k_gemm<BN, S, NW>, grid, NW * 32, smem, n->stream,
+                   ma, mb, M, N, K, ep, n->status);
   GWM_CUDA(n, cudaGetLastError());
   return GW_OK;
 }
@@ -1498,7 +1538,8 @@ extern "C" int gwm_set_layer(gwm_net* n, int32_t l, const float* w, const float*
   adam_layer(n, l, &aa, 1);
   aa.lr = 0.f;
   aa.c1 = aa.c2 = 1.f;
-  gwm::k_adam<<<aa.n_tiles, 256, 0, n->stream>>>(aa);
+  launch_dependent(gwm::k_adam, aa.n_tiles, 256, 0, n->stream,
+                   aa);
   GWM_CUDA(n, cudaGetLastError());
   GWM_CUDA(n, cudaStreamSynchronize(n->stream));
   n->step = 0;
@@ -1539,6 +1580,7 @@ static int forward(gwm_net* n, int B, Keep keep, const Loss* loss = nullptr) {
   for (int l = 0; l < L; ++l) {
     gwm::Epilogue ep{};
     ep.bias = n->b[l];
+    ep.b_ready = keep != kKeepAll;
     if (l + 1 < L) {
       ep.act = 1;
       if (keep != kKeepNone) ep.out_f32 = n->z[l];
@@ -1568,8 +1610,8 @@ static dim3 tiles32(int rows, int cols) { return dim3((unsigned)((cols + 31) / 3
 // Input rows to BF16 (and transposed) for the first GEMM; row r is perm[r] of x (perm null: r).
 // The transposed copy feeds the weight gradient of the first layer.
 static int stage_input(gwm_net* n, const float* x, const int32_t* perm, int B) {
-  gwm::k_rows_to_bf16<<<tiles32(B, n->dims[0]), dim3(32, 8), 0, n->stream>>>(
-      x, perm, B, n->dims[0], n->h[0], n->ht[0], B);
+  launch_dependent(gwm::k_rows_to_bf16, tiles32(B, n->dims[0]), dim3(32, 8), 0, n->stream,
+                   x, perm, B, n->dims[0], n->h[0], n->ht[0], B);
   GWM_CUDA(n, cudaGetLastError());
   return GW_OK;
 }
@@ -1638,7 +1680,8 @@ static int adam_all(gwm_net* n, int B, float lr) {
   a.lr = lr;
   a.c1 = 1.f - powf(0.9f, (float)n->step);
   a.c2 = 1.f - powf(0.999f, (float)n->step);
-  gwm::k_adam<<<a.n_tiles + bias_blocks, 256, 0, n->stream>>>(a);
+  launch_dependent(gwm::k_adam, a.n_tiles + bias_blocks, 256, 0, n->stream,
+                   a);
   GWM_CUDA(n, cudaGetLastError());
   return GW_OK;
 }
@@ -1655,7 +1698,8 @@ extern "C" int gwm_gradients(gwm_net* n, const float* x, const float* t, int32_t
   if (!rc) rc = backward(n, B);
   if (rc) return rc;
   for (int l = 0; l < n->n_layers; ++l)
-    gwm::k_bias_grad<<<(n->dims[l + 1] + 15) / 16, 256, 0, n->stream>>>(n->dzt[l], n->dims[l + 1], B, n->gb[l]);
+    launch_dependent(gwm::k_bias_grad, (n->dims[l + 1] + 15) / 16, 256, 0, n->stream,
+                     n->dzt[l], n->dims[l + 1], B, n->gb[l]);
   GWM_CUDA(n, cudaGetLastError());
   rc = check_status(n);
   if (rc) return rc;
@@ -1849,8 +1893,8 @@ static int launch_head(gwm_net* n, int C, int llh_type, const gwm::HeadOut& out)
       cudaFuncSetAttribute(gwm::k_head_staged<GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kShm);
     });
     const dim3 grid(head_parts(n), (C + gwm::kHeadPts - 1) / gwm::kHeadPts);
-    gwm::k_head_staged<GRAD><<<grid, gwm::kHeadThreads, kShm, n->stream>>>(
-        tab, rw, head_view(n), n->xin, n->z[L - 1], C, n->h_data, llh_type, out, n->status);
+    launch_dependent(gwm::k_head_staged<GRAD>, grid, gwm::kHeadThreads, kShm, n->stream,
+                     tab, rw, head_view(n), n->xin, n->z[L - 1], C, n->h_data, llh_type, out, n->status);
   } else {
     if (shm > 48 * 1024) {
       static std::once_flag once;
@@ -1859,8 +1903,8 @@ static int launch_head(gwm_net* n, int C, int llh_type, const gwm::HeadOut& out)
       });
     }
     const dim3 grid(head_parts(n), (C + 8 * kPPT - 1) / (8 * kPPT));
-    gwm::k_head_llh<kPPT, GRAD><<<grid, dim3(32, 8), shm, n->stream>>>(head_view(n), n->xin, n->z[L - 1], C,
-                                                                       n->h_data, llh_type, out);
+    launch_dependent(gwm::k_head_llh<kPPT, GRAD>, grid, dim3(32, 8), shm, n->stream,
+                     head_view(n), n->xin, n->z[L - 1], C, n->h_data, llh_type, out);
   }
   GWM_CUDA(n, cudaGetLastError());
   return GW_OK;
@@ -1882,8 +1926,8 @@ static int launch_base_grad(gwm_net* n, int C) {
     });
     constexpr int kTile = 8 * gwm::kGradM;
     const dim3 grid(8, (din + gwm::kGradK - 1) / gwm::kGradK, (C + kTile - 1) / kTile);
-    gwm::k_base_grad_staged<<<grid, 256, kShm, n->stream>>>(tab, rw, head_view(n), n->xin, n->g_G, n->g_S, C,
-                                                            n->g_gz, n->status);
+    launch_dependent(gwm::k_base_grad_staged, grid, 256, kShm, n->stream,
+                     tab, rw, head_view(n), n->xin, n->g_G, n->g_S, C, n->g_gz, n->status);
   } else {
     if (shb > 48 * 1024) {
       static std::once_flag once;
@@ -1891,7 +1935,8 @@ static int launch_base_grad(gwm_net* n, int C) {
         cudaFuncSetAttribute(gwm::k_base_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       });
     }
-    gwm::k_base_grad<<<dim3(C, (din + 7) / 8), 256, shb, n->stream>>>(head_view(n), n->xin, n->g_G, n->g_S, n->g_gz);
+    launch_dependent(gwm::k_base_grad, dim3(C, (din + 7) / 8), 256, shb, n->stream,
+                     head_view(n), n->xin, n->g_G, n->g_S, n->g_gz);
   }
   GWM_CUDA(n, cudaGetLastError());
   return GW_OK;
@@ -1911,7 +1956,8 @@ static int head_llh(gwm_net* n, int C, int llh_type, bool outputs, bool finish =
   const int rc = launch_head<false>(n, C, llh_type, out);
   if (rc) return rc;
   const int nbx = head_parts(n);
-  if (finish) gwm::k_llh_finish<<<(C + 7) / 8, 256, 0, n->stream>>>(n->h_part, nbx, C, n->h_llh);
+  if (finish) launch_dependent(gwm::k_llh_finish, (C + 7) / 8, 256, 0, n->stream,
+                     n->h_part, nbx, C, n->h_llh);
   GWM_CUDA(n, cudaGetLastError());
   return GW_OK;
 }
@@ -2152,6 +2198,8 @@ __device__ __forceinline__ double u01(uint64_t h) { return ((double)(h >> 11) + 
 __global__ void k_propose_stage(const double* __restrict__ phi, int P, const float* __restrict__ Lt, uint64_t seed,
                                 uint64_t step, double* __restrict__ prop, const float* __restrict__ mean,
                                 const float* __restrict__ scale, float* __restrict__ x, bf16* __restrict__ h0) {
+  dep_launch();
+  dep_wait();
   // blockDim.x = G * P32: group g of the column's partial sums covers the
   // k-range [g*ks, (g+1)*ks); the groups are combined in a fixed order
   extern __shared__ float shp[];
@@ -2200,6 +2248,8 @@ __global__ void k_finish_accept(const double* __restrict__ part, int nblk, const
                                 const double* __restrict__ m, const float* __restrict__ icov, uint64_t seed,
                                 uint64_t step, int first, double* __restrict__ phi, double* __restrict__ f,
                                 int32_t* __restrict__ n_acc) {
+  dep_launch();
+  dep_wait();
   // blockDim.x = G * P32 as k_propose_stage
   extern __shared__ float shf[];
   const int P32 = (P + 31) & ~31, G = blockDim.x / P32;
@@ -2376,21 +2426,22 @@ extern "C" int gwm_substeps(gwm_net* n, const double* theta0, const double* f0, 
                                 n->stream));
     rc = surrogate_llh_device(n, C, llh_type);
     if (rc) return rc;
-    gwm::k_finish_accept<<<C, thr, sh_fin, n->stream>>>(n->h_part, nbx, s->phi, P, prior ? s->m : nullptr, s->icov,
-                                                       seed, 0, 1, s->phi, s->f, s->nacc);
+    launch_dependent(gwm::k_finish_accept, C, thr, sh_fin, n->stream,
+                     n->h_part, nbx, s->phi, P, prior ? s->m : nullptr, s->icov, seed, 0, 1, s->phi, s->f, s->nacc);
     GWM_CUDA(n, cudaGetLastError());
   }
   // rows C..Bp of the first GEMM's input stay zero through the sub-steps
   if (Bp > C) GWM_CUDA(n, cudaMemsetAsync(n->h[0] + (size_t)C * P, 0, sizeof(bf16) * (size_t)(Bp - C) * P, n->stream));
   for (int st = 0; st < n_sub && rc == GW_OK; ++st) {
-    gwm::k_propose_stage<<<C, thr, sh_prop, n->stream>>>(s->phi, P, s->Lt, seed, (uint64_t)st + 1, n->h_theta,
-                                                        n->h_mean, n->h_scale, n->xin, n->h[0]);
+    launch_dependent(gwm::k_propose_stage, C, thr, sh_prop, n->stream,
+                     s->phi, P, s->Lt, seed, (uint64_t)st + 1, n->h_theta, n->h_mean, n->h_scale, n->xin, n->h[0]);
     GWM_CUDA(n, cudaGetLastError());
     rc = forward(n, Bp, kKeepNone);
     if (!rc) rc = head_llh(n, C, llh_type, false, false);
     if (rc) break;
-    gwm::k_finish_accept<<<C, thr, sh_fin, n->stream>>>(n->h_part, nbx, n->h_theta, P, prior ? s->m : nullptr,
-                                                       s->icov, seed, (uint64_t)st + 1, 0, s->phi, s->f, s->nacc);
+    launch_dependent(gwm::k_finish_accept, C, thr, sh_fin, n->stream,
+                     n->h_part, nbx, n->h_theta, P, prior ? s->m : nullptr, s->icov, seed, (uint64_t)st + 1, 0, s->phi,
+                     s->f, s->nacc);
     GWM_CUDA(n, cudaGetLastError());
   }
   if (rc) return rc;
@@ -2412,11 +2463,13 @@ static int backward_dx(gwm_net* n, int B) {
     gwm::Epilogue e{};
     e.gate = n->z[l - 1];
     e.out_bf16 = n->dz[l - 1];
+    e.b_ready = 1;
     int rc = gemm(n, n->dz[l], n->wt[l], B, n->dims[l], n->dims[l + 1], e);
     if (rc) return rc;
   }
   gwm::Epilogue e0{};
   e0.out_f32 = n->g_dx;
+  e0.b_ready = 1;
   return gemm(n, n->dz[0], n->wt[0], B, n->dims[0], n->dims[1], e0);
 }
 
@@ -2458,9 +2511,9 @@ extern "C" int gwm_value_grad(gwm_net* n, const double* theta, int32_t C, int32_
   const int P32 = (din + 31) & ~31;
   const int Gn = std::max(1, std::min(4, 1024 / P32));
   const bool prior = n->chain && n->chain->prior;
-  gwm::k_grad_finish<<<C, (unsigned)(Gn * P32), sizeof(float) * (size_t)P32 * (Gn + 2), n->stream>>>(
-      n->h_part, nbx, n->h_theta, din, n->h_scale, n->g_gz, n->g_dx, prior ? n->chain->m : nullptr,
-      prior ? n->chain->icov : nullptr, n->g_f, n->g_grad);
+  launch_dependent(gwm::k_grad_finish, C, (unsigned)(Gn * P32), sizeof(float) * (size_t)P32 * (Gn + 2), n->stream,
+                   n->h_part, nbx, n->h_theta, din, n->h_scale, n->g_gz, n->g_dx, prior ? n->chain->m : nullptr,
+                   prior ? n->chain->icov : nullptr, n->g_f, n->g_grad);
   GWM_CUDA(n, cudaGetLastError());
   GWM_CUDA(n, cudaMemcpyAsync(f, n->g_f, sizeof(double) * C, cudaMemcpyDeviceToHost, n->stream));
   GWM_CUDA(n, cudaMemcpyAsync(grad, n->g_grad, sizeof(double) * (size_t)C * din, cudaMemcpyDeviceToHost, n->stream));
