@@ -1162,7 +1162,11 @@ int build_and_upload(gw_engine* e) {
   GW_CUDA(e, cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, e->device));
   GW_CUDA(e, cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
   GW_CUDA(e, cudaEventCreateWithFlags(&e->chain_done, cudaEventDisableTiming));
-  e->kpad = ((e->cfg.k_max + 63) / 64) * 64;  // a batched pass covers up to 64 points
+  // point columns per row: a batched pass covers up to 64 points; an engine of one
+  // point keeps one column, so that its parameters, clamps aside, fit a few L1
+  // lines (200 parameters 64 columns apart are 200 lines, more than the L1 that
+  // the K = 1 kernels' shared memory leaves: 171 against 146 us for 1M events)
+  e->kpad = e->cfg.k_max == 1 ? 1 : ((e->cfg.k_max + 63) / 64) * 64;
   const int P = e->cfg.n_params;
   const int kpad = e->kpad;
 
