@@ -283,7 +283,8 @@ __device__ __forceinline__ void load_points(const T* __restrict__ p, int kstep, 
   }
 }
 
-template <typename T, int KR, bool VX = false>
+// WARP: the whole warp holds the same dial.
+template <typename T, int KR, bool VX = false, bool WARP = false>
 __device__ __forceinline__ void dial_values(const DevView& v, uint64_t h, const T* __restrict__ pl, int k0,
                                             int kstep, T (&val)[KR]) {
   const int type = hdr_type(h);
@@ -374,11 +375,19 @@ __device__ __forceinline__ void dial_values(const DevView& v, uint64_t h, const 
         else
           prepared_values<T, false, KR>(d, n, x, trunc, val);
       } else if (type == kGeneral) {
+        if constexpr (WARP) {
+          general_values<T, KR>(d, n, x, trunc, val);
+        } else {
 #pragma unroll
-        for (int j = 0; j < KR; ++j) val[j] = eval_general<T>(d, n, x[j], trunc);
+          for (int j = 0; j < KR; ++j) val[j] = eval_general<T>(d, n, x[j], trunc);
+        }
       } else if (type == kGraph) {
+        if constexpr (WARP) {
+          graph_values<T, KR>(d, n, x, trunc, val);
+        } else {
 #pragma unroll
-        for (int j = 0; j < KR; ++j) val[j] = eval_graph<T>(d, n, x[j], trunc);
+          for (int j = 0; j < KR; ++j) val[j] = eval_graph<T>(d, n, x[j], trunc);
+        }
       } else if (type == kBilinear) {
         T y[KR];
         load_points<T, KR, VX>((const T*)v.x + (size_t)hdr_p1(h) * v.kpad + k0, kstep, y);

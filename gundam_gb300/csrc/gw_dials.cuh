@@ -422,6 +422,24 @@ __device__ __forceinline__ T lin(T x, T x0, T p0, T x1, T p1) {
   return p0 + fdiv((p1 - p0) * (x - x0), x1 - x0);
 }
 
+// The facet of a bilinear surface whose lower corner is q[0] (rows of ny
+// values) between the knots ax[0], ax[1] and ay[0], ay[1].
+template <typename T>
+__device__ __forceinline__ T bilinear_facet(const T* __restrict__ q, int ny, const T* __restrict__ ax,
+                                            const T* __restrict__ ay, T x, T y) {
+  if constexpr (sizeof(T) >= 8) {
+    // FP64 and double-float: one quotient per axis instead of one per line
+    const T fx = fdiv(x - ax[0], ax[1] - ax[0]), fy = fdiv(y - ay[0], ay[1] - ay[0]);
+    const T v0 = q[0] + (q[ny] - q[0]) * fx;
+    const T v1 = q[1] + (q[ny + 1] - q[1]) * fx;
+    return v0 + (v1 - v0) * fy;
+  } else {
+    const T v0 = lin(x, ax[0], q[0], ax[1], q[ny]);
+    const T v1 = lin(x, ax[0], q[1], ax[1], q[ny + 1]);
+    return lin(y, ay[0], v0, ay[1], v1);
+  }
+}
+
 // Bilinear surface: CalculateBilinearInterpolation.h:103-152.
 // d = [nx, ny, xx[nx], yy[ny], z[nx*ny]] (z index = ix*ny + iy).
 template <typename T>
@@ -439,17 +457,7 @@ __device__ __forceinline__ T eval_bilinear(const T* __restrict__ d, T x, T y, bo
   }
   const int ix = surface_index(x, xx, nx - 1);
   const int iy = surface_index(y, yy, ny - 1);
-  if constexpr (sizeof(T) >= 8) {
-    // FP64 and double-float: one quotient per axis instead of one per line
-    const T fx = fdiv(x - xx[ix], xx[ix + 1] - xx[ix]), fy = fdiv(y - yy[iy], yy[iy + 1] - yy[iy]);
-    const T* q = z + ix * ny + iy;
-    const T v0 = q[0] + (q[ny] - q[0]) * fx;
-    const T v1 = q[1] + (q[ny + 1] - q[1]) * fx;
-    return v0 + (v1 - v0) * fy;
-  }
-  const T v0 = lin(x, xx[ix], z[ix * ny + iy], xx[ix + 1], z[(ix + 1) * ny + iy]);
-  const T v1 = lin(x, xx[ix], z[ix * ny + iy + 1], xx[ix + 1], z[(ix + 1) * ny + iy + 1]);
-  return (lin(y, yy[iy], v0, yy[iy + 1], v1));
+  return bilinear_facet(z + ix * ny + iy, ny, xx + ix, yy + iy, x, y);
 }
 
 // One Catmull-Rom segment through (x0,p0)..(x3,p3) evaluated between x1 and
@@ -516,6 +524,88 @@ __device__ __forceinline__ T eval_bicubic(const T* __restrict__ d, T x, T y, boo
                      surf_knot(z, nx, ny, ix + 1, j), a3, surf_knot(z, nx, ny, ix + 2, j));
   }
   return (cubic_seg(y, u[0], v[0], u[1], v[1], u[2], v[2], u[3], v[3]));
+}
+
+// ---------------------------------------------------------------------------
+// One dial at KR points by a whole warp (the lanes-over-points kernel): every
+// lane holds the same dial, so loops over its knots are uniform.  The interval
+// is found by halving steps that stay in range, a load, a comparison and a
+// select per point, where the five-step searches of eval_general and eval_graph
+// test every candidate's index as well (64 points: general spline 229 -> 192
+// warp instructions, graph 205 -> 147); the arithmetic on the interval is
+// theirs.
+// ---------------------------------------------------------------------------
+
+// The last of the records 0 .. n - 2 (stride elements apart) whose knot, at
+// key, is below x (`strict`; else not above x), or record 0, as an element
+// offset.  Knots do not decrease, so it is the one the five-step searches find.
+template <typename T, int KR, bool strict>
+__device__ __forceinline__ void find_interval(const T* __restrict__ key, int stride, int n, const T (&x)[KR],
+                                              int (&a)[KR]) {
+#pragma unroll
+  for (int j = 0; j < KR; ++j) a[j] = 0;
+  for (int len = n - 1; len > 1;) {
+    const int half = len >> 1, by = half * stride;
+#pragma unroll
+    for (int j = 0; j < KR; ++j) {
+      const T k = key[a[j] + by];
+      if (strict ? above(x[j], k) : !above(k, x[j])) a[j] += by;
+    }
+    len -= half;
+  }
+}
+
+template <typename T, int KR>
+__device__ __forceinline__ void general_values(const T* __restrict__ d, int n, const T (&xin)[KR], bool trunc,
+                                               T (&val)[KR]) {
+  T x[KR];
+#pragma unroll
+  for (int j = 0; j < KR; ++j) x[j] = xin[j];
+  if (trunc) {
+    const T lo = d[2], hi = d[3 * (n - 1) + 2];
+#pragma unroll
+    for (int j = 0; j < KR; ++j) {
+      if (x[j] <= lo) x[j] = lo;
+      else if (x[j] >= hi) x[j] = hi;
+    }
+  }
+  int a[KR];
+  find_interval<T, KR, true>(d + 2, 3, n, x, a);
+#pragma unroll
+  for (int j = 0; j < KR; ++j) {
+    const T* q = d + a[j];
+    const T step = q[5] - q[2];
+    const T fx = fdiv(x[j] - q[2], step);
+    const T m1 = q[1] * step;
+    const T m2 = q[4] * step;
+    val[j] = hermite(q[0], m1, q[3], m2, fx);
+  }
+}
+
+template <typename T, int KR>
+__device__ __forceinline__ void graph_values(const T* __restrict__ d, int n, const T (&x)[KR], bool trunc,
+                                             T (&val)[KR]) {
+  if (n < 2) {
+#pragma unroll
+    for (int j = 0; j < KR; ++j) val[j] = d[0];
+    return;
+  }
+  int a[KR];
+  find_interval<T, KR, true>(d + 1, 2, n, x, a);
+#pragma unroll
+  for (int j = 0; j < KR; ++j) {
+    const T* q = d + a[j];
+    const T fx = fdiv(x[j] - q[1], q[3] - q[1]);
+    const T m = q[2] - q[0];
+    val[j] = q[0] + fx * m;
+  }
+  if (trunc) {
+#pragma unroll
+    for (int j = 0; j < KR; ++j) {
+      if (x[j] <= d[1]) val[j] = d[0];
+      else if (x[j] >= d[2 * n - 1]) val[j] = d[2 * n - 2];
+    }
+  }
 }
 
 }  // namespace gw

@@ -153,14 +153,14 @@ __global__ void __launch_bounds__(NT, MB) k_batched(const DevView v, int K) {
               if (hdr_type(h) == kGrid)
                 grid_eval<T, KR>(pl, h, a, val);
               else
-                dial_values<T, KR>(v, h, pl, k0, KC, val);
+                dial_values<T, KR, false, KC == 32>(v, h, pl, k0, KC, val);
 #pragma unroll
               for (int j = 0; j < KR; ++j) w[j] *= val[j];
             }
           } else {
             for (int sl = s0; sl < s1; ++sl) {
               T val[KR];
-              dial_values<T, KR>(v, shdr[sl], pl, k0, KC, val);
+              dial_values<T, KR, false, KC == 32>(v, shdr[sl], pl, k0, KC, val);
 #pragma unroll
               for (int j = 0; j < KR; ++j) w[j] *= val[j];
             }
