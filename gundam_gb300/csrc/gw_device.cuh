@@ -213,33 +213,6 @@ __device__ __forceinline__ void prepared_values(const T* __restrict__ d, int n, 
   }
 }
 
-// A grid-form dial's inputs at KR points (k0, k0 + kstep, ...): the grid's
-// interval and fraction per point and its response clamp.  The lanes kernel
-// loads them one dial ahead of the evaluation, so the (mostly L2) latency of
-// the grid table overlaps the previous dial's arithmetic.
-template <typename T, int KR>
-struct GridAhead {
-  GridPoint<T> g[KR];
-  typename Vec2<T>::type c;
-};
-
-template <typename T, int KR>
-__device__ __forceinline__ void grid_load(const DevView& v, uint64_t h, int k0, int kstep, GridAhead<T, KR>& a) {
-  const int g = hdr_p0(h);
-  const GridPoint<T>* gp = (const GridPoint<T>*)v.grid_pts + (size_t)g * v.kpad + k0;
-#pragma unroll
-  for (int j = 0; j < KR; ++j) a.g[j] = gp[j * kstep];
-  a.c = ((const typename Vec2<T>::type*)v.grid_clamp)[g];
-}
-
-template <typename T, int KR>
-__device__ __forceinline__ void grid_eval(const T* __restrict__ pl, uint64_t h, const GridAhead<T, KR>& a,
-                                          T (&val)[KR]) {
-  const T* d = pl + hdr_off(h);
-#pragma unroll
-  for (int j = 0; j < KR; ++j) val[j] = clamp_response(coef_cubic(d + a.g[j].jb, a.g[j].u), a.c.x, a.c.y);
-}
-
 // The KR values of one parameter at points k0, k0 + kstep, ...  With VX the
 // points are contiguous (kstep == 1) and k0 * sizeof(T) is a multiple of
 // KR * sizeof(T) (at most 16), so whole 8- or 16-byte vectors are loaded.
@@ -283,8 +256,7 @@ __device__ __forceinline__ void load_points(const T* __restrict__ p, int kstep, 
   }
 }
 
-// WARP: the whole warp holds the same dial.
-template <typename T, int KR, bool VX = false, bool WARP = false>
+template <typename T, int KR, bool VX = false>
 __device__ __forceinline__ void dial_values(const DevView& v, uint64_t h, const T* __restrict__ pl, int k0,
                                             int kstep, T (&val)[KR]) {
   const int type = hdr_type(h);
@@ -375,19 +347,11 @@ __device__ __forceinline__ void dial_values(const DevView& v, uint64_t h, const 
         else
           prepared_values<T, false, KR>(d, n, x, trunc, val);
       } else if (type == kGeneral) {
-        if constexpr (WARP) {
-          general_values<T, KR>(d, n, x, trunc, val);
-        } else {
 #pragma unroll
-          for (int j = 0; j < KR; ++j) val[j] = eval_general<T>(d, n, x[j], trunc);
-        }
+        for (int j = 0; j < KR; ++j) val[j] = eval_general<T>(d, n, x[j], trunc);
       } else if (type == kGraph) {
-        if constexpr (WARP) {
-          graph_values<T, KR>(d, n, x, trunc, val);
-        } else {
 #pragma unroll
-          for (int j = 0; j < KR; ++j) val[j] = eval_graph<T>(d, n, x[j], trunc);
-        }
+        for (int j = 0; j < KR; ++j) val[j] = eval_graph<T>(d, n, x[j], trunc);
       } else if (type == kBilinear) {
         T y[KR];
         load_points<T, KR, VX>((const T*)v.x + (size_t)hdr_p1(h) * v.kpad + k0, kstep, y);

@@ -526,86 +526,4 @@ __device__ __forceinline__ T eval_bicubic(const T* __restrict__ d, T x, T y, boo
   return (cubic_seg(y, u[0], v[0], u[1], v[1], u[2], v[2], u[3], v[3]));
 }
 
-// ---------------------------------------------------------------------------
-// One dial at KR points by a whole warp (the lanes-over-points kernel): every
-// lane holds the same dial, so loops over its knots are uniform.  The interval
-// is found by halving steps that stay in range, a load, a comparison and a
-// select per point, where the five-step searches of eval_general and eval_graph
-// test every candidate's index as well (64 points: general spline 229 -> 192
-// warp instructions, graph 205 -> 147); the arithmetic on the interval is
-// theirs.
-// ---------------------------------------------------------------------------
-
-// The last of the records 0 .. n - 2 (stride elements apart) whose knot, at
-// key, is below x (`strict`; else not above x), or record 0, as an element
-// offset.  Knots do not decrease, so it is the one the five-step searches find.
-template <typename T, int KR, bool strict>
-__device__ __forceinline__ void find_interval(const T* __restrict__ key, int stride, int n, const T (&x)[KR],
-                                              int (&a)[KR]) {
-#pragma unroll
-  for (int j = 0; j < KR; ++j) a[j] = 0;
-  for (int len = n - 1; len > 1;) {
-    const int half = len >> 1, by = half * stride;
-#pragma unroll
-    for (int j = 0; j < KR; ++j) {
-      const T k = key[a[j] + by];
-      if (strict ? above(x[j], k) : !above(k, x[j])) a[j] += by;
-    }
-    len -= half;
-  }
-}
-
-template <typename T, int KR>
-__device__ __forceinline__ void general_values(const T* __restrict__ d, int n, const T (&xin)[KR], bool trunc,
-                                               T (&val)[KR]) {
-  T x[KR];
-#pragma unroll
-  for (int j = 0; j < KR; ++j) x[j] = xin[j];
-  if (trunc) {
-    const T lo = d[2], hi = d[3 * (n - 1) + 2];
-#pragma unroll
-    for (int j = 0; j < KR; ++j) {
-      if (x[j] <= lo) x[j] = lo;
-      else if (x[j] >= hi) x[j] = hi;
-    }
-  }
-  int a[KR];
-  find_interval<T, KR, true>(d + 2, 3, n, x, a);
-#pragma unroll
-  for (int j = 0; j < KR; ++j) {
-    const T* q = d + a[j];
-    const T step = q[5] - q[2];
-    const T fx = fdiv(x[j] - q[2], step);
-    const T m1 = q[1] * step;
-    const T m2 = q[4] * step;
-    val[j] = hermite(q[0], m1, q[3], m2, fx);
-  }
-}
-
-template <typename T, int KR>
-__device__ __forceinline__ void graph_values(const T* __restrict__ d, int n, const T (&x)[KR], bool trunc,
-                                             T (&val)[KR]) {
-  if (n < 2) {
-#pragma unroll
-    for (int j = 0; j < KR; ++j) val[j] = d[0];
-    return;
-  }
-  int a[KR];
-  find_interval<T, KR, true>(d + 1, 2, n, x, a);
-#pragma unroll
-  for (int j = 0; j < KR; ++j) {
-    const T* q = d + a[j];
-    const T fx = fdiv(x[j] - q[1], q[3] - q[1]);
-    const T m = q[2] - q[0];
-    val[j] = q[0] + fx * m;
-  }
-  if (trunc) {
-#pragma unroll
-    for (int j = 0; j < KR; ++j) {
-      if (x[j] <= d[1]) val[j] = d[0];
-      else if (x[j] >= d[2 * n - 1]) val[j] = d[2 * n - 2];
-    }
-  }
-}
-
 }  // namespace gw

@@ -1071,6 +1071,10 @@ int build_and_upload(gw_engine* e) {
   std::vector<uint64_t> hdr((size_t)hdr_total, 0);
   // the lanes kernel walks a tile's dials event by event: it bulk-copies the
   // headers in slot order (engines of more than one point)
+  auto common_clamp = [&](int par) {
+    const double lo = e->clamp_lo[(size_t)par];
+    return lo == 0.0 && !std::signbit(lo) && e->clamp_hi[(size_t)par] >= 1e20;
+  };
   std::vector<uint64_t> hdr_ev(e->cfg.k_max > 1 ? (size_t)hdr_total : 0, 0);
   std::vector<unsigned char> payload((size_t)payload_total, 0);
   std::vector<uint16_t> evinfo((size_t)N);
@@ -1125,7 +1129,17 @@ int build_and_upload(gw_engine* e) {
             const int p1 = r.p1 >= 0 ? r.p1 : 0;
             hdr[(size_t)(tp.dial0 + j)] = make_header(g >= 0 ? (int)kGrid : (int)r.type, pn[(size_t)di], slot, off,
                                                       p0, p1);
-            if (!hdr_ev.empty()) hdr_ev[(size_t)(tp.dial0 + slot)] = hdr[(size_t)(tp.dial0 + j)];
+            if (!hdr_ev.empty()) {
+              const int type = g >= 0 ? (int)kGrid : (int)r.type;
+              uint32_t flags = 0;
+              if (r.type < kTabulated) {
+                flags = ((e->pflags[(size_t)r.p0] & 1) ? kLhTrunc : 0u) | (common_clamp(r.p0) ? kLhCommonClamp : 0u);
+                if (type == kGrid && (flags & kLhCommonClamp)) flags |= kLhGrid;
+                if (type == kNorm && common_clamp(r.p0) && e->clamp_hi[(size_t)r.p0] >= DBL_MAX) flags |= kLhNorm;
+              }
+              hdr_ev[(size_t)(tp.dial0 + slot)] =
+                  make_lane_header(type, pn[(size_t)di], flags, (uint32_t)((size_t)off * tsz), p0, p1);
+            }
             if (r.type == kMonotonic || r.type == kCompact || r.type == kUniform)
               write_prepared<T>(r, e->dial_data.data() + r.data_off, pn[(size_t)di], pl + off,
                                 g >= 0 ? kFormGrid : dial_form);

@@ -1,6 +1,6 @@
 // gw_lanes.cu -- K > 1 reweighting kernel with lanes over parameter points
 // (one warp evaluates one dial for up to 32*KR points at once).
-#include "gw_device.cuh"
+#include "gw_lane_dials.cuh"
 
 namespace gw {
 namespace {
@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(NT, MB) k_batched(const DevView v, int K) {
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
+  const T cap = v.has_cap ? (T)v.cap : (T)HUGE_VAL;
   int tile = blockIdx.x;
   if (tid == 0) {
     mbar_init(&bar[0], 1);
@@ -57,7 +58,7 @@ __global__ void __launch_bounds__(NT, MB) k_batched(const DevView v, int K) {
 
     const int nd = td.ndials, ne = td.nevents;
     unsigned char* stage = smem + st * SB;
-    const uint64_t* shdr = (const uint64_t*)(stage + TB);  // indexed by slot
+    const uint32_t pl = smem_u32(stage), shdr = pl + (uint32_t)TB;  // headers indexed by slot
     unsigned char* evb = stage + TB + HB;
     // sev[e]: event e's first slot and local bin, sev[ne] the sentinel;
     // secc[e]: estimated work through event e; sw0[e]: its base weight
@@ -79,8 +80,6 @@ __global__ void __launch_bounds__(NT, MB) k_batched(const DevView v, int K) {
       return;
     }
     for (int e = tid; e < ne; e += NT) s_present[ev_lbin(sev[e])] = 1;
-    const T* pl = (const T*)stage;
-
     // Each warp takes a contiguous run of events holding ~1/NW of the tile's
     // estimated work (dial_cost): the first event whose preceding work
     // reaches warp*total/NW (a fixed, deterministic split, so the FP64
@@ -127,43 +126,54 @@ __global__ void __launch_bounds__(NT, MB) k_batched(const DevView v, int K) {
         const int e = base + sub;
         if (e < e_hi) {
           const uint16_t ei = sev[e];
-          const int s0 = ev_slot(ei), s1 = ev_slot(sev[e + 1]);
+          const uint32_t h0 = shdr + 8u * (uint32_t)ev_slot(ei), h1 = shdr + 8u * (uint32_t)ev_slot(sev[e + 1]);
           T w[KR];
 #pragma unroll
           for (int j = 0; j < KR; ++j) w[j] = T(1);
-          if constexpr (KR >= 4) {
-            // four or more points per lane: a grid-form dial's table entries
-            // are loaded one dial ahead (K = 256 on 2M mixed events: 9.05
-            // against 9.79 ms); with two points per lane the extra live
-            // registers cost more than the hidden latency (+7 % at K = 64)
-            uint64_t hn = 0;
-            GridAhead<T, KR> an;
-            if (s0 < s1) {
-              hn = shdr[s0];
-              if (hdr_type(hn) == kGrid) grid_load<T, KR>(v, hn, k0, KC, an);
-            }
-            for (int sl = s0; sl < s1; ++sl) {
-              const uint64_t h = hn;
-              const GridAhead<T, KR> a = an;
-              if (sl + 1 < s1) {
-                hn = shdr[sl + 1];
-                if (hdr_type(hn) == kGrid) grid_load<T, KR>(v, hn, k0, KC, an);
+          // four or more points per lane: a grid dial's table entries are
+          // loaded one dial ahead (K = 256 on 2M mixed events: 9.05 against
+          // 9.79 ms); with two points per lane the extra live registers cost
+          // more than the hidden latency (K = 64 on 1M: 1.18 against 1.11 ms)
+          constexpr bool kAhead = KR >= 4;
+          uint2 hn = make_uint2(0u, 0u);
+          GridPoints<T, KR> gn;
+          if (kAhead && h0 < h1) {
+            hn = lds64(h0);
+            if (lhdr_type(hn.x) == kGrid) grid_points<T, KR>(v, hn.y & 0xFFFFu, k0, KC, gn);
+          }
+          for (uint32_t hp = h0; hp < h1; hp += 8) {
+            uint2 h;
+            GridPoints<T, KR> g;
+            if constexpr (kAhead) {
+              h = hn;
+              g = gn;
+              if (hp + 8 < h1) {
+                hn = lds64(hp + 8);
+                if (lhdr_type(hn.x) == kGrid) grid_points<T, KR>(v, hn.y & 0xFFFFu, k0, KC, gn);
               }
-              T val[KR];
-              if (hdr_type(h) == kGrid)
-                grid_eval<T, KR>(pl, h, a, val);
-              else
-                dial_values<T, KR, false, KC == 32>(v, h, pl, k0, KC, val);
-#pragma unroll
-              for (int j = 0; j < KR; ++j) w[j] *= val[j];
+            } else {
+              h = lds64(hp);
             }
-          } else {
-            for (int sl = s0; sl < s1; ++sl) {
-              T val[KR];
-              dial_values<T, KR, false, KC == 32>(v, shdr[sl], pl, k0, KC, val);
+            T val[KR];
+            if ((int32_t)h.x < 0) {  // grid dial with the common clamp
+              if constexpr (!kAhead) grid_points<T, KR>(v, h.y & 0xFFFFu, k0, KC, g);
+              grid_values<T, KR>(h.x, pl, g, val);
+              clamp_common<T, KR>(val);
+            } else if (h.x & kLhNorm) {
+              points_of<T, KR>(v, h.y & 0xFFFFu, k0, KC, val);
 #pragma unroll
-              for (int j = 0; j < KR; ++j) w[j] *= val[j];
+              for (int j = 0; j < KR; ++j) val[j] = clamp_response(val[j], T(0.0f), open_bound<T>());
+            } else {
+              if (lhdr_type(h.x) == kGrid) {
+                if constexpr (!kAhead) grid_points<T, KR>(v, h.y & 0xFFFFu, k0, KC, g);
+                grid_values<T, KR>(h.x, pl, g, val);
+              } else {
+                other_values<T, KR>(v, h.x, h.y, pl, k0, KC, val);
+              }
+              clamp_values<T, KR>(v, h.x, h.y, val);
             }
+#pragma unroll
+            for (int j = 0; j < KR; ++j) w[j] *= val[j];
           }
           const T w0 = sw0[e];
           const int lb = ev_lbin(ei);
@@ -172,7 +182,7 @@ __global__ void __launch_bounds__(NT, MB) k_batched(const DevView v, int K) {
 #pragma unroll
             for (int j = 0; j < KR; ++j) {
               T wj = w[j];
-              if (v.has_cap && wj > (T)v.cap) wj = (T)v.cap;
+              if (wj > cap) wj = cap;
               wj = w0 * wj;
               const double wd = (double)wj;
               double2 q = part[j * 32];
@@ -194,7 +204,7 @@ __global__ void __launch_bounds__(NT, MB) k_batched(const DevView v, int K) {
 #pragma unroll
             for (int j = 0; j < KR; ++j) {
               T wj = w[j];
-              if (v.has_cap && wj > (T)v.cap) wj = (T)v.cap;
+              if (wj > cap) wj = cap;
               wj = w0 * wj;
               const double wd = (double)wj;
               s[j] += wd;

@@ -68,6 +68,24 @@ GW_HD int hdr_off(uint64_t h) { return (int)((h >> 19) & 0x1FFF); }
 GW_HD int hdr_p0(uint64_t h) { return (int)((h >> 32) & 0xFFFF); }
 GW_HD int hdr_p1(uint64_t h) { return (int)((h >> 48) & 0xFFFF); }
 
+// Headers of the lanes-over-points kernel, a tile's in slot order:
+//   x: [0,16) payload offset inside the tile in bytes, [16,20) type, [20,25) n,
+//      then the flags below
+//   y: [0,16) parameter, knot grid (grid dials) or table (table dials),
+//      [16,32) second parameter of surface dials
+constexpr uint32_t kLhTrunc = 1u << 25;        // no extrapolation
+constexpr uint32_t kLhCommonClamp = 1u << 26;  // the response clamp is [0, 1e20] or [0, more]
+constexpr uint32_t kLhNorm = 1u << 30;         // a norm dial of a parameter clamped to [0, no bound]
+constexpr uint32_t kLhGrid = 1u << 31;         // a grid dial with the common clamp
+GW_HD uint64_t make_lane_header(int type, int n, uint32_t flags, uint32_t off, int p0, int p1) {
+  const uint32_t x = (off & 0xFFFFu) | (uint32_t)(type & 0xF) << 16 | (uint32_t)(n & 0x1F) << 20 | flags;
+  const uint32_t y = (uint32_t)(p0 & 0xFFFF) | (uint32_t)(p1 & 0xFFFF) << 16;
+  return (uint64_t)x | (uint64_t)y << 32;
+}
+GW_HD int lhdr_type(uint32_t x) { return (int)((x >> 16) & 0xFu); }
+GW_HD int lhdr_n(uint32_t x) { return (int)((x >> 20) & 0x1Fu); }
+GW_HD uint32_t lhdr_off(uint32_t x) { return x & 0xFFFFu; }
+
 // Relative work of one dial in the lanes-over-points kernel (about ten warp
 // instructions per unit at 64 points, from instruction counts of one-type
 // workloads), and of one event's product and sums.  A tile's warps take runs
