@@ -79,6 +79,10 @@ __device__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, uint64_t limit
 
 constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s per tile copy
 
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 // Named barriers of warp-specialised kernels: `count` threads (a multiple of
 // 32) complete a phase; arrive does not wait, sync does.
 __device__ __forceinline__ void named_sync(int id, int count) {

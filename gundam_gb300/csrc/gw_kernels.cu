@@ -274,20 +274,23 @@ __global__ void __launch_bounds__(kPlainThreads) k_plain(const DevView v) {
 // dials of a tile into one of two dial-value buffers while warps 6..7
 // (reducers) form the ordered products and the bin partials of the previous
 // tile from the other buffer, so the serial per-tile phases run beside the
-// next tile's evaluation instead of behind a block barrier.  Hand-over by
-// named barriers, per buffer b: FULL_b (evaluators arrive, reducers wait) and
-// EMPTY_b (reducers arrive, evaluators wait); EVAL among the evaluators
-// before a payload stage is refilled, RED among the reducers.  Every CTA runs
-// the same number of iterations on both sides, so the hand-over cannot
-// deadlock; a timed-out copy marks the block failed and the protocol runs on
-// without work: no further copy is issued, no header is decoded, and before
-// the CTA exits thread 0 waits (bounded) for every copy still in flight.
+// next tile's evaluation instead of behind a block barrier.  Hand-over per
+// buffer b: FULL_b, a named barrier at which the evaluators arrive and the
+// reducers wait, and ebar[b], an mbarrier at which the reducer warps arrive and
+// the evaluators wait.  The evaluator warps never meet: a tile's types differ in
+// cost, and a warp that is done goes on with the next tile, up to the buffer the
+// reducers still hold.  The last evaluator warp to be done with a tile issues
+// the copies of the tile after next into its stage.  Every CTA runs the same
+// number of iterations on both sides and every mbarrier wait is bounded; a
+// timed-out wait marks the block failed and the protocol runs on without work:
+// no further copy is issued, no header is decoded, and before the CTA exits
+// thread 0 waits (bounded) for every copy in flight.
 // ---------------------------------------------------------------------------
 // NEV evaluator threads (192: six warps, the default; 256: eight warps, for
 // double-float, whose tiles hold fewer dials than one round of 192 threads
 // would cover evenly) and two reducer warps.
 constexpr int kWsRed = 64;
-constexpr int kBarEval = 1, kBarFull = 2, kBarEmpty = 4, kBarRed = 6;
+constexpr int kBarFull = 2, kBarRed = 6;
 
 template <typename T, int NEV>
 __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_ws(const DevView v) {
@@ -299,9 +302,10 @@ __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_
   T* dval = (T*)(smem + 2 * TB + 2 * HB);                     // [2][1024]
   double* wsh = (double*)(smem + 2 * TB + 2 * HB + 2048 * sizeof(T));  // [kMaxTileEvents]
   uint16_t* sev = (uint16_t*)(wsh + kMaxTileEvents);      // [kMaxTileEvents]
-  __shared__ uint64_t bar[2];
+  __shared__ uint64_t bar[2], ebar[2];
   __shared__ int s_bstart[kMaxLocalBins], s_bend[kMaxLocalBins];
-  __shared__ volatile int s_fail;
+  __shared__ int s_done[2];                 // evaluator warps done with a stage's tile
+  __shared__ volatile int s_fail, s_issued;  // s_issued: tiles whose copies the CTA has started
 
   const int tid = threadIdx.x;
   const int ntile = (int)blockIdx.x < v.n_tiles ? (v.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x
@@ -310,8 +314,12 @@ __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
+    mbar_init(&ebar[0], kWsRed / 32);
+    mbar_init(&ebar[1], kWsRed / 32);
     fence_mbar_init();
     s_fail = 0;
+    s_done[0] = s_done[1] = 0;
+    s_issued = ntile < 2 ? ntile : 2;
     if (ntile > 0) issue_tile_hdr(v, blockIdx.x, smem, shdr, &bar[0]);
     if (ntile > 1) issue_tile_hdr(v, blockIdx.x + gridDim.x, smem + TB, shdr + hstride, &bar[1]);
   }
@@ -325,19 +333,13 @@ __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_
     int nd = 0, nd_next = 0;
     if (ntile > 0) nd = v.tiles[blockIdx.x].ndials;
     if (ntile > 1) nd_next = v.tiles[blockIdx.x + gridDim.x].ndials;
-    // thread 0: iteration whose copy was last issued into each stage and not
-    // yet seen complete (-1: none)
-    int pend0 = ntile > 0 ? 0 : -1, pend1 = ntile > 1 ? 1 : -1;
     for (int it = 0; it < ntile; ++it) {
       const int tile = blockIdx.x + it * gridDim.x;
       const int st = it & 1;
-      const bool ok = mbar_wait_bounded(&bar[st], (uint32_t)((it >> 1) & 1), kWaitLimitNs);
+      bool ok = !s_fail && mbar_wait_bounded(&bar[st], (uint32_t)((it >> 1) & 1), kWaitLimitNs);
+      if (it >= 2)  // the reducers are done with buffer st (tile it - 2), after a failure too
+        ok &= mbar_wait_bounded(&ebar[st], (uint32_t)(((it >> 1) - 1) & 1), kWaitLimitNs);
       if (!ok) s_fail = 1;
-      if (tid == 0 && ok) {
-        if (st) pend1 = -1;
-        else pend0 = -1;
-      }
-      if (it >= 2) named_sync(kBarEmpty + st, NT);  // the reducers are done with buffer st
       T* dv = dval + st * 1024;
       // after any failed wait the stages hold nothing trustworthy: headers
       // are not decoded, so no shared-memory index comes from them
@@ -352,27 +354,21 @@ __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_
         }
       }
       named_arrive(kBarFull + st, NT);
-      if (it + 1 < ntile) {
-        nd = nd_next;
-        if (it + 2 < ntile) nd_next = v.tiles[tile + 2 * gridDim.x].ndials;
+      __syncwarp();
+      if ((tid & 31) == 0) {
+        __threadfence_block();  // this warp's reads of the stage come first
+        if (atomicAdd(&s_done[st], 1) == kWsEval / 32 - 1) {
+          s_done[st] = 0;
+          // after a failed wait no further copy is issued: a stage whose copy
+          // timed out may still be written by it
+          if (it + 2 < ntile && !s_fail) {
+            issue_tile_hdr(v, tile + 2 * gridDim.x, smem + st * TB, shdr + st * hstride, &bar[st]);
+            s_issued = it + 3;
+          }
+        }
       }
-      named_sync(kBarEval, kWsEval);  // stage st (payload and headers) fully read; s_fail visible
-      // after a failed wait no further copy is issued: a stage whose copy
-      // timed out may still be written by it
-      if (tid == 0 && it + 2 < ntile && !s_fail) {
-        issue_tile_hdr(v, tile + 2 * gridDim.x, smem + st * TB, shdr + st * hstride, &bar[st]);
-        if (st) pend1 = it + 2;
-        else pend0 = it + 2;
-      }
-    }
-    // the reducers' last two EMPTY arrivals, so every named-barrier phase
-    // gets its full count of threads
-    for (int j = ntile >= 2 ? ntile - 2 : 0; j < ntile; ++j) named_sync(kBarEmpty + (j & 1), NT);
-    // after a failure, wait (bounded) for every copy still in flight before
-    // the CTA's shared memory is released
-    if (tid == 0 && s_fail) {
-      if (pend0 >= 0) mbar_wait_bounded(&bar[0], (uint32_t)((pend0 >> 1) & 1), kWaitLimitNs);
-      if (pend1 >= 0) mbar_wait_bounded(&bar[1], (uint32_t)((pend1 >> 1) & 1), kWaitLimitNs);
+      nd = nd_next;
+      if (it + 2 < ntile) nd_next = v.tiles[tile + 2 * gridDim.x].ndials;
     }
   } else {
     const int r = tid - kWsEval;
@@ -433,7 +429,8 @@ __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_
         if (e == 0 || ev_lbin(sev[e - 1]) != lb) s_bstart[lb] = e;
         if (e + 1 == td.nevents || ev_lbin(sev[e + 1]) != lb) s_bend[lb] = e + 1;
       }
-      named_arrive(kBarEmpty + b, NT);  // buffer b consumed
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ebar[b]);  // buffer b consumed
       named_sync(kBarRed, kWsRed);
       // one warp per local bin (two warps: bins w, w + 2): fixed-order FP64 sums
       for (int lb = rwarp; lb < (int)td.nbins; lb += 2) {
@@ -459,7 +456,14 @@ __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_
     }
   }
   __syncthreads();
-  if (tid == 0 && s_fail) atomicOr(v.status, kStatusCopyTimeout);
+  if (tid == 0 && s_fail) {
+    atomicOr(v.status, kStatusCopyTimeout);
+    // the copies that may still be in flight, the last two issued, land
+    // (bounded) before the CTA's shared memory is released
+    const int n = s_issued;
+    for (int j = n > 2 ? n - 2 : 0; j < n; ++j)
+      mbar_wait_bounded(&bar[j & 1], (uint32_t)((j >> 1) & 1), kWaitLimitNs);
+  }
 }
 
 // ---------------------------------------------------------------------------

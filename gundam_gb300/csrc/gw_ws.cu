@@ -6,10 +6,13 @@
 // and write the dial's KP values into its event-major slot of a [slot][KP]
 // buffer; two reducer warps form each event's ordered product
 // (EventDialCache.cpp:156-171) for the KP points and reduce w and w^2 per
-// (tile, bin, point) in FP64, one warp per (local bin, point), lanes over the
-// bin's events in a fixed order.  Two value buffers alternate between the two
-// sides (named barriers FULL_b / EMPTY_b), so the next chunk of points (or the
-// next tile) is evaluated while the reducers empty the previous one.  A tile's
+// (tile, bin, point) in FP64, one warp per local bin, lanes over the points and
+// the bin's events in a fixed order.  Two value buffers alternate between the two
+// sides (FULL_b, a named barrier at which the evaluators arrive and the reducers
+// wait; ebar[b], an mbarrier at which the reducer warps arrive and the evaluators
+// wait), so the next chunk of points (or the next tile) is evaluated while the
+// reducers empty the previous one, and the evaluator warps never wait for one
+// another.  A tile's
 // payload and headers arrive by one bulk copy and stay in shared memory for
 // all ceil(K / KP) chunks, so HBM sees each dial once per K points; at small
 // K the kernel stays bound by HBM bandwidth, as the K = 1 kernel is, while
@@ -17,9 +20,9 @@
 // points and pairs of points go through the packed FP32 (f32x2) arithmetic.
 //
 // Every CTA runs the same number of hand-overs on both sides (each named
-// barrier phase gets its full thread count), so the protocol cannot
-// deadlock.  A bulk-copy wait that gives up marks the block failed: no
-// further copy is issued, no header is decoded, and thread 0 waits (bounded)
+// barrier phase gets its full thread count) and every mbarrier wait is bounded,
+// so the protocol cannot deadlock.  A wait that gives up marks the block failed:
+// no further copy is issued, no header is decoded, and thread 0 waits (bounded)
 // for the copies still in flight before the CTA exits.
 #include "gw_device.cuh"
 
@@ -27,7 +30,7 @@ namespace gw {
 namespace {
 
 constexpr int kSEval = 192, kSRed = 64, kSThreads = kSEval + kSRed;
-constexpr int kSBarEval = 1, kSBarFull = 2, kSBarEmpty = 4, kSBarRed = 6;
+constexpr int kSBarFull = 2, kSBarRed = 6;
 
 // The KP values of one slot: stores, loads and the elementwise product.
 template <typename T, int KP>
@@ -74,7 +77,7 @@ __device__ __forceinline__ void slot_mul(T (&w)[KP], const T* src) {
 
 // Shared memory (all sizes multiples of 16 bytes):
 //   [2][TB] payload stages | [2][HB] tile headers (tile order) |
-//   [2][NS][KP] dial values (NS = HB / 8 slots) | [KP][256] FP64 event
+//   [2][NS][KP] dial values (NS = HB / 8 slots) | [256][KP] FP64 event
 //   weights | [256] base weights | [264] event words
 template <typename T, int KP>
 size_t ws_bytes(const DevView& v) {
@@ -92,10 +95,12 @@ __global__ void __launch_bounds__(kSThreads, MB) k_ws(const DevView v, int K) {
   const int NS = HB / 8;
   uint64_t* shdr = (uint64_t*)(smem + 2 * TB);                     // [2][NS]
   T* dval = (T*)(smem + 2 * TB + 2 * HB);                          // [2][NS][KP]
-  double* wsh = (double*)(dval + 2 * (size_t)NS * KP);             // [KP][256]
+  double* wsh = (double*)(dval + 2 * (size_t)NS * KP);             // [256][KP]
   T* sw0 = (T*)(wsh + kMaxTileEvents * KP);                        // [256]
   uint16_t* sev = (uint16_t*)(sw0 + kMaxTileEvents);               // [264]
-  __shared__ uint64_t bar[2];
+  __shared__ uint64_t bar[2], ebar[2];
+  __shared__ int s_done[2];        // evaluator warps done with a stage's tile
+  __shared__ volatile int s_issued;  // tiles whose copies the CTA has started
   __shared__ int s_bstart[kMaxLocalBins], s_bend[kMaxLocalBins];
   __shared__ volatile int s_fail;
 
@@ -104,12 +109,15 @@ __global__ void __launch_bounds__(kSThreads, MB) k_ws(const DevView v, int K) {
                         ? (v.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x
                         : 0;
   const int nch = (K + KP - 1) / KP;
-  const int Q = ntile * nch;
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
+    mbar_init(&ebar[0], kSRed / 32);
+    mbar_init(&ebar[1], kSRed / 32);
     fence_mbar_init();
     s_fail = 0;
+    s_done[0] = s_done[1] = 0;
+    s_issued = ntile < 2 ? ntile : 2;
     if (ntile > 0) issue_tile_hdr(v, blockIdx.x, smem, shdr, &bar[0]);
     if (ntile > 1) issue_tile_hdr(v, blockIdx.x + gridDim.x, smem + TB, shdr + NS, &bar[1]);
   }
@@ -120,22 +128,18 @@ __global__ void __launch_bounds__(kSThreads, MB) k_ws(const DevView v, int K) {
     int nd = 0, nd_next = 0;
     if (ntile > 0) nd = v.tiles[blockIdx.x].ndials;
     if (ntile > 1) nd_next = v.tiles[blockIdx.x + gridDim.x].ndials;
-    int pend0 = ntile > 0 ? 0 : -1, pend1 = ntile > 1 ? 1 : -1;  // thread 0: copy in flight per stage
     for (int it = 0; it < ntile; ++it) {
       const int tile = blockIdx.x + it * gridDim.x;
       const int st = it & 1;
-      const bool ok = mbar_wait_bounded(&bar[st], (uint32_t)((it >> 1) & 1), kWaitLimitNs);
-      if (!ok) s_fail = 1;
-      if (tid == 0 && ok) {
-        if (st) pend1 = -1;
-        else pend0 = -1;
-      }
+      bool ok = !s_fail && mbar_wait_bounded(&bar[st], (uint32_t)((it >> 1) & 1), kWaitLimitNs);
       const T* pl = (const T*)(smem + st * TB);
       const uint64_t* hs = shdr + st * NS;
       for (int c = 0; c < nch; ++c) {
         const int q = it * nch + c;
         const int b = q & 1;
-        if (q >= 2) named_sync(kSBarEmpty + b, kSThreads);  // the reducers are done with buffer b
+        if (q >= 2)  // the reducers are done with buffer b (chunk q - 2), after a failure too
+          ok &= mbar_wait_bounded(&ebar[b], (uint32_t)(((q >> 1) - 1) & 1), kWaitLimitNs);
+        if (!ok) s_fail = 1;
         if (ok && !s_fail) {
           T* dv = dval + (size_t)b * NS * KP;
           for (int i = tid; i < nd; i += kSEval) {
@@ -147,22 +151,19 @@ __global__ void __launch_bounds__(kSThreads, MB) k_ws(const DevView v, int K) {
         }
         named_arrive(kSBarFull + b, kSThreads);
       }
-      if (it + 1 < ntile) {
-        nd = nd_next;
-        if (it + 2 < ntile) nd_next = v.tiles[tile + 2 * gridDim.x].ndials;
+      __syncwarp();
+      if ((tid & 31) == 0) {
+        __threadfence_block();  // this warp's reads of the stage come first
+        if (atomicAdd(&s_done[st], 1) == kSEval / 32 - 1) {
+          s_done[st] = 0;
+          if (it + 2 < ntile && !s_fail) {
+            issue_tile_hdr(v, tile + 2 * gridDim.x, smem + st * TB, shdr + st * NS, &bar[st]);
+            s_issued = it + 3;
+          }
+        }
       }
-      named_sync(kSBarEval, kSEval);  // stage st fully read; s_fail visible
-      if (tid == 0 && it + 2 < ntile && !s_fail) {
-        issue_tile_hdr(v, tile + 2 * gridDim.x, smem + st * TB, shdr + st * NS, &bar[st]);
-        if (st) pend1 = it + 2;
-        else pend0 = it + 2;
-      }
-    }
-    // the reducers' last two EMPTY arrivals
-    for (int q = Q >= 2 ? Q - 2 : 0; q < Q; ++q) named_sync(kSBarEmpty + (q & 1), kSThreads);
-    if (tid == 0 && s_fail) {
-      if (pend0 >= 0) mbar_wait_bounded(&bar[0], (uint32_t)((pend0 >> 1) & 1), kWaitLimitNs);
-      if (pend1 >= 0) mbar_wait_bounded(&bar[1], (uint32_t)((pend1 >> 1) & 1), kWaitLimitNs);
+      nd = nd_next;
+      if (it + 2 < ntile) nd_next = v.tiles[tile + 2 * gridDim.x].ndials;
     }
   } else {
     // ---------------- reducers ----------------
@@ -227,28 +228,33 @@ __global__ void __launch_bounds__(kSThreads, MB) k_ws(const DevView v, int K) {
           for (int j = 0; j < KP; ++j) {
             T wj = w[j];
             if (v.has_cap && wj > (T)v.cap) wj = (T)v.cap;
-            wsh[j * kMaxTileEvents + e] = (double)(w0 * wj);
+            wsh[e * KP + j] = (double)(w0 * wj);
           }
         }
-        named_arrive(kSBarEmpty + b, kSThreads);  // buffer b consumed
-        named_sync(kSBarRed, kSRed);              // wsh and the bin markers complete
-        // one warp per (local bin, point): fixed-order FP64 sums of w and w^2
-        for (int task = rwarp; task < (int)td.nbins * KP; task += kSRed / 32) {
-          const int lb = task / KP, j = task - lb * KP;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ebar[b]);  // buffer b consumed
+        named_sync(kSBarRed, kSRed);           // wsh and the bin markers complete
+        // one warp per local bin, a lane per point and one of 32 / KP event
+        // lanes: fixed-order FP64 sums of w and w^2 (a warp per bin and point,
+        // with a shuffle tree over 32 lanes each, took KP times the steps and
+        // kept the evaluators waiting for the buffer)
+        for (int lb = rwarp; lb < (int)td.nbins; lb += kSRed / 32) {
+          const int j = lane % KP;
           const int kg = c * KP + j;
           const int b0 = s_bstart[lb], b1 = s_bend[lb];
-          if (b1 > b0 && kg < K) {
+          if (b1 > b0) {
             double sw = 0.0, sw2 = 0.0;
-            for (int e = b0 + lane; e < b1; e += 32) {
-              const double w = wsh[j * kMaxTileEvents + e];
+            for (int e = b0 + lane / KP; e < b1; e += 32 / KP) {
+              const double w = wsh[e * KP + j];
               sw += w;
               sw2 += w * w;
             }
-            for (int o = 16; o; o >>= 1) {
+#pragma unroll
+            for (int o = 16; o >= KP; o >>= 1) {
               sw += __shfl_xor_sync(0xffffffffu, sw, o);
               sw2 += __shfl_xor_sync(0xffffffffu, sw2, o);
             }
-            if (lane == 0) {
+            if (lane < KP && kg < K) {
               const int slot = (lb == 0) ? (int)td.slot0 : v.bin_slot[td.bin0 + lb];
               v.partials[(size_t)slot * v.kpad + kg] = make_double2(sw, sw2);
             }
@@ -259,7 +265,14 @@ __global__ void __launch_bounds__(kSThreads, MB) k_ws(const DevView v, int K) {
     }
   }
   __syncthreads();
-  if (tid == 0 && s_fail) atomicOr(v.status, kStatusCopyTimeout);
+  if (tid == 0 && s_fail) {
+    atomicOr(v.status, kStatusCopyTimeout);
+    // the copies that may still be in flight, the last two issued, land
+    // (bounded) before the CTA's shared memory is released
+    const int n = s_issued;
+    for (int j = n > 2 ? n - 2 : 0; j < n; ++j)
+      mbar_wait_bounded(&bar[j & 1], (uint32_t)((j >> 1) & 1), kWaitLimitNs);
+  }
 }
 
 template <typename T, int KP, int MB>
