@@ -238,9 +238,8 @@ __device__ __forceinline__ void row_store(bf16* p, int n, bool vec, const bf16 (
 // Every wait is bounded; on a timeout the tile records the failure in
 // *status, drains its own copies (bounded) and frees TMEM.
 template <int BN, int S, int NW>
-__global__ void __launch_bounds__(NW * 32) k_gemm(const __grid_constant__ CUtensorMap tmA,
-                                                  const __grid_constant__ CUtensorMap tmB, int M, int N, int K,
-                                                  Epilogue ep, uint32_t* status) {
+__device__ __forceinline__ void gemm_tile(const CUtensorMap& tmA, const CUtensorMap& tmB, int m0, int n0, int M,
+                                          int N, int K, const Epilogue& ep, uint32_t* status) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   constexpr int kA = kBM * kBK * 2;  // 16 KB
@@ -255,7 +254,6 @@ __global__ void __launch_bounds__(NW * 32) k_gemm(const __grid_constant__ CUtens
   __shared__ volatile int failed;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * BN;
   if (warp == 0) tmem_alloc(&tmem_base, BN);
   if (tid == 0) {
     for (int i = 0; i < S; ++i) {
@@ -426,6 +424,37 @@ __global__ void __launch_bounds__(NW * 32) k_gemm(const __grid_constant__ CUtens
     for (int w = 0; w < NW; ++w) t += sloss[w];
     atomicAdd(ep.loss, t * ep.inv * ep.scale);
   }
+}
+
+template <int BN, int S, int NW>
+__global__ void __launch_bounds__(NW * 32) k_gemm(const __grid_constant__ CUtensorMap tmA,
+                                                  const __grid_constant__ CUtensorMap tmB, int M, int N, int K,
+                                                  Epilogue ep, uint32_t* status) {
+  gemm_tile<BN, S, NW>(tmA, tmB, blockIdx.y * kBM, blockIdx.x * BN, M, N, K, ep, status);
+}
+
+// Products of one K that do not depend on one another, in one launch: the tiles
+// of product i are the blocks [tile0[i], tile0[i + 1]).  The weight gradients
+// are such a set once the output gradients of all layers are there.  One after
+// another they left most of the chip idle: of 2048 rows the hidden layers' 512 x
+// 512 products are 64 tiles each and the launches took 15 + 15 + 15 + 18 us;
+// together they take 17 us.
+constexpr int kMaxGroup = 8;
+struct GemmGroup {
+  CUtensorMap a[kMaxGroup], b[kMaxGroup];
+  float* out[kMaxGroup];  // [M x N]
+  int M[kMaxGroup], N[kMaxGroup], tile0[kMaxGroup + 1];
+  int n, K;
+};
+
+template <int BN, int S, int NW>
+__global__ void __launch_bounds__(NW * 32) k_gemm_group(const __grid_constant__ GemmGroup g, uint32_t* status) {
+  int i = 0;
+  while (i + 1 < g.n && (int)blockIdx.x >= g.tile0[i + 1]) ++i;
+  const int N = g.N[i], t = blockIdx.x - g.tile0[i], cols = (N + BN - 1) / BN;
+  Epilogue ep{};
+  ep.out_f32 = g.out[i];
+  gemm_tile<BN, S, NW>(g.a[i], g.b[i], t / cols * kBM, t % cols * BN, g.M[i], N, g.K, ep, status);
 }
 
 // ---- small kernels ----
@@ -1402,26 +1431,94 @@ static int launch_gemm(gwm_net* n, const bf16* A, const bf16* B, int M, int N, i
   return GW_OK;
 }
 
+struct Product {
+  const bf16 *A, *B;
+  float* out;
+  int M, N;
+};
+
+template <int BN, int S, int NW>
+static int launch_group(gwm_net* n, const Product* p, int cnt, int K) {
+  gwm::GemmGroup g;
+  g.n = cnt;
+  g.K = K;
+  g.tile0[0] = 0;
+  for (int i = 0; i < cnt; ++i) {
+    int rc = make_map(n, &g.a[i], p[i].A, p[i].M, K, gwm::kBM);
+    if (!rc) rc = make_map(n, &g.b[i], p[i].B, p[i].N, K, BN);
+    if (rc) return rc;
+    g.out[i] = p[i].out;
+    g.M[i] = p[i].M;
+    g.N[i] = p[i].N;
+    g.tile0[i + 1] = g.tile0[i] + ((p[i].N + BN - 1) / BN) * ((p[i].M + gwm::kBM - 1) / gwm::kBM);
+  }
+  const size_t smem = gemm_smem(BN, S);
+  static std::once_flag once;
+  std::call_once(once, [smem]() {
+    cudaFuncSetAttribute(gwm::k_gemm_group<BN, S, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
+  launch_dependent(gwm::k_gemm_group<BN, S, NW>, g.tile0[cnt], NW * 32, smem, n->stream, g, n->status);
+  GWM_CUDA(n, cudaGetLastError());
+  return GW_OK;
+}
+
+constexpr int kWave = 148;  // tiles that give (nearly) each of GB300's 152 SMs one
+
+static int tiles(int M, int N, int BN) { return ((M + gwm::kBM - 1) / gwm::kBM) * ((N + BN - 1) / BN); }
+
 // C[M x N] = A[M x K] * B[N x K]^T with the given epilogue.  The widest tile
 // that still gives one CTA per SM or more (148 of GB300's 152): at the
 // network's sizes a launch is one wave, and a tile runs few K steps, so more
-// CTAs, not wider tiles, keep the chip busy.  128 x 256 tiles take a ring of
-// two stages, so that two CTAs (and their accumulators, 256 TMEM columns each)
-// share an SM and one's epilogue overlaps the other's MMAs.  Where even
-// 64-column tiles leave half of the SMs idle (few rows, or the weight
-// gradients of the hidden layers), 32-column tiles with a ring of eight
-// stages: a product is then one latency chain per CTA, and eight stages put
-// the whole of K = 512 in flight at once (64 rows, N = K = 512: 17 us with
-// 64-column tiles and four stages, 9 us now; 3000 columns: 10.4 -> 8 us).
+// CTAs, not wider tiles, keep the chip busy.
+//   * 128 x 256 tiles take a ring of two stages, so that two CTAs (and their
+//     accumulators, 256 TMEM columns each) share an SM and one's epilogue
+//     overlaps the other's MMAs.
+//   * With the loss in the epilogue and up to three such tiles per SM, 64-column
+//     tiles instead: a thread then has the targets of all its columns on the way
+//     before it waits for the accumulator, and the last wave is finer (3000
+//     outputs, K = 512, a whole training step: 2048 rows 159 -> 155 us, 4096
+//     rows 253 -> 239; 8192 rows 461 -> 465, and 128-column tiles at 1024 rows
+//     122 -> 125, which therefore stay).
+//   * 64-column tiles that share no SM take eight stages: the K steps are a chain
+//     of L2 latencies over the ring's depth (K = 3000, M = 2048, N = 512: 24 ->
+//     11 us), and four only where a second tile shares the SM.
+//   * Where even 64-column tiles leave half of the SMs idle (few rows),
+//     32-column tiles with a ring of eight stages (64 rows, N = K = 512: 17 us
+//     with 64-column tiles and four stages, 9 us now; 3000 columns: 10.4 -> 8 us).
 // The tile shape does not change the order of any accumulation.
 static int gemm(gwm_net* n, const bf16* A, const bf16* B, int M, int N, int K, const gwm::Epilogue& ep) {
   if (K % 8 != 0) return gwm_fail(n, GW_ERR_ARG, "GEMM K must be a multiple of 8");
-  const int tiles_m = (M + gwm::kBM - 1) / gwm::kBM;
-  constexpr int kWave = 148;
-  if (N > 128 && tiles_m * ((N + 255) / 256) >= kWave) return launch_gemm<256, 2, 8>(n, A, B, M, N, K, ep);
-  if (N > 64 && tiles_m * ((N + 127) / 128) >= kWave) return launch_gemm<128, 4, 8>(n, A, B, M, N, K, ep);
-  if (N > 32 && tiles_m * ((N + 63) / 64) >= kWave / 2) return launch_gemm<64, 4, 8>(n, A, B, M, N, K, ep);
+  const int t256 = tiles(M, N, 256), t64 = tiles(M, N, 64);
+  if (N > 128 && t256 >= kWave && !(ep.target && t256 < 3 * kWave))
+    return launch_gemm<256, 2, 8>(n, A, B, M, N, K, ep);
+  if (N > 64 && t256 < kWave && tiles(M, N, 128) >= kWave) return launch_gemm<128, 4, 8>(n, A, B, M, N, K, ep);
+  if (N > 32 && t64 > 152) return launch_gemm<64, 4, 8>(n, A, B, M, N, K, ep);
+  if (N > 32 && t64 >= kWave / 2) return launch_gemm<64, 8, 8>(n, A, B, M, N, K, ep);
   return launch_gemm<32, 8, 4>(n, A, B, M, N, K, ep);
+}
+
+// The products p[0..cnt), all of depth K, in launches of kMaxGroup.  The widest
+// tiles that give half of the SMs one each, with rings as deep as one tile per
+// SM allows.  2048 rows of 200-512-512-512-3000 (136 tiles of 128 columns, 272
+// of 64 in rings of four, two to an SM, or in rings of eight): a training step
+// takes 155, 157 and 168 us, and 190 us with 32-column tiles; 256 rows: 97, 98,
+// 100 and 106.
+static int gemm_set(gwm_net* n, const Product* p, int cnt, int K) {
+  if (K % 8 != 0) return gwm_fail(n, GW_ERR_ARG, "GEMM K must be a multiple of 8");
+  for (; cnt > 0; p += gwm::kMaxGroup, cnt -= gwm::kMaxGroup) {
+    const int c = cnt < gwm::kMaxGroup ? cnt : gwm::kMaxGroup;
+    int t128 = 0, t64 = 0;
+    for (int i = 0; i < c; ++i) {
+      t128 += tiles(p[i].M, p[i].N, 128);
+      t64 += tiles(p[i].M, p[i].N, 64);
+    }
+    int rc;
+    if (t128 >= kWave / 2) rc = launch_group<128, 6, 8>(n, p, c, K);
+    else if (t64 >= kWave / 2) rc = launch_group<64, 8, 8>(n, p, c, K);
+    else rc = launch_group<32, 8, 4>(n, p, c, K);
+    if (rc) return rc;
+  }
+  return GW_OK;
 }
 
 static int check_status(gwm_net* n) {
@@ -1641,24 +1738,20 @@ static int backward(gwm_net* n, int B) {
   const int L = n->n_layers;
   // dz[L-1] (and its transpose) was written by the forward pass's loss epilogue;
   // the bias gradients follow from the dzt (k_adam, k_bias_grad)
-  for (int l = L - 1; l >= 0; --l) {
-    // dW_l = dz_l^T h_l : [dims[l+1] x dims[l]], K = B
-    gwm::Epilogue e1{};
-    e1.out_f32 = n->gw_[l];
-    int rc = gemm(n, n->dzt[l], n->ht[l], n->dims[l + 1], n->dims[l], B, e1);
+  for (int l = L - 1; l > 0; --l) {
+    // dz_{l-1} = (dz_l W_l) * silu'(z_{l-1}) : [B x dims[l]], K = dims[l+1]
+    gwm::Epilogue ep{};
+    ep.gate = n->z[l - 1];
+    ep.out_bf16 = n->dz[l - 1];
+    ep.out_bf16_t = n->dzt[l - 1];
+    ep.ld_t = B;
+    int rc = gemm(n, n->dz[l], n->wt[l], B, n->dims[l], n->dims[l + 1], ep);
     if (rc) return rc;
-    if (l > 0) {
-      // dz_{l-1} = (dz_l W_l) * silu'(z_{l-1}) : [B x dims[l]], K = dims[l+1]
-      gwm::Epilogue e2{};
-      e2.gate = n->z[l - 1];
-      e2.out_bf16 = n->dz[l - 1];
-      e2.out_bf16_t = n->dzt[l - 1];
-      e2.ld_t = B;
-      rc = gemm(n, n->dz[l], n->wt[l], B, n->dims[l], n->dims[l + 1], e2);
-      if (rc) return rc;
-    }
   }
-  return GW_OK;
+  // dW_l = dz_l^T h_l : [dims[l+1] x dims[l]], K = B
+  std::vector<Product> dw(L);
+  for (int l = 0; l < L; ++l) dw[l] = {n->dzt[l], n->ht[l], n->gw_[l], n->dims[l + 1], n->dims[l]};
+  return gemm_set(n, dw.data(), L, B);
 }
 
 // Forward pass with the loss against host or device targets t [B x dims[L]] in *n->loss.
