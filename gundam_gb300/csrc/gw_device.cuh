@@ -9,6 +9,7 @@
 #include "gw_dials.cuh"
 #include "gw_internal.h"
 #include "gw_launch.h"
+#include "gw_log.cuh"
 
 namespace gw {
 namespace {
@@ -395,29 +396,40 @@ __device__ __forceinline__ double llh_poisson(double data, double pred) {
 }
 
 // log(data) as the Barlow-Beeston term uses it (bins with data only).
-__device__ __forceinline__ double log_data_of(double data) { return data > DBL_EPSILON ? log(data) : 0.0; }
+__device__ __forceinline__ double log_data_of(double data) {
+  if (!(data > DBL_EPSILON)) return 0.0;
+  return positive_normal(data) ? log_normal(data) : log(data);
+}
 
-__device__ __forceinline__ double llh_bb_oa2021(double data, double log_data, double pred, double mcuncert) {
-  // BarlowBeestonBanff2022.h:150-294 with its defaults (expectedValueMinimum
-  // = -1, fractionalErrorLimit = 1e150, usePoissonLikelihood = false).
-  if (pred <= -1.0) {
+// BarlowBeestonBanff2022.h:150-294 with its defaults (expectedValueMinimum
+// = -1, fractionalErrorLimit = 1e150, usePoissonLikelihood = false); root =
+// sqrt(mcuncert).  Its FP64 operations bound k_bins_llh, so the tests that
+// nearly always go one way look at the high words first, and the logarithm is
+// that of gw_log.cuh (10000 bins, 100 points: 232 -> 203 us with both).
+__device__ __forceinline__ double llh_bb_oa2021(double data, double log_data, double pred, double mcuncert,
+                                                double root) {
+  if (__double2hiint(pred) < 0 && pred <= -1.0) {
     if (pred <= 0.0 && data > 0.0) return HUGE_VAL;
     return 0.0;
   }
   double newmc = pred;
   double penalty = 0.0;
-  if (mcuncert > 0.0) {
-    const double fractional = fmin(sqrt(mcuncert) / pred, 1.0e150);
+  if (positive_normal(mcuncert) || mcuncert > 0.0) {
+    double fractional = root / pred;
+    if (__double2hiint(fractional) >= 0x5f138d35) fractional = fmin(fractional, 1.0e150);  // from 9.99e149
     const double temp = pred * fractional * fractional - 1;
     const double temp2 = temp * temp + 4 * data * fractional * fractional;
-    if (temp2 < 0) return HUGE_VAL;
+    if (__double2hiint(temp2) < 0 && temp2 < 0) return HUGE_VAL;
     const double beta = (-1 * temp + sqrt(temp2)) / 2.;
-    newmc = fmax(pred * beta, DBL_MIN);
+    newmc = pred * beta;
+    if (!positive_normal(newmc)) newmc = fmax(newmc, DBL_MIN);
     penalty = (beta - 1) * (beta - 1) / (2 * fractional * fractional);
   }
   double stat;
-  if (data <= DBL_EPSILON) {
+  if (__double2hiint(data) <= 0x3cb00000 && data <= DBL_EPSILON) {  // 2^-52
     stat = newmc;
+  } else if (positive_normal(newmc)) {
+    stat = newmc - data + data * (log_data - log_normal(newmc));
   } else if (newmc > DBL_MIN) {
     stat = newmc - data + data * (log_data - log(newmc));
   } else {
@@ -430,12 +442,14 @@ __device__ __forceinline__ double llh_bb_oa2021(double data, double log_data, do
 // One Barlow-Beeston bin from the histogram's (sum of w, sqrt of sum of w^2),
 // as BarlowBeestonBanff2022::eval(const SamplePair&, int) takes it
 // (BarlowBeestonBanff2022.h:92-148): the stored sqrt squared again, and +inf
-// for a non-finite value (the reference's throwIfInfLlh = false branch).
+// for a non-finite value (the reference's throwIfInfLlh = false branch).  The
+// square root of a rounded square is the number itself (radix 2, round to
+// nearest, no underflow), so it is not taken again.
 __device__ __forceinline__ double llh_bb_bin(double data, double log_data, double pred, double sqrt_sum_w2) {
-  double mcuncert = sqrt_sum_w2;
-  mcuncert *= mcuncert;
-  if (!isfinite(mcuncert) || mcuncert < 0.0) return HUGE_VAL;
-  return llh_bb_oa2021(data, log_data, pred, mcuncert);
+  const double mcuncert = sqrt_sum_w2 * sqrt_sum_w2;
+  if ((__double2hiint(mcuncert) & 0x7ff00000) == 0x7ff00000) return HUGE_VAL;
+  const double root = positive_normal(mcuncert) ? fabs(sqrt_sum_w2) : sqrt(mcuncert);
+  return llh_bb_oa2021(data, log_data, pred, mcuncert, root);
 }
 
 }  // namespace

@@ -477,10 +477,13 @@ __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_
 //      likelihood term; the BT terms of a point are added by a shuffle tree;
 //   3. the last block of a point tile adds its blocks' parts and the penalty's
 //      in a fixed order.
-// A Barlow-Beeston term is ~150 FP64 instructions and an SM issues one warp of
-// them every 16 cycles, so the terms are cut into many small blocks with full
-// warps: 256 bins per block left 140 SMs idle at K = 1 (19.2 us for 3000 bins,
-// now 14.8 us; the launch alone is 5 us).  The small KT give their threads to the slots of a bin instead,
+// A Barlow-Beeston term is ~80 FP64 operations and an SM issues one warp of
+// them every 16 cycles (pipe busy 84 % at 10000 bins, 100 points: 203 us, 232
+// with CUDA's logarithm, a third square root and FP64 compares; see
+// llh_bb_oa2021), so the terms are cut into many small blocks with full warps:
+// 256 bins per block left 140 SMs idle at K = 1 (19.2 us for 3000 bins, now
+// 13.5 us; the launch alone is 5 us).  The small KT give their threads to the
+// slots of a bin instead,
 // whose reads are a chain of L2 latencies.
 template <int KT, int BT>
 __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double* sums, double* sums2,
