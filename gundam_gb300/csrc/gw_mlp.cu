@@ -1296,6 +1296,9 @@ struct gwm_net {
   int batch_max = 0;
   int device = 0;
   cudaStream_t stream = nullptr;
+  // the base's gradient beside the network's (gwm_value_grad), made on first use
+  cudaStream_t side = nullptr;
+  cudaEvent_t side_go = nullptr, side_done = nullptr;
   std::vector<void*> allocs;
   // per layer l (0..L-1): weights [dims[l+1] x dims[l]]
   std::vector<float*> w, b, gw_, gb, mw, vw, mb, vb;
@@ -1578,6 +1581,12 @@ extern "C" int gwm_destroy(gwm_net* n) {
   if (!n) return GW_ERR_ARG;
   cudaSetDevice(n->device);
   cudaStreamSynchronize(n->stream);
+  if (n->side) {
+    cudaStreamSynchronize(n->side);
+    cudaStreamDestroy(n->side);
+  }
+  if (n->side_go) cudaEventDestroy(n->side_go);
+  if (n->side_done) cudaEventDestroy(n->side_done);
   for (void* p : n->allocs) cudaFree(p);
   cudaFree(n->train_x);
   cudaFree(n->train_t);
@@ -2004,7 +2013,7 @@ static int launch_head(gwm_net* n, int C, int llh_type, const gwm::HeadOut& out)
 }
 
 // The base's part of the input gradient, eight parts per (point, parameter) in g_gz.
-static int launch_base_grad(gwm_net* n, int C) {
+static int launch_base_grad(gwm_net* n, int C, cudaStream_t stream) {
   const int din = n->dims[0], nb = n->dims[n->n_layers];
   const size_t shb = sizeof(float) * 2 * (size_t)nb;
   if (shb > 200 * 1024) return gwm_fail(n, GW_ERR_LIMIT, "gwm_value_grad: too many bins");
@@ -2019,7 +2028,7 @@ static int launch_base_grad(gwm_net* n, int C) {
     });
     constexpr int kTile = 8 * gwm::kGradM;
     const dim3 grid(8, (din + gwm::kGradK - 1) / gwm::kGradK, (C + kTile - 1) / kTile);
-    launch_dependent(gwm::k_base_grad_staged, grid, 256, kShm, n->stream,
+    launch_dependent(gwm::k_base_grad_staged, grid, 256, kShm, stream,
                      tab, rw, head_view(n), n->xin, n->g_G, n->g_S, C, n->g_gz, n->status);
   } else {
     if (shb > 48 * 1024) {
@@ -2028,7 +2037,7 @@ static int launch_base_grad(gwm_net* n, int C) {
         cudaFuncSetAttribute(gwm::k_base_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       });
     }
-    launch_dependent(gwm::k_base_grad, dim3(C, (din + 7) / 8), 256, shb, n->stream,
+    launch_dependent(gwm::k_base_grad, dim3(C, (din + 7) / 8), 256, shb, stream,
                      head_view(n), n->xin, n->g_G, n->g_S, n->g_gz);
   }
   GWM_CUDA(n, cudaGetLastError());
@@ -2580,6 +2589,9 @@ extern "C" int gwm_value_grad(gwm_net* n, const double* theta, int32_t C, int32_
              gwm_alloc(n, &n->g_f, Bm) | gwm_alloc(n, &n->g_grad, (size_t)Bm * din);
     if (rc) return rc;
   }
+  if (!n->side) GWM_CUDA(n, cudaStreamCreateWithFlags(&n->side, cudaStreamNonBlocking));
+  if (!n->side_go) GWM_CUDA(n, cudaEventCreateWithFlags(&n->side_go, cudaEventDisableTiming));
+  if (!n->side_done) GWM_CUDA(n, cudaEventCreateWithFlags(&n->side_done, cudaEventDisableTiming));
   if (Bp > C) GWM_CUDA(n, cudaMemsetAsync(n->h_theta, 0, sizeof(double) * (size_t)Bp * din, n->stream));
   GWM_CUDA(n, cudaMemcpyAsync(n->h_theta, theta, sizeof(double) * (size_t)C * din, cudaMemcpyHostToDevice, n->stream));
   gwm::k_standardize<<<(unsigned)(((size_t)Bp * din + 255) / 256), 256, 0, n->stream>>>(
@@ -2597,10 +2609,21 @@ extern "C" int gwm_value_grad(gwm_net* n, const double* theta, int32_t C, int32_
   out.S = n->g_S;
   out.dy = n->dz[L - 1];
   rc = launch_head<true>(n, C, llh_type, out);
-  if (!rc) rc = backward_dx(n, Bp);
   if (rc) return rc;
-  rc = launch_base_grad(n, C);
-  if (rc) return rc;
+  // The base's gradient and the network's input gradient need only the head's
+  // results: the first bounds 152 SMs by shared-memory reads (33 us at 64 points,
+  // 200 parameters, 3000 bins), the second is a chain of four latency-bound
+  // products on 7 to 16 SMs (27 us), so they run side by side (a call 215 -> 195
+  // us; 16 parameters, 200 bins, one point: 117 either way).  Whatever fails, the
+  // network's stream goes on only after both.
+  GWM_CUDA(n, cudaEventRecord(n->side_go, n->stream));
+  GWM_CUDA(n, cudaStreamWaitEvent(n->side, n->side_go, 0));
+  rc = launch_base_grad(n, C, n->side);
+  const cudaError_t rec = cudaEventRecord(n->side_done, n->side);
+  const int rc2 = rc ? rc : backward_dx(n, Bp);
+  GWM_CUDA(n, rec);
+  GWM_CUDA(n, cudaStreamWaitEvent(n->stream, n->side_done, 0));
+  if (rc2) return rc2;
   const int P32 = (din + 31) & ~31;
   const int Gn = std::max(1, std::min(4, 1024 / P32));
   const bool prior = n->chain && n->chain->prior;
