@@ -18,7 +18,7 @@ trained for `steps` (default 8) Adam steps of batch 2048 on a device-resident
 set of 8192 random points (the tcgen05 GEMMs k_gemm, the loss, Adam).
 
 substeps: 64 surrogate sub-chains of n_sub (default 4) steps with an additive
-head fitted to a synthetic response (k_propose, the GEMMs, k_head_llh,
+head fitted to a synthetic response (k_propose, the GEMMs, k_head_staged,
 k_penalty, k_accept).
 
 Profile with e.g.
