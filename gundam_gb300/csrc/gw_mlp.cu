@@ -539,10 +539,10 @@ struct AdamArgs {
 };
 
 // Adam on the FP32 master weights and biases of every layer in one launch.
-// Blocks [0, n_tiles): 32 x 32 weight tiles, whose BF16 copy and its
+// The last n_tiles blocks: 32 x 32 weight tiles, whose BF16 copy and its
 // transpose are both stored coalesced (the transpose through shared memory);
-// the blocks after them: 16 biases each, whose gradient is formed here from
-// the layer's transposed output gradients.  A launch per weight and bias array
+// the blocks before them: 16 biases each, whose gradient is formed here from
+// the layer's transposed output gradients (chains of loads, so they start first).  A launch per weight and bias array
 // with a scattered transpose, and a column-sum launch per layer, took 99 us of a
 // 440 us step at 200 -> 512 -> 512 -> 512 -> 3000 and batch 2048; this launch
 // takes 24 us.  The bound is the 32 bytes per weight that w, g, m, v and the BF16
@@ -551,8 +551,9 @@ __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamArgs a
   dep_launch();
   dep_wait();
   const int tid = threadIdx.x;
-  int blk = blockIdx.x, li = 0;
-  if (blk < a.n_tiles) {
+  const int n_bias = (int)gridDim.x - a.n_tiles;
+  int blk = (int)blockIdx.x - n_bias, li = 0;
+  if (blk >= 0) {
     while (li + 1 < a.n_layers && blk >= a.l[li + 1].tile0) ++li;
     const AdamLayer& L = a.l[li];
     const int t = blk - L.tile0, tc = (L.cols + 31) / 32;
@@ -594,7 +595,7 @@ __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamArgs a
     }
     return;
   }
-  blk -= a.n_tiles;
+  blk = blockIdx.x;
   while (li + 1 < a.n_layers && blk >= a.l[li + 1].bias0) ++li;
   const AdamLayer& L = a.l[li];
   const int r = (blk - L.bias0) * 16 + (tid >> 4);
