@@ -277,9 +277,12 @@ __global__ void __launch_bounds__(kPlainThreads) k_plain(const DevView v) {
 // next tile's evaluation instead of behind a block barrier.  Hand-over per
 // buffer b: FULL_b, a named barrier at which the evaluators arrive and the
 // reducers wait, and ebar[b], an mbarrier at which the reducer warps arrive and
-// the evaluators wait.  The evaluator warps never meet: a tile's types differ in
+// the evaluators wait.  The evaluator warps do not meet: a tile's types differ in
 // cost, and a warp that is done goes on with the next tile, up to the buffer the
-// reducers still hold.  The last evaluator warp to be done with a tile issues
+// reducers still hold.  Double-float is the exception: its dial code is several
+// times as long, and warps on different tiles run different types' code, so there
+// the evaluators meet at the end of a tile (1M events, eight warps: 400 us so, 521
+// without; FP64 the other way round, 348 and 333 us for 500k).  The last evaluator warp to be done with a tile issues
 // the copies of the tile after next into its stage.  Every CTA runs the same
 // number of iterations on both sides and every mbarrier wait is bounded; a
 // timed-out wait marks the block failed and the protocol runs on without work:
@@ -290,7 +293,7 @@ __global__ void __launch_bounds__(kPlainThreads) k_plain(const DevView v) {
 // double-float, whose tiles hold fewer dials than one round of 192 threads
 // would cover evenly) and two reducer warps.
 constexpr int kWsRed = 64;
-constexpr int kBarFull = 2, kBarRed = 6;
+constexpr int kBarFull = 2, kBarEval = 4, kBarRed = 6;
 
 template <typename T, int NEV>
 __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_ws(const DevView v) {
@@ -354,6 +357,7 @@ __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_
         }
       }
       named_arrive(kBarFull + st, NT);
+      if constexpr (kIsDf<T>) named_sync(kBarEval, kWsEval);
       __syncwarp();
       if ((tid & 31) == 0) {
         __threadfence_block();  // this warp's reads of the stage come first

@@ -11,8 +11,8 @@
 // sides (FULL_b, a named barrier at which the evaluators arrive and the reducers
 // wait; ebar[b], an mbarrier at which the reducer warps arrive and the evaluators
 // wait), so the next chunk of points (or the next tile) is evaluated while the
-// reducers empty the previous one, and the evaluator warps never wait for one
-// another.  A tile's
+// reducers empty the previous one, and the evaluator warps do not wait for one
+// another (but in double-float, see k_plain_ws).  A tile's
 // payload and headers arrive by one bulk copy and stay in shared memory for
 // all ceil(K / KP) chunks, so HBM sees each dial once per K points; at small
 // K the kernel stays bound by HBM bandwidth, as the K = 1 kernel is, while
@@ -30,7 +30,7 @@ namespace gw {
 namespace {
 
 constexpr int kSEval = 192, kSRed = 64, kSThreads = kSEval + kSRed;
-constexpr int kSBarFull = 2, kSBarRed = 6;
+constexpr int kSBarFull = 2, kSBarEval = 4, kSBarRed = 6;
 
 // The KP values of one slot: stores, loads and the elementwise product.
 template <typename T, int KP>
@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(kSThreads, MB) k_ws(const DevView v, int K) {
           }
         }
         named_arrive(kSBarFull + b, kSThreads);
+        if constexpr (kIsDf<T>) named_sync(kSBarEval, kSEval);  // as in k_plain_ws
       }
       __syncwarp();
       if ((tid & 31) == 0) {
