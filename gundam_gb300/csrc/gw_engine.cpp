@@ -1711,7 +1711,7 @@ static int autotune_plain(gw_engine* e) {
   GW_CUDA(e, cudaDeviceSynchronize());  // every earlier chain, whichever stream
   std::vector<double> pts((size_t)e->cfg.n_params);
   for (size_t i = 0; i < pts.size(); ++i) pts[i] = 0.001 * (double)((i * 7919) % 17) - 0.008;
-  GW_CUDA(e, cudaMemcpy(e->d_params, pts.data(), sizeof(double) * pts.size(), cudaMemcpyHostToDevice));
+  GW_CUDA(e, cudaMemcpyAsync(e->d_params, pts.data(), sizeof(double) * pts.size(), cudaMemcpyHostToDevice, e->stream));
   cudaEvent_t a, b;
   GW_CUDA(e, cudaEventCreate(&a));
   GW_CUDA(e, cudaEventCreate(&b));
@@ -1758,7 +1758,7 @@ extern "C" int gw_autotune(gw_engine* e, int32_t K) {
   // deterministic synthetic points: all parameters at 0 except tiny offsets
   std::vector<double> pts((size_t)K * e->cfg.n_params);
   for (size_t i = 0; i < pts.size(); ++i) pts[i] = 0.001 * (double)((i * 7919) % 17) - 0.008;
-  GW_CUDA(e, cudaMemcpy(e->d_params, pts.data(), sizeof(double) * pts.size(), cudaMemcpyHostToDevice));
+  GW_CUDA(e, cudaMemcpyAsync(e->d_params, pts.data(), sizeof(double) * pts.size(), cudaMemcpyHostToDevice, e->stream));
   cudaEvent_t a, b_ev;
   GW_CUDA(e, cudaEventCreate(&a));
   GW_CUDA(e, cudaEventCreate(&b_ev));

@@ -1347,16 +1347,26 @@ static int gwm_fail(gwm_net* n, int code, const char* msg) {
     if (_e != cudaSuccess) return gwm_fail((n), GW_ERR_CUDA, cudaGetErrorString(_e)); \
   } while (0)
 
+// Clears and uploads go through the network's stream, which does not wait for the
+// legacy default stream: there a memset returns before it is done, and so may a
+// copy from pageable memory.
 template <typename T>
 static int gwm_alloc(gwm_net* n, T** p, size_t count) {
   void* q = nullptr;
-  if (cudaMalloc(&q, sizeof(T) * (count ? count : 1)) != cudaSuccess) {
+  const size_t bytes = sizeof(T) * (count ? count : 1);
+  if (cudaMalloc(&q, bytes) == cudaSuccess) n->allocs.push_back(q);
+  if (!q || cudaMemsetAsync(q, 0, bytes, n->stream) != cudaSuccess) {
     cudaGetLastError();
     return gwm_fail(n, GW_ERR_NOMEM, "cudaMalloc failed");
   }
-  cudaMemset(q, 0, sizeof(T) * (count ? count : 1));
-  n->allocs.push_back(q);
   *p = (T*)q;
+  return GW_OK;
+}
+
+// The host array belongs to the copy until the stream is synchronised.
+template <typename T>
+static int gwm_upload(gwm_net* n, T* dst, const T* src, size_t count) {
+  GWM_CUDA(n, cudaMemcpyAsync(dst, src, sizeof(T) * count, cudaMemcpyHostToDevice, n->stream));
   return GW_OK;
 }
 
@@ -1633,14 +1643,14 @@ extern "C" int gwm_set_layer(gwm_net* n, int32_t l, const float* w, const float*
   GWM_CUDA(n, cudaSetDevice(n->device));
   const int rows = n->dims[l + 1], cols = n->dims[l];
   const size_t nw = (size_t)rows * cols;
-  GWM_CUDA(n, cudaMemcpy(n->w[l], w, sizeof(float) * nw, cudaMemcpyHostToDevice));
-  GWM_CUDA(n, cudaMemcpy(n->b[l], b, sizeof(float) * rows, cudaMemcpyHostToDevice));
+  const int rc = gwm_upload(n, n->w[l], w, nw) | gwm_upload(n, n->b[l], b, rows);
+  if (rc) return rc;
   // BF16 copies through a zero-learning-rate Adam pass (also clears the moments)
-  GWM_CUDA(n, cudaMemset(n->gw_[l], 0, sizeof(float) * nw));
-  GWM_CUDA(n, cudaMemset(n->mw[l], 0, sizeof(float) * nw));
-  GWM_CUDA(n, cudaMemset(n->vw[l], 0, sizeof(float) * nw));
-  GWM_CUDA(n, cudaMemset(n->mb[l], 0, sizeof(float) * rows));
-  GWM_CUDA(n, cudaMemset(n->vb[l], 0, sizeof(float) * rows));
+  GWM_CUDA(n, cudaMemsetAsync(n->gw_[l], 0, sizeof(float) * nw, n->stream));
+  GWM_CUDA(n, cudaMemsetAsync(n->mw[l], 0, sizeof(float) * nw, n->stream));
+  GWM_CUDA(n, cudaMemsetAsync(n->vw[l], 0, sizeof(float) * nw, n->stream));
+  GWM_CUDA(n, cudaMemsetAsync(n->mb[l], 0, sizeof(float) * rows, n->stream));
+  GWM_CUDA(n, cudaMemsetAsync(n->vb[l], 0, sizeof(float) * rows, n->stream));
   gwm::AdamArgs aa{};
   adam_layer(n, l, &aa, 1);
   aa.lr = 0.f;
@@ -1903,25 +1913,24 @@ static int head_alloc(gwm_net* n, size_t tab_elems) {
   return GW_OK;
 }
 
-// Uploads the parts shared by both head forms.
+// Uploads the parts shared by both head forms; ends with the stream's work done.
 static int head_common(gwm_net* n, const float* in_mean, const float* in_scale, const float* base_b,
                        const float* out_mu, const float* out_sd, const float* ratio_w, const double* data) {
   const int din = n->dims[0], nb = n->dims[n->n_layers];
-  GWM_CUDA(n, cudaMemcpy(n->h_mean, in_mean, sizeof(float) * din, cudaMemcpyHostToDevice));
-  GWM_CUDA(n, cudaMemcpy(n->h_scale, in_scale, sizeof(float) * din, cudaMemcpyHostToDevice));
-  GWM_CUDA(n, cudaMemcpy(n->h_b0, base_b, sizeof(float) * nb, cudaMemcpyHostToDevice));
-  GWM_CUDA(n, cudaMemcpy(n->h_mu, out_mu, sizeof(float) * nb, cudaMemcpyHostToDevice));
-  GWM_CUDA(n, cudaMemcpy(n->h_sd, out_sd, sizeof(float) * nb, cudaMemcpyHostToDevice));
-  GWM_CUDA(n, cudaMemcpy(n->h_data, data, sizeof(double) * nb, cudaMemcpyHostToDevice));
+  std::vector<float> rt;
   n->h_has_rw = ratio_w != nullptr;
   if (ratio_w) {
     // [nb x din] -> [din x nb]
-    std::vector<float> rt((size_t)din * nb);
+    rt.resize((size_t)din * nb);
     for (int b = 0; b < nb; ++b)
       for (int k = 0; k < din; ++k) rt[(size_t)k * nb + b] = ratio_w[(size_t)b * din + k];
-    GWM_CUDA(n, cudaMemcpy(n->h_rw, rt.data(), sizeof(float) * rt.size(), cudaMemcpyHostToDevice));
   }
-  return GW_OK;
+  const int rc = gwm_upload(n, n->h_mean, in_mean, din) | gwm_upload(n, n->h_scale, in_scale, din) |
+                 gwm_upload(n, n->h_b0, base_b, nb) | gwm_upload(n, n->h_mu, out_mu, nb) |
+                 gwm_upload(n, n->h_sd, out_sd, nb) | gwm_upload(n, n->h_data, data, nb) |
+                 (rt.empty() ? GW_OK : gwm_upload(n, n->h_rw, rt.data(), rt.size()));
+  GWM_CUDA(n, cudaStreamSynchronize(n->stream));
+  return rc;
 }
 
 extern "C" int gwm_set_head(gwm_net* n, const float* in_mean, const float* in_scale, const float* base_w,
@@ -1937,11 +1946,10 @@ extern "C" int gwm_set_head(gwm_net* n, const float* in_mean, const float* in_sc
   for (int b = 0; b < nb; ++b)
     for (int k = 0; k < din; ++k) wt[(size_t)k * nb + b] = base_w[(size_t)b * din + k];
   for (int b = 0; b < nb; ++b) lr[b] = ratio[b] > 0.f ? logf(ratio[b]) : -1e30f;
-  GWM_CUDA(n, cudaMemcpy(n->h_tab, wt.data(), sizeof(float) * wt.size(), cudaMemcpyHostToDevice));
-  GWM_CUDA(n, cudaMemcpy(n->h_rb, lr.data(), sizeof(float) * nb, cudaMemcpyHostToDevice));
+  rc = gwm_upload(n, n->h_tab, wt.data(), wt.size()) | gwm_upload(n, n->h_rb, lr.data(), nb);
   n->h_nodes = 0;
   n->h_lim = 0.f;
-  return head_common(n, in_mean, in_scale, base_b, out_mu, out_sd, nullptr, data);
+  return rc | head_common(n, in_mean, in_scale, base_b, out_mu, out_sd, nullptr, data);
 }
 
 extern "C" int gwm_set_head_additive(gwm_net* n, const float* in_mean, const float* in_scale, int32_t nodes,
@@ -1956,11 +1964,10 @@ extern "C" int gwm_set_head_additive(gwm_net* n, const float* in_mean, const flo
   const size_t te = (size_t)din * nodes * nb;
   int rc = head_alloc(n, te);
   if (rc) return rc;
-  GWM_CUDA(n, cudaMemcpy(n->h_tab, base_tab, sizeof(float) * te, cudaMemcpyHostToDevice));
-  GWM_CUDA(n, cudaMemcpy(n->h_rb, ratio_b, sizeof(float) * nb, cudaMemcpyHostToDevice));
+  rc = gwm_upload(n, n->h_tab, base_tab, te) | gwm_upload(n, n->h_rb, ratio_b, nb);
   n->h_nodes = nodes;
   n->h_lim = lim;
-  return head_common(n, in_mean, in_scale, base_b, out_mu, out_sd, ratio_w, data);
+  return rc | head_common(n, in_mean, in_scale, base_b, out_mu, out_sd, ratio_w, data);
 }
 
 // Tensor maps of the base table and of r_w in boxes of box_cols bins x
@@ -2477,20 +2484,21 @@ extern "C" int gwm_set_chain(gwm_net* n, const double* prop_chol, const double* 
     }
     n->chain = s;
   }
-  std::vector<float> f32((size_t)P * P);
+  std::vector<float> lt((size_t)P * P), icov;
   for (int p = 0; p < P; ++p)
-    for (int k = 0; k < P; ++k) f32[(size_t)k * P + p] = (float)prop_chol[(size_t)p * P + k];
-  GWM_CUDA(n, cudaMemcpy(s->Lt, f32.data(), sizeof(float) * f32.size(), cudaMemcpyHostToDevice));
+    for (int k = 0; k < P; ++k) lt[(size_t)k * P + p] = (float)prop_chol[(size_t)p * P + k];
+  int rc = gwm_upload(n, s->Lt, lt.data(), lt.size());
   s->prior = prior_mean != nullptr;
   if (s->prior) {
     // symmetric: C^-1 [k][p] read as column p; symmetrised in FP64 first
+    icov.resize((size_t)P * P);
     for (int p = 0; p < P; ++p)
       for (int k = 0; k < P; ++k)
-        f32[(size_t)k * P + p] = (float)(0.5 * (prior_icov[(size_t)k * P + p] + prior_icov[(size_t)p * P + k]));
-    GWM_CUDA(n, cudaMemcpy(s->m, prior_mean, sizeof(double) * P, cudaMemcpyHostToDevice));
-    GWM_CUDA(n, cudaMemcpy(s->icov, f32.data(), sizeof(float) * f32.size(), cudaMemcpyHostToDevice));
+        icov[(size_t)k * P + p] = (float)(0.5 * (prior_icov[(size_t)k * P + p] + prior_icov[(size_t)p * P + k]));
+    rc |= gwm_upload(n, s->m, prior_mean, P) | gwm_upload(n, s->icov, icov.data(), icov.size());
   }
-  return GW_OK;
+  GWM_CUDA(n, cudaStreamSynchronize(n->stream));
+  return rc;
 }
 
 // Runs n_sub surrogate Metropolis steps for C chains from theta0 [C x P]
