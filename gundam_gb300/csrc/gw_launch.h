@@ -8,6 +8,11 @@
 // writes are visible.  Every kernel of such a chain waits, so all earlier
 // kernels have completed too.  After a copy or an event in the stream the
 // launch is an ordinary one.
+//
+// What such a kernel reads changes while it is resident, so of its parameters
+// only arrays that no kernel of the chain writes are __restrict__: of the others
+// the compiler could move loads above the wait, or read them by the path that
+// takes data to be unchanged for the whole kernel.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -174,7 +174,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 
 // A thread's 32 consecutive values of one row of an FP32 matrix (p: the first,
 // 16-byte aligned when `vec`); only the first n are read or written.
-__device__ __forceinline__ void row_load(const float* __restrict__ p, int n, bool vec, float (&v)[32]) {
+__device__ __forceinline__ void row_load(const float* p, int n, bool vec, float (&v)[32]) {
   if (vec && n == 32) {
 #pragma unroll
     for (int q = 0; q < 32; q += 4) {
@@ -461,8 +461,7 @@ __global__ void __launch_bounds__(NW * 32) k_gemm_group(const __grid_constant__ 
 // Rows of a row-major FP32 matrix to BF16, row-major and transposed.  Row r
 // of the output is row perm[r] of x (perm null: row r).  32 x 32 tiles go
 // through shared memory so both stores are coalesced; block (32, 8).
-__global__ void k_rows_to_bf16(const float* __restrict__ x, const int32_t* __restrict__ perm, int rows, int cols,
-                               bf16* y, bf16* yt, int ld_t) {
+__global__ void k_rows_to_bf16(const float* x, const int32_t* perm, int rows, int cols, bf16* y, bf16* yt, int ld_t) {
   dep_launch();
   dep_wait();
   __shared__ bf16 tile[32][34];
@@ -488,7 +487,7 @@ __global__ void k_rows_to_bf16(const float* __restrict__ x, const int32_t* __res
 // Bias gradient of one output unit by 16 lanes: the FP32 sum of its BF16 row
 // dzt [B].  Lane q adds the elements q, q + 16, ... in order, then the 16 parts
 // are added in lane order; the sum on every lane of the half-warp.
-__device__ __forceinline__ float bias_grad(const bf16* __restrict__ dzt, int B) {
+__device__ __forceinline__ float bias_grad(const bf16* dzt, int B) {
   const int q = threadIdx.x & 15;
   float s = 0.f;
   int i = q;
@@ -508,7 +507,7 @@ __device__ __forceinline__ float bias_grad(const bf16* __restrict__ dzt, int B) 
 }
 
 // Bias gradients of one layer, a half-warp per unit (gwm_gradients).
-__global__ void __launch_bounds__(256) k_bias_grad(const bf16* __restrict__ dzt, int rows, int B, float* out) {
+__global__ void __launch_bounds__(256) k_bias_grad(const bf16* dzt, int rows, int B, float* out) {
   dep_launch();
   dep_wait();
   const int r = blockIdx.x * 16 + (threadIdx.x >> 4);
@@ -743,7 +742,7 @@ struct HeadOut {
 // Likelihood term of one (point m, bin) from the base `acc` and the log ratio
 // `racc`, with its optional outputs.
 template <bool GRAD>
-__device__ __forceinline__ double head_term(const Head& h, const float* __restrict__ mlp, int C, int m, int bin,
+__device__ __forceinline__ double head_term(const Head& h, const float* mlp, int C, int m, int bin,
                                             const double* __restrict__ data, int llh_type, float acc, float racc,
                                             const HeadOut& out) {
   if (bin >= h.nb || m >= C) return 0.0;
@@ -765,7 +764,7 @@ __device__ __forceinline__ double head_term(const Head& h, const float* __restri
 }
 
 // The warp's sum of t by a fixed shuffle tree, into part[m][blockIdx.x] (FP64).
-__device__ __forceinline__ void head_part(double t, int C, int m, double* __restrict__ part) {
+__device__ __forceinline__ void head_part(double t, int C, int m, double* part) {
   for (int off = 16; off; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
   if ((threadIdx.x & 31) == 0 && m < C) part[(size_t)m * gridDim.x + blockIdx.x] = t;
 }
@@ -817,9 +816,9 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 template <bool GRAD>
 __global__ void __launch_bounds__(kHeadThreads, 3) k_head_staged(const __grid_constant__ CUtensorMap tm_tab,
                                                         const __grid_constant__ CUtensorMap tm_rw, Head h,
-                                                        const float* __restrict__ x, const float* __restrict__ mlp,
-                                                        int C, const double* __restrict__ data, int llh_type,
-                                                        HeadOut out, uint32_t* status) {
+                                                        const float* x, const float* mlp, int C,
+                                                        const double* __restrict__ data, int llh_type, HeadOut out,
+                                                        uint32_t* status) {
   dep_launch();
   extern __shared__ __align__(128) float sh_h[];  // [kHeadStages][kHeadStage]
   __shared__ float4 s_pt[2][kHeadK][kHeadPts];  // (weight, input, staged row of the interval * kHeadBins, 0)
@@ -926,8 +925,8 @@ __global__ void __launch_bounds__(kHeadThreads, 3) k_head_staged(const __grid_co
 // parameter, with the table lines of a bin shared through L1 across the
 // block's points.
 template <int PPT, bool GRAD>
-__global__ void __launch_bounds__(256) k_head_llh(Head h, const float* __restrict__ x, const float* __restrict__ mlp,
-                                                  int C, const double* __restrict__ data, int llh_type, HeadOut out) {
+__global__ void __launch_bounds__(256) k_head_llh(Head h, const float* x, const float* mlp, int C,
+                                                  const double* __restrict__ data, int llh_type, HeadOut out) {
   dep_launch();
   dep_wait();
   extern __shared__ unsigned char sh_raw[];
@@ -994,7 +993,7 @@ __global__ void __launch_bounds__(256) k_head_llh(Head h, const float* __restric
 }
 
 // llh[m] = sum over blocks of part[m][*], one warp per point, fixed order.
-__global__ void k_llh_finish(const double* __restrict__ part, int nblk, int C, double* __restrict__ llh) {
+__global__ void k_llh_finish(const double* part, int nblk, int C, double* llh) {
   dep_launch();
   dep_wait();
   const int m = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
@@ -1015,8 +1014,7 @@ __global__ void k_llh_finish(const double* __restrict__ part, int nblk, int C, d
 // (point, parameter) go to gz[m][k][0..7], which k_grad_finish adds in order.
 // The general form, for an affine base or one of more nodes than
 // k_base_grad_staged holds.
-__global__ void __launch_bounds__(256) k_base_grad(Head h, const float* __restrict__ x, const float* __restrict__ G,
-                                                   const float* __restrict__ S, float* __restrict__ gz) {
+__global__ void __launch_bounds__(256) k_base_grad(Head h, const float* x, const float* G, const float* S, float* gz) {
   dep_launch();
   dep_wait();
   extern __shared__ float shg[];
@@ -1072,10 +1070,8 @@ constexpr int kGradK = 8, kGradM = 8, kGradStages = 8;
 constexpr int kGradRows = kGradK * kHeadNodes;
 __global__ void __launch_bounds__(256, 2) k_base_grad_staged(const __grid_constant__ CUtensorMap tm_tab,
                                                              const __grid_constant__ CUtensorMap tm_rw, Head h,
-                                                             const float* __restrict__ x,
-                                                             const float* __restrict__ G,
-                                                             const float* __restrict__ S, int C,
-                                                             float* __restrict__ gz, uint32_t* status) {
+                                                             const float* x, const float* G, const float* S, int C,
+                                                             float* gz, uint32_t* status) {
   dep_launch();
   extern __shared__ __align__(128) float sh_g[];  // [kGradStages][kGradRows + kGradK][32]
   constexpr int kStage = (kGradRows + kGradK) * 32;
@@ -1213,10 +1209,9 @@ __device__ __forceinline__ double warp_sum(const float* red, int n) {
 // Per point (block), G groups of P32 threads as k_finish_accept: the value
 // f = llh + penalty and the gradient with respect to the parameters,
 // (gz + dx) / scale + 2 C^-1 (theta - mean) (prior optional).
-__global__ void k_grad_finish(const double* __restrict__ part, int nblk, const double* __restrict__ theta, int P,
-                              const float* __restrict__ scale, const float* __restrict__ gz,
-                              const float* __restrict__ dx, const double* __restrict__ m,
-                              const float* __restrict__ icov, double* __restrict__ f, double* __restrict__ grad) {
+__global__ void k_grad_finish(const double* part, int nblk, const double* theta, int P,
+                              const float* __restrict__ scale, const float* gz, const float* dx,
+                              const double* __restrict__ m, const float* __restrict__ icov, double* f, double* grad) {
   dep_launch();
   dep_wait();
   extern __shared__ float shf2[];
@@ -2305,9 +2300,9 @@ __device__ __forceinline__ double u01(uint64_t h) { return ((double)(h >> 11) + 
 // symmetric), written in FP64, and its standardised inputs
 // x = (prop - mean) / scale (FP32, as k_standardize) with the BF16 row of the
 // first GEMM (as k_rows_to_bf16).
-__global__ void k_propose_stage(const double* __restrict__ phi, int P, const float* __restrict__ Lt, uint64_t seed,
-                                uint64_t step, double* __restrict__ prop, const float* __restrict__ mean,
-                                const float* __restrict__ scale, float* __restrict__ x, bf16* __restrict__ h0) {
+__global__ void k_propose_stage(const double* phi, int P, const float* __restrict__ Lt, uint64_t seed,
+                                uint64_t step, double* prop, const float* __restrict__ mean,
+                                const float* __restrict__ scale, float* x, bf16* h0) {
   dep_launch();
   dep_wait();
   // blockDim.x = G * P32: group g of the column's partial sums covers the
@@ -2354,10 +2349,9 @@ __global__ void k_propose_stage(const double* __restrict__ phi, int P, const flo
 // f = llh + penalty: accept when log u < -(f - f_current) / 2 with u from the
 // hash of (seed, step, chain); NaN proposals are rejected.  first != 0 takes
 // the value unconditionally (the initial evaluation).
-__global__ void k_finish_accept(const double* __restrict__ part, int nblk, const double* __restrict__ prop, int P,
+__global__ void k_finish_accept(const double* part, int nblk, const double* prop, int P,
                                 const double* __restrict__ m, const float* __restrict__ icov, uint64_t seed,
-                                uint64_t step, int first, double* __restrict__ phi, double* __restrict__ f,
-                                int32_t* __restrict__ n_acc) {
+                                uint64_t step, int first, double* phi, double* f, int32_t* n_acc) {
   dep_launch();
   dep_wait();
   // blockDim.x = G * P32 as k_propose_stage
