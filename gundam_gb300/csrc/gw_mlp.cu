@@ -1296,6 +1296,8 @@ struct gwm_net {
   cudaStream_t side = nullptr;
   cudaEvent_t side_go = nullptr, side_done = nullptr;
   std::vector<void*> allocs;
+  const void* opened[24] = {};  // kernels whose shared-memory limit this network has raised (open_shared)
+  int n_opened = 0;
   // per layer l (0..L-1): weights [dims[l+1] x dims[l]]
   std::vector<float*> w, b, gw_, gb, mw, vw, mb, vb;
   std::vector<bf16*> wb, wt;
@@ -1365,6 +1367,23 @@ static int gwm_upload(gwm_net* n, T* dst, const T* src, size_t count) {
   return GW_OK;
 }
 
+// Raises the kernel's limit of dynamic shared memory (48 KB by default) to
+// `bytes`, the same for every call with this kernel, on the network's device.  The
+// limit belongs to a device, so each network sees to its own.
+template <typename... P>
+static int open_shared(gwm_net* n, void (*kernel)(P...), size_t bytes) {
+  const void* fn = (const void*)kernel;
+  for (int i = 0; i < n->n_opened; ++i)
+    if (n->opened[i] == fn) return GW_OK;
+  const cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (r != cudaSuccess) {
+    cudaGetLastError();
+    return gwm_fail(n, GW_ERR_CUDA, cudaGetErrorString(r));
+  }
+  if (n->n_opened < (int)(sizeof(n->opened) / sizeof(n->opened[0]))) n->opened[n->n_opened++] = fn;
+  return GW_OK;
+}
+
 static size_t gemm_smem(int bn, int stages) {
   return (size_t)stages * (gwm::kBM * gwm::kBK * 2 + bn * gwm::kBK * 2) + 1024;
 }
@@ -1429,10 +1448,7 @@ static int launch_gemm(gwm_net* n, const bf16* A, const bf16* B, int M, int N, i
   if (!rc) rc = make_map(n, &mb, B, N, K, BN);
   if (rc) return rc;
   const size_t smem = gemm_smem(BN, S);
-  static std::once_flag once;
-  std::call_once(once, [smem]() {
-    cudaFuncSetAttribute(gwm::k_gemm<BN, S, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  });
+  if ((rc = open_shared(n, gwm::k_gemm<BN, S, NW>, smem))) return rc;
   dim3 grid((N + BN - 1) / BN, (M + gwm::kBM - 1) / gwm::kBM);
   launch_dependent(gwm::k_gemm<BN, S, NW>, grid, NW * 32, smem, n->stream,
                    ma, mb, M, N, K, ep, n->status);
@@ -1462,10 +1478,8 @@ static int launch_group(gwm_net* n, const Product* p, int cnt, int K) {
     g.tile0[i + 1] = g.tile0[i] + ((p[i].N + BN - 1) / BN) * ((p[i].M + gwm::kBM - 1) / gwm::kBM);
   }
   const size_t smem = gemm_smem(BN, S);
-  static std::once_flag once;
-  std::call_once(once, [smem]() {
-    cudaFuncSetAttribute(gwm::k_gemm_group<BN, S, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  });
+  const int rc = open_shared(n, gwm::k_gemm_group<BN, S, NW>, smem);
+  if (rc) return rc;
   launch_dependent(gwm::k_gemm_group<BN, S, NW>, g.tile0[cnt], NW * 32, smem, n->stream, g, n->status);
   GWM_CUDA(n, cudaGetLastError());
   return GW_OK;
@@ -1990,22 +2004,17 @@ static int launch_head(gwm_net* n, int C, int llh_type, const gwm::HeadOut& out)
   if (shm > 200 * 1024) return gwm_fail(n, GW_ERR_LIMIT, "surrogate head: too many inputs");
   if (head_staged(n)) {
     CUtensorMap tab, rw;
-    const int rc = head_maps(n, &tab, &rw, gwm::kHeadBins, gwm::kHeadK);
+    int rc = head_maps(n, &tab, &rw, gwm::kHeadBins, gwm::kHeadK);
     if (rc) return rc;
     constexpr int kShm = gwm::kHeadStages * gwm::kHeadStage * 4;
-    static std::once_flag once;
-    std::call_once(once, []() {
-      cudaFuncSetAttribute(gwm::k_head_staged<GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kShm);
-    });
+    if ((rc = open_shared(n, gwm::k_head_staged<GRAD>, kShm))) return rc;
     const dim3 grid(head_parts(n), (C + gwm::kHeadPts - 1) / gwm::kHeadPts);
     launch_dependent(gwm::k_head_staged<GRAD>, grid, gwm::kHeadThreads, kShm, n->stream,
                      tab, rw, head_view(n), n->xin, n->z[L - 1], C, n->h_data, llh_type, out, n->status);
   } else {
     if (shm > 48 * 1024) {
-      static std::once_flag once;
-      std::call_once(once, []() {
-        cudaFuncSetAttribute(gwm::k_head_llh<kPPT, GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      });
+      const int rc = open_shared(n, gwm::k_head_llh<kPPT, GRAD>, 200 * 1024);
+      if (rc) return rc;
     }
     const dim3 grid(head_parts(n), (C + 8 * kPPT - 1) / (8 * kPPT));
     launch_dependent(gwm::k_head_llh<kPPT, GRAD>, grid, dim3(32, 8), shm, n->stream,
@@ -2022,23 +2031,18 @@ static int launch_base_grad(gwm_net* n, int C, cudaStream_t stream) {
   if (shb > 200 * 1024) return gwm_fail(n, GW_ERR_LIMIT, "gwm_value_grad: too many bins");
   if (head_staged(n)) {
     CUtensorMap tab, rw;
-    const int rc = head_maps(n, &tab, &rw, 32, gwm::kGradK);
+    int rc = head_maps(n, &tab, &rw, 32, gwm::kGradK);
     if (rc) return rc;
     constexpr int kShm = gwm::kGradStages * (gwm::kGradRows + gwm::kGradK) * 32 * 4;
-    static std::once_flag once;
-    std::call_once(once, []() {
-      cudaFuncSetAttribute(gwm::k_base_grad_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, kShm);
-    });
+    if ((rc = open_shared(n, gwm::k_base_grad_staged, kShm))) return rc;
     constexpr int kTile = 8 * gwm::kGradM;
     const dim3 grid(8, (din + gwm::kGradK - 1) / gwm::kGradK, (C + kTile - 1) / kTile);
     launch_dependent(gwm::k_base_grad_staged, grid, 256, kShm, stream,
                      tab, rw, head_view(n), n->xin, n->g_G, n->g_S, C, n->g_gz, n->status);
   } else {
     if (shb > 48 * 1024) {
-      static std::once_flag once;
-      std::call_once(once, []() {
-        cudaFuncSetAttribute(gwm::k_base_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      });
+      const int rc = open_shared(n, gwm::k_base_grad, 200 * 1024);
+      if (rc) return rc;
     }
     launch_dependent(gwm::k_base_grad, dim3(C, (din + 7) / 8), 256, shb, stream,
                      head_view(n), n->xin, n->g_G, n->g_S, n->g_gz);

@@ -31,7 +31,8 @@ struct Event {
   Stream* stream;
 };
 constexpr int kDevices = 2;
-constexpr int kOptin = 227 * 1024, kStatic = 4096;
+int optin = 227 * 1024;  // largest shared memory of a block
+constexpr int kStatic = 4096;  // what every kernel has of it without asking
 std::recursive_mutex mu;
 thread_local int device = 0;
 thread_local cudaError_t last = cudaSuccess;
@@ -84,6 +85,8 @@ int encode_tiled(void*, ...) { return 0; }
 }  // namespace
 
 extern "C" {
+void fake_set_optin(int bytes) { optin = bytes; }
+
 // the log since the last call, cut to n - 1 bytes
 void fake_take(char* b, size_t n) {
   std::lock_guard<std::recursive_mutex> g(mu);
@@ -129,7 +132,7 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* fn, voi
 cudaError_t cudaFuncSetAttribute(const void* fn, cudaFuncAttribute a, int v) {
   std::lock_guard<std::recursive_mutex> g(mu);
   if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) {
-    if (v < 0 || v + kStatic > kOptin) return ret(cudaErrorInvalidValue);
+    if (v < 0 || v + kStatic > optin) return ret(cudaErrorInvalidValue);
     limits[{device, fn}] = v;
   }
   return cudaSuccess;
@@ -140,7 +143,7 @@ cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void*) {
   return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int, size_t smem) {
-  *n = smem + kStatic > (size_t)kOptin ? 0 : 1;
+  *n = smem + kStatic > (size_t)optin ? 0 : 1;
   return cudaSuccess;
 }
 
@@ -158,7 +161,7 @@ cudaError_t cudaGetDevice(int* d) {
   return cudaSuccess;
 }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
-  *v = a == cudaDevAttrMultiProcessorCount ? 152 : a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? kOptin : 1;
+  *v = a == cudaDevAttrMultiProcessorCount ? 152 : a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? optin : 1;
   return cudaSuccess;
 }
 cudaError_t cudaGetLastError() {
