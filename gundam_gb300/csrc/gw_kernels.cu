@@ -671,15 +671,34 @@ static const void* pick_plain(const DevView& v) {
   return v.precision ? plain_fn<float>(v.plain_kind) : plain_fn<double>(v.plain_kind);
 }
 
-int plain_blocks_per_sm(const DevView& v) {
-  const void* fn = pick_plain(v);
-  const size_t smem = plain_smem_bytes(v);
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return 0;
+// Raises the kernel's limit of dynamic shared memory on the current device to all
+// that a block may have there.  The limit is the kernel's, not an engine's: set to
+// the need of the engine built last, it would refuse the launches of an earlier
+// one with larger tiles or more parameters.
+static cudaError_t open_shared(const void* fn) {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes a;
+  cudaError_t r = cudaGetDevice(&dev);
+  if (r == cudaSuccess) r = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (r == cudaSuccess) r = cudaFuncGetAttributes(&a, fn);
+  if (r == cudaSuccess)
+    r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes);
+  return r;
+}
+
+// Resident blocks per SM, 0 when the kernel cannot run with that much shared memory.
+static int blocks_per_sm(const void* fn, int threads, size_t smem) {
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, plain_threads(v.plain_kind), smem) != cudaSuccess)
+  if (open_shared(fn) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, smem) != cudaSuccess) {
+    cudaGetLastError();
     return 0;
+  }
   return n;
+}
+
+int plain_blocks_per_sm(const DevView& v) {
+  return blocks_per_sm(pick_plain(v), plain_threads(v.plain_kind), plain_smem_bytes(v));
 }
 
 int batched_blocks_per_sm(const DevView& v, const BatchedShape& b) {
@@ -687,26 +706,15 @@ int batched_blocks_per_sm(const DevView& v, const BatchedShape& b) {
   if (!e) return 0;
   const void* fn = e->fn[v.precision];
   if (!fn) return 0;  // not compiled for this precision
-  const size_t smem = batched_smem_bytes(v, b);
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, b.threads, smem) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return n;
+  return blocks_per_sm(fn, b.threads, batched_smem_bytes(v, b));
 }
 
 size_t params_smem_bytes(const DevView& v) { return (size_t)v.n_params * sizeof(double) * (v.n_eigen > 0 ? 2 : 1); }
 
 cudaError_t prepare_params(const DevView& v) {
-  const size_t smem = params_smem_bytes(v);
-  const void* fn = v.precision == 2 ? (const void*)k_params<dfloat>
-                    : v.precision ? (const void*)k_params<float> : (const void*)k_params<double>;
-  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return open_shared(v.precision == 2 ? (const void*)k_params<dfloat>
+                     : v.precision   ? (const void*)k_params<float>
+                                     : (const void*)k_params<double>);
 }
 
 cudaError_t launch_params(const DevView& v, const double* params, int K, cudaStream_t s) {

@@ -40,3 +40,30 @@ def test_a_refused_limit_is_reported(tmp_path):
             raise AssertionError("no error")
         assert not [x for x in log() if x.startswith("refused")]  # nothing was launched with it
     """, tmp_path)
+
+
+def test_engines_of_different_sizes_side_by_side(tmp_path):
+    fake_device.run("""
+        wl = Workload("mixed", seed=3)
+        def small_last(build, use):
+            for order in ((0, 1), (1, 0)):
+                engines = [build(i) for i in order]
+                log()
+                for e in engines:
+                    use(e)
+                assert not [x for x in log() if x.startswith("refused")], order
+                for e in engines:
+                    e.close()
+        for precision in ("fp32", "fp64", "df64"):
+            # tiles of two sizes, through the one-point and the batched kernels
+            for k in (1, 4, 64):
+                small_last(lambda i: Engine.from_workload(wl, precision=precision, k_max=k, tile_bytes=(0, 8192)[i]),
+                           lambda e: e.eval(wl.draw_points(k, 1)))
+            # numbers of parameters
+            def engine(i):
+                e = Engine(4, (8192, 16)[i], 4, precision=precision)
+                e.set_event_indices(np.arange(4, dtype=np.int32))
+                e.initialize()
+                return e
+            small_last(engine, lambda e: e.eval(np.zeros((1, e.n_params))))
+    """, tmp_path)
