@@ -1646,6 +1646,10 @@ extern "C" int gw_eval(gw_engine* e, const double* params, int32_t K, double* su
   } else {
     copy_out(0, bytes);
   }
+  if (e->llh_type == GW_LLH_NONE) {  // the kernels write neither: the block there holds an earlier call's bytes
+    if (llh) std::fill_n(llh, K, 0.0);
+    if (llh_stat) std::fill_n(llh_stat, K, 0.0);
+  }
   e->weights_valid = e->copy_weights && K == 1;
   return GW_OK;
 }

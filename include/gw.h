@@ -253,6 +253,7 @@ int gw_initialize(gw_engine* e);
  *   sums2    [K * n_bins]    sum of squared weights per bin (may be NULL)
  *   llh      [K]             stat + penalty                 (may be NULL)
  *   llh_stat [K]             stat part only                 (may be NULL)
+ * llh and llh_stat are zero without a likelihood (GW_LLH_NONE).
  * Blocks until the results are on the host. */
 int gw_eval(gw_engine* e, const double* params, int32_t K, double* sums, double* sums2,
             double* llh, double* llh_stat);
