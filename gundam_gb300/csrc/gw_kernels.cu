@@ -474,9 +474,11 @@ __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_
 // Bin sums and likelihood.
 // ---------------------------------------------------------------------------
 // One block covers BT bins of KT points, 256 threads:
-//   1. thread (point kk, slot lane sl, bin bb), points fastest so that the
-//      reads of a slot's row are contiguous, adds slots i0 + sl, + SL, ... of
-//      its bin in order; the SL lanes' sums are added in lane order;
+//   1. a bin's slots belong to eight runs, slot i0 + r to run r % 8: thread (point
+//      kk, slot lane sl, bin bb), points fastest so that the reads of a slot's row
+//      are contiguous, adds the slots of its runs sl, sl + SL, ... in order; the
+//      runs are added in order, so that a point's sums do not depend on how many
+//      points share the call;
 //   2. thread (bin, point), bins fastest, writes the sums and evaluates the
 //      likelihood term; the BT terms of a point are added by a shuffle tree;
 //   3. the last block of a point tile adds its blocks' parts and the penalty's
@@ -494,7 +496,9 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
                                                   double* llh, double* llh_stat) {
   constexpr int NT = 256, SL = NT / (KT * BT);
   static_assert(SL >= 1 && SL * KT * BT == NT && BT <= 32 && NT % KT == 0, "tile shape");
-  __shared__ double2 part[SL][BT][KT + (KT > 1 ? 1 : 0)];
+  constexpr int kRuns = 8, kParts = SL > 1 ? kRuns : 1;  // one thread per bin and point adds its runs itself
+  static_assert(kRuns % SL == 0, "whole runs per slot lane");
+  __shared__ double2 part[kParts][BT][KT + (KT > 1 ? 1 : 0)];
   __shared__ double red[NT];
   __shared__ bool last;
   const int tid = threadIdx.x;
@@ -503,29 +507,68 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
   {
     const int kk = tid % KT, sl = (tid / KT) % SL, bb = tid / (KT * SL);
     const int b = b0 + bb, k = kb + kk;
-    double s = 0.0, s2 = 0.0;
-    if (b < v.n_bins && k < K) {
-      const int i1 = v.bin_slot[b + 1];
-      int i = v.bin_slot[b] + sl;
-      const double2* src = v.partials + k;
-      // four rows in flight, added in order
-      for (; i + 3 * SL < i1; i += 4 * SL) {
-        double2 p[4];
+    const int i0 = b < v.n_bins ? v.bin_slot[b] : 0;
+    const int n = b < v.n_bins && k < K ? v.bin_slot[b + 1] - i0 : 0;
+    const double2* src = v.partials + (size_t)i0 * v.kpad + k;
+    if constexpr (SL > 1) {
+      constexpr int A = kRuns / SL, U = A < 4 ? 4 / A : 1;  // runs of this thread; four rows in flight
+      double s[A] = {}, s2[A] = {};
+      for (int r = sl; r < n; r += U * kRuns) {
+        double2 p[U][A];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) p[q] = src[(size_t)(i + q * SL) * v.kpad];
+        for (int q = 0; q < U * A; ++q) {
+          const int i = r + q * SL;
+          p[q / A][q % A] = i < n ? src[(size_t)i * v.kpad] : make_double2(0.0, 0.0);
+        }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          s += p[q].x;
-          s2 += p[q].y;
+        for (int q = 0; q < U * A; ++q) {
+          s[q % A] += p[q / A][q % A].x;
+          s2[q % A] += p[q / A][q % A].y;
         }
       }
-      for (; i < i1; i += SL) {
-        const double2 p = src[(size_t)i * v.kpad];
-        s += p.x;
-        s2 += p.y;
+#pragma unroll
+      for (int q = 0; q < A; ++q) part[sl + q * SL][bb][kk] = make_double2(s[q], s2[q]);
+    } else {
+      double s = 0.0, s2 = 0.0;
+      if (n <= kRuns) {  // a slot per run at most: the runs in order are the slots in order
+        int r = 0;
+        for (; r + 3 < n; r += 4) {  // four rows in flight
+          double2 p[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) p[q] = src[(size_t)(r + q) * v.kpad];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            s += p[q].x;
+            s2 += p[q].y;
+          }
+        }
+        for (; r < n; ++r) {
+          const double2 p = src[(size_t)r * v.kpad];
+          s += p.x;
+          s2 += p.y;
+        }
+      } else {
+        for (int h = 0; h < kRuns; h += 4) {  // four runs at a time, a row of each in flight
+          double t[4] = {}, t2[4] = {};
+          for (int r = h; r < n; r += kRuns) {
+            double2 p[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) p[q] = r + q < n ? src[(size_t)(r + q) * v.kpad] : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              t[q] += p[q].x;
+              t2[q] += p[q].y;
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            s += t[q];
+            s2 += t2[q];
+          }
+        }
       }
+      part[0][bb][kk] = make_double2(s, s2);
     }
-    part[sl][bb][kk] = make_double2(s, s2);
   }
   __syncthreads();
   const bool want_llh = v.llh_type != 0 && (llh != nullptr || llh_stat != nullptr);
@@ -537,7 +580,7 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
     if (in) {
       double s = 0.0, s2 = 0.0;
 #pragma unroll
-      for (int q = 0; q < SL; ++q) {
+      for (int q = 0; q < kParts; ++q) {
         const double2 p = part[q][bb][kk];
         s = q ? s + p.x : p.x;
         s2 = q ? s2 + p.y : p.y;
