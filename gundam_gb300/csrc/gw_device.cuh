@@ -418,7 +418,9 @@ __device__ __forceinline__ double llh_bb_oa2021(double data, double log_data, do
     double fractional = root / pred;
     if (__double2hiint(fractional) >= 0x5f138d35) fractional = fmin(fractional, 1.0e150);  // from 9.99e149
     const double temp = pred * fractional * fractional - 1;
-    const double temp2 = temp * temp + 4 * data * fractional * fractional;
+    // fused explicitly, so that every kernel gives a bin the same term; temp's square
+    // rounded, so that temp cancels below where the square is all there is
+    const double temp2 = __fma_rn(4 * data * fractional, fractional, __dmul_rn(temp, temp));
     if (__double2hiint(temp2) < 0 && temp2 < 0) return HUGE_VAL;
     const double beta = (-1 * temp + sqrt(temp2)) / 2.;
     newmc = pred * beta;
@@ -450,6 +452,23 @@ __device__ __forceinline__ double llh_bb_bin(double data, double log_data, doubl
   if ((__double2hiint(mcuncert) & 0x7ff00000) == 0x7ff00000) return HUGE_VAL;
   const double root = positive_normal(mcuncert) ? fabs(sqrt_sum_w2) : sqrt(mcuncert);
   return llh_bb_oa2021(data, log_data, pred, mcuncert, root);
+}
+
+// The order in which the likelihood terms of a point are added, in k_bins_llh for
+// every number of points and in k_llh_noalloc, so that all give the same sum:
+//   * the terms of 256 bins, zeros beyond the last bin, by a tree of neighbours
+//     ((0 + 1) + (2 + 3)) + ...;
+//   * these sums in eight runs, sum i in run i % 8, a run's in order;
+//   * the eight runs by the tree of neighbours.
+constexpr int kLlhGroup = 256, kLlhRuns = 8;
+
+// The tree of neighbours over the lanes' values: aligned groups of TO lanes whose
+// values already stand for groups of FROM.
+template <int FROM, int TO>
+__device__ __forceinline__ double neighbour_tree(double x) {
+#pragma unroll
+  for (int o = FROM; o < TO; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
 }
 
 }  // namespace

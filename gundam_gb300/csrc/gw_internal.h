@@ -124,6 +124,6 @@ int batched_blocks_per_sm(const DevView& v, const BatchedShape& b);
 
 constexpr int kPlainThreads = 256;
 constexpr int kPenRows = 8;  // rows of C^-1 per penalty block of k_params
-constexpr int kLlhBins = 8;  // bins of k_bins_llh's smallest block
+constexpr int kLlhBins = 8;  // bins per part of k_bins_llh's likelihood sum (its smallest block)
 
 }  // namespace gw

@@ -480,9 +480,10 @@ __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_
 //      runs are added in order, so that a point's sums do not depend on how many
 //      points share the call;
 //   2. thread (bin, point), bins fastest, writes the sums and evaluates the
-//      likelihood term; the BT terms of a point are added by a shuffle tree;
-//   3. the last block of a point tile adds its blocks' parts and the penalty's
-//      in a fixed order.
+//      likelihood term; the terms of 8 bins of a point are added;
+//   3. the last block of a point tile adds these parts, in the order of
+//      kLlhGroup, and the penalty's: warp w run w, thread (point kk, sub) of it KT
+//      parts of each sum of 256 bins, all on the way at once.
 // A Barlow-Beeston term is ~80 FP64 operations and an SM issues one warp of
 // them every 16 cycles (pipe busy 84 % at 10000 bins, 100 points: 203 us, 232
 // with CUDA's logarithm, a third square root and FP64 compares; see
@@ -499,7 +500,7 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
   constexpr int kRuns = 8, kParts = SL > 1 ? kRuns : 1;  // one thread per bin and point adds its runs itself
   static_assert(kRuns % SL == 0, "whole runs per slot lane");
   __shared__ double2 part[kParts][BT][KT + (KT > 1 ? 1 : 0)];
-  __shared__ double red[NT];
+  __shared__ double red[kLlhRuns * KT];
   __shared__ bool last;
   const int tid = threadIdx.x;
   const int kb = blockIdx.y * KT, b0 = blockIdx.x * BT;
@@ -596,9 +597,8 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
     }
     if (want_llh) {
       // whole warps are in this branch (KT * BT is a multiple of 32)
-#pragma unroll
-      for (int o = BT / 2; o; o >>= 1) term += __shfl_xor_sync(0xffffffffu, term, o);
-      if (bb == 0 && k < K) v.llh_blocks[(size_t)blockIdx.x * v.kpad + k] = term;
+      term = neighbour_tree<1, kLlhBins>(term);
+      if (in && bb % kLlhBins == 0) v.llh_blocks[(size_t)(b / kLlhBins) * v.kpad + k] = term;
     }
   }
   if (!want_llh) return;
@@ -608,18 +608,30 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
   __syncthreads();
   if (!last) return;
   __threadfence();
-  constexpr int NL = NT / KT;
-  const int kk = tid % KT, l = tid / KT, k = kb + kk;
+  static_assert(NT == 32 * kLlhRuns && kLlhGroup == 32 * kLlhBins && KT <= 32, "a warp per run");
+  const int warp = tid >> 5, kk = tid % KT, sub = (tid & 31) / KT, k = kb + kk;
+  const int parts = (v.n_bins + kLlhBins - 1) / kLlhBins;
   double t = 0.0;
-  if (k < K)
-    for (int i = l; i < (int)gridDim.x; i += NL) t += __ldcg(&v.llh_blocks[(size_t)i * v.kpad + k]);
-  red[tid] = t;
-  for (int h = NL / 2; h; h >>= 1) {
-    __syncthreads();
-    if (l < h) red[tid] += red[tid + h * KT];
+  for (int g = warp; g * 32 < parts; g += kLlhRuns) {
+    double x[KT];
+#pragma unroll
+    for (int j = 0; j < KT; ++j) {
+      const int i = g * 32 + sub * KT + j;
+      x[j] = i < parts && k < K ? __ldcg(&v.llh_blocks[(size_t)i * v.kpad + k]) : 0.0;
+    }
+#pragma unroll
+    for (int h = 1; h < KT; h <<= 1)
+#pragma unroll
+      for (int j = 0; j < KT; j += 2 * h) x[j] += x[j + h];
+    t += neighbour_tree<KT, 32>(x[0]);
   }
-  if (l == 0 && k < K) {
-    t = red[tid];
+  if (sub == 0) red[warp * KT + kk] = t;
+  __syncthreads();
+  if (tid < KT && k < K) {
+    double r[kLlhRuns];
+#pragma unroll
+    for (int w = 0; w < kLlhRuns; ++w) r[w] = red[w * KT + tid];
+    t = ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7]));
     double pen = 0.0;
     for (int q = 0; q < v.n_pen; ++q) pen += v.penalty[(size_t)q * v.kpad + k];
     if (llh_stat) llh_stat[k] = t;

@@ -3,9 +3,9 @@
 //
 // gw_llh_noalloc computes, for K parameter points, the summed per-bin
 // likelihood from bin sums the caller already holds on the device: the same
-// per-bin terms as the engine's k_bins_llh, and a fixed-order block /
-// last-block reduction.  That reduction needs scratch memory (one partial per
-// block and one arrival counter per point).  The engine allocates it with
+// per-bin terms as the engine's k_bins_llh, added in the same order (kLlhGroup),
+// by blocks of 256 bins and the last of them.  That needs scratch memory (one
+// partial per block and one arrival counter per point).  The engine allocates it with
 // cudaMalloc; here it is a fixed-size array in device global memory that the
 // library defines at file scope, so the call itself allocates nothing.
 //
@@ -51,9 +51,9 @@ static __device__ __align__(256) unsigned char gw_noalloc_scratch[kNoAllocBytes]
 namespace gw {
 namespace {
 
-// Per-bin terms of k_bins_llh from caller-provided sums, reduced per point in a
-// fixed order; scratch = the file-scope array.
-__global__ void __launch_bounds__(256) k_llh_noalloc(const double* __restrict__ sums,
+// Per-bin terms of k_bins_llh from caller-provided sums, added per point in its
+// order; scratch = the file-scope array.
+__global__ void __launch_bounds__(kLlhGroup) k_llh_noalloc(const double* __restrict__ sums,
                                                      const double* __restrict__ sums2,
                                                      const double* __restrict__ data, int n_bins, int llh_type,
                                                      double* blocks, unsigned int* counters, double* llh) {
@@ -69,16 +69,14 @@ __global__ void __launch_bounds__(256) k_llh_noalloc(const double* __restrict__ 
       term = llh_bb_bin(data[b], log_data_of(data[b]), s, sqrt(s2));
     }
   }
-  __shared__ double red[32];
+  __shared__ double red[kLlhGroup / 32];
   __shared__ bool last;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int o = 16; o; o >>= 1) term += __shfl_xor_sync(0xffffffffu, term, o);
+  term = neighbour_tree<1, 32>(term);
   if (lane == 0) red[warp] = term;
   __syncthreads();
   if (warp == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    double t = lane < nw ? red[lane] : 0.0;
-    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    const double t = neighbour_tree<1, kLlhGroup / 32>(red[lane % (kLlhGroup / 32)]);
     if (lane == 0) {
       blocks[(size_t)k * gridDim.x + blockIdx.x] = t;
       __threadfence();
@@ -90,9 +88,15 @@ __global__ void __launch_bounds__(256) k_llh_noalloc(const double* __restrict__ 
   if (!last) return;
   if (warp == 0) {
     __threadfence();
+    // lane l holds run l % 8; 32 sums on the way at once
+    const int run = lane % kLlhRuns;
     double t = 0.0;
-    for (int i = lane; i < (int)gridDim.x; i += 32) t += __ldcg(&blocks[(size_t)k * gridDim.x + i]);
-    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    for (int i0 = 0; i0 < (int)gridDim.x; i0 += 32) {
+      const double x = i0 + lane < (int)gridDim.x ? __ldcg(&blocks[(size_t)k * gridDim.x + i0 + lane]) : 0.0;
+#pragma unroll
+      for (int q = 0; q < 32; q += kLlhRuns) t += __shfl_sync(0xffffffffu, x, run + q);
+    }
+    t = neighbour_tree<1, kLlhRuns>(t);
     if (lane == 0) {
       llh[k] = t;
       counters[k] = 0u;

@@ -17,8 +17,8 @@ EVENTS = (1, 40, 256, 300, 900, 2100, 2400, 5000)  # per bin: a slot holds at mo
 def _engine(llh_type, n_bins=len(EVENTS)):
     rng = np.random.default_rng(8)
     bins = np.repeat(np.arange(len(EVENTS)), EVENTS)
-    if n_bins > len(EVENTS):  # and many bins of a few events
-        bins = np.concatenate([bins, rng.integers(len(EVENTS), n_bins, 4 * n_bins)])
+    if n_bins > len(EVENTS):  # and many bins of a few events, none empty (a Poisson term without expectation is inf)
+        bins = np.concatenate([bins, np.arange(len(EVENTS), n_bins), rng.integers(len(EVENTS), n_bins, 4 * n_bins)])
     e = Engine(bins.size, 16, n_bins, k_max=64, precision="fp64")
     e.set_event_indices(bins.astype(np.int32))
     e.set_initial_values(rng.uniform(0.5, 1.5, bins.size))
@@ -53,4 +53,32 @@ def test_sums_of_a_point_at_every_number_of_points():
         for k in POINTS:
             s, s2, _, _ = e.eval(pts[:k])
             assert np.array_equal(s, sums[:k]) and np.array_equal(s2, sums2[:k]), (kind, k)
+    e.close()
+
+
+# bins: one part of 8, one group of 256 and a bin, more groups than runs
+@pytest.mark.parametrize("n_bins", [8, 257, 2500])
+@pytest.mark.parametrize("llh_type", [N.GW_LLH_POISSON, N.GW_LLH_BARLOW_BEESTON_OA2021])
+def test_likelihood_of_a_point_at_every_number_of_points(llh_type, n_bins):
+    torch = pytest.importorskip("torch")
+    e, pts = _engine(llh_type, n_bins)
+    rng = np.random.default_rng(8)
+    data = rng.poisson(rng.uniform(0.0, 9.0, n_bins)).astype(np.float64)
+    e.set_data(data)
+    d_data = torch.from_numpy(data).cuda()
+    for kind in _batched_shapes(e):
+        _, _, llh, stat = e.eval(pts)
+        for k in POINTS + (1, 64):
+            s, s2, f, t = e.eval(pts[:k])
+            assert np.isfinite(t).all()
+            if k > 1:  # one point has kernels, and so tile sums, of its own
+                assert np.array_equal(f, llh[:k]) and np.array_equal(t, stat[:k]), (kind, k)
+            # the same from the sums
+            d_s, d_s2 = torch.from_numpy(s).cuda(), torch.from_numpy(s2).cuda()
+            out = torch.full((k,), float("nan"), dtype=torch.float64, device="cuda")
+            torch.cuda.synchronize()
+            assert N.libgw().gw_llh_noalloc(d_s.data_ptr(), d_s2.data_ptr(), d_data.data_ptr(), n_bins, k, llh_type,
+                                            out.data_ptr(), None) == N.GW_OK
+            torch.cuda.synchronize()
+            assert np.array_equal(out.cpu().numpy(), t), (kind, k)
     e.close()
