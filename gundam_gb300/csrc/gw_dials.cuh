@@ -343,7 +343,9 @@ __device__ __forceinline__ int coef_interval(T& xx, int n, bool trunc, T& u) {
     fj = fminf(fmaxf(f, -1.0f), nm1);
     j = __float_as_int(fj + 8388609.0f) - 0x4B000000;  // j + 1
   } else {
-    const T xc = (xx < T(-1)) ? T(-1) : ((xx > T(n - 1)) ? T(n - 1) : xx);
+    // NaN goes to the first block (its conversion to an integer is no index), and
+    // comes out through u
+    const T xc = (xx > T(-1)) ? ((xx < T(n - 1)) ? xx : T(n - 1)) : T(-1);
     int i = (int)xc;     // truncation, in [-1, n - 1]
     if (T(i) > xc) --i;  // floor
     fj = T(i);

@@ -1,0 +1,83 @@
+"""Parameters that are no ordinary numbers, through every stored form of the splines
+and every family of kernels."""
+import numpy as np
+import pytest
+
+from gundam_gb300 import Engine
+from gundam_gb300 import _native as N
+
+pytestmark = pytest.mark.gpu
+
+rng = np.random.default_rng(4)
+X4, X3 = np.array([-3.0, -1.0, 0.0, 2.5]), np.array([-3.0, 0.5, 2.0])
+Y = rng.uniform(0.5, 1.5, 16)
+DIALS = [  # one event and one bin each; parameter 1 (and 2 for the surfaces)
+    (N.GW_DIAL_NORM, np.zeros(0)),
+    (N.GW_DIAL_MONOTONIC, np.concatenate([[-3.0, 1.0], Y[:7]])),
+    (N.GW_DIAL_COMPACT, np.concatenate([[-3.0, 1.0], Y[:7]])),
+    (N.GW_DIAL_UNIFORM, np.concatenate([[-3.0, 2.0], np.stack([Y[:4], rng.normal(0, 0.2, 4)], 1).ravel()])),
+    (N.GW_DIAL_GENERAL, np.concatenate([[-3.0, 1.0], np.stack([Y[:4], rng.normal(0, 0.2, 4), X4], 1).ravel()])),
+    (N.GW_DIAL_GRAPH, np.stack([Y[:4], X4], 1).ravel()),
+    (N.GW_DIAL_BILINEAR, np.concatenate([[4, 3], X4, X3, Y[:12]])),
+    (N.GW_DIAL_BICUBIC, np.concatenate([[4, 3], X4, X3, Y[:12]])),
+]
+
+
+def engine(precision, k_max, layout="auto", truncate=False, lo=None, hi=None):
+    n = len(DIALS)
+    e = Engine(n, 3, n, k_max=k_max, precision=precision, spline_layout=layout)
+    for p in (1, 2):
+        if truncate:
+            e.set_extrapolation(p, False)
+        if lo is not None:
+            e.set_lower_clamp(p, lo)
+        if hi is not None:
+            e.set_upper_clamp(p, hi)
+    e.set_event_indices(np.arange(n, dtype=np.int32))
+    start = np.cumsum([0] + [d.size for _, d in DIALS]).astype(np.int64)
+    e.add_dials(np.array([t for t, _ in DIALS], np.uint8), np.arange(n, dtype=np.int32), np.full(n, 1, np.int32),
+                np.full(n, 2, np.int32), start, np.concatenate([d for _, d in DIALS]))
+    e.set_data(np.ones(n))
+    e.initialize()
+    return e
+
+
+def families(e, k):
+    """Each family of kernels the engine has for k points (the first shape of each)."""
+    if k == 1:
+        for kind in (0, 1, 2):
+            e.set_plain_kernel(kind)
+            yield kind
+        return
+    done = set()
+    for i, (kind, _, _, _, _, _) in enumerate(Engine.compiled_shapes()):
+        if kind in done:
+            continue
+        try:
+            e.set_shape_index(i)
+        except RuntimeError:
+            continue
+        done.add(kind)
+        yield kind
+    assert len(done) >= 2
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "df64"])
+@pytest.mark.parametrize("layout", ["auto", "knots", "slopes", "coefs", "grid"])
+def test_nan_parameter(precision, layout):
+    """NaN gives NaN in the bins of that point and nothing else."""
+    for k in (1, 4, 24, 64):
+        e = engine(precision, k, layout)
+        pts = np.zeros((k, 3))
+        pts[:, 1:] = np.linspace(-2.0, 1.5, k)[:, None]
+        for _ in families(e, k):
+            ref = e.eval(pts)[0]
+            assert np.isfinite(ref).all()
+            for sign in (1.0, -1.0):
+                bad = pts.copy()
+                bad[k // 2, 1:] = np.copysign(np.nan, sign)
+                got = e.eval(bad)[0]
+                assert np.isnan(got[k // 2]).all(), (k, got[k // 2])
+                rest = np.arange(k) != k // 2
+                assert np.array_equal(got[rest], ref[rest])
+        e.close()
