@@ -1135,7 +1135,8 @@ int build_and_upload(gw_engine* e) {
               if (r.type < kTabulated) {
                 flags = ((e->pflags[(size_t)r.p0] & 1) ? kLhTrunc : 0u) | (common_clamp(r.p0) ? kLhCommonClamp : 0u);
                 if (type == kGrid && (flags & kLhCommonClamp)) flags |= kLhGrid;
-                if (type == kNorm && common_clamp(r.p0) && e->clamp_hi[(size_t)r.p0] >= DBL_MAX) flags |= kLhNorm;
+                // an upper bound of +inf lets more through than the default
+                if (type == kNorm && common_clamp(r.p0) && e->clamp_hi[(size_t)r.p0] == DBL_MAX) flags |= kLhNorm;
               }
               hdr_ev[(size_t)(tp.dial0 + slot)] =
                   make_lane_header(type, pn[(size_t)di], flags, (uint32_t)((size_t)off * tsz), p0, p1);

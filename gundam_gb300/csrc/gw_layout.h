@@ -75,7 +75,7 @@ GW_HD int hdr_p1(uint64_t h) { return (int)((h >> 48) & 0xFFFF); }
 //      [16,32) second parameter of surface dials
 constexpr uint32_t kLhTrunc = 1u << 25;        // no extrapolation
 constexpr uint32_t kLhCommonClamp = 1u << 26;  // the response clamp is [0, 1e20] or [0, more]
-constexpr uint32_t kLhNorm = 1u << 30;         // a norm dial of a parameter clamped to [0, no bound]
+constexpr uint32_t kLhNorm = 1u << 30;         // a norm dial of a parameter clamped to [0, largest number]
 constexpr uint32_t kLhGrid = 1u << 31;         // a grid dial with the common clamp
 GW_HD uint64_t make_lane_header(int type, int n, uint32_t flags, uint32_t off, int p0, int p1) {
   const uint32_t x = (off & 0xFFFFu) | (uint32_t)(type & 0xF) << 16 | (uint32_t)(n & 0x1F) << 20 | flags;

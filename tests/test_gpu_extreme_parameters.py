@@ -81,3 +81,34 @@ def test_nan_parameter(precision, layout):
                 rest = np.arange(k) != k // 2
                 assert np.array_equal(got[rest], ref[rest])
         e.close()
+
+
+def _around(values):
+    v = np.asarray(values, dtype=np.float64)
+    with np.errstate(over="ignore"):
+        return np.unique(np.concatenate([v, np.nextafter(v, np.inf), np.nextafter(v, -np.inf)]))
+
+
+BOUNDS = [(None, None), (0.0, None), (-0.0, 1.0), (0.75, 1.25), (-1.5, -0.25), (-2.0, 0.0), (0.0, 0.0), (0.0, np.inf)]
+
+
+@pytest.mark.parametrize("lo,hi", BOUNDS)
+@pytest.mark.parametrize("k", [1, 64])
+def test_fp64_clamp_at_its_bounds(k, lo, hi):
+    """A norm dial's response is its parameter, so the clamp shows by itself: the same
+    number as the comparisons v < lo and v > hi give."""
+    big = np.finfo(np.float64).max
+    edges = [0.0, 5e-324, 1.0, 1e20, 1e21, big] + [b for b in (lo, hi) if b is not None and np.isfinite(b)]
+    vals = _around(edges + [-v for v in edges])
+    vals = np.concatenate([vals, [-0.0, np.inf, -np.inf]])
+    a, b = -big if lo is None else lo, big if hi is None else hi
+    want = np.where(vals < a, a, np.where(vals > b, b, vals))
+    e = engine("fp64", k, lo=lo, hi=hi)
+    for _ in families(e, k):
+        got = []
+        for i in range(0, vals.size, k):
+            pts = np.zeros((k, 3))
+            pts[:vals[i:i + k].size, 1] = vals[i:i + k]
+            got.append(e.eval(pts)[0][:vals[i:i + k].size, 0])
+        assert np.array_equal(np.concatenate(got), want)
+    e.close()
