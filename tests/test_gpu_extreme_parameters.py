@@ -112,3 +112,40 @@ def test_fp64_clamp_at_its_bounds(k, lo, hi):
             got.append(e.eval(pts)[0][:vals[i:i + k].size, 0])
         assert np.array_equal(np.concatenate(got), want)
     e.close()
+
+
+@pytest.mark.parametrize("layout", ["auto", "knots", "slopes", "coefs", "grid"])
+@pytest.mark.parametrize("truncate", [False, True])
+def test_fp64_responses_at_the_knots(layout, truncate):
+    """On every knot, next to it and at both zeros (a knot of the surfaces' first axis
+    is 0): the oracle's response.  A response between the ends is about sixteen
+    operations on terms up to 8 (a cubic of unit values and slopes, its expansion
+    about another origin); beyond the ends, three intervals out, the terms of the
+    cubics reach 8 * 4^3.  The search picks either interval of a knot, where both
+    give the knot's value."""
+    from oracle import oracle as O
+
+    x = np.concatenate([_around([-3.0, -2.0, -1.0, 0.0, 0.5, 1.0, 2.0, 2.5, 3.0]), [-0.0, 1e-300, -1e-300, 0.3, -1.7],
+                        [-5.0, 6.0]])
+    ends = [(t, *({N.GW_DIAL_GENERAL: (-3.0, 2.5), N.GW_DIAL_GRAPH: (-3.0, 2.5), N.GW_DIAL_BILINEAR: (-3.0, 2.0),
+                   N.GW_DIAL_BICUBIC: (-3.0, 2.0), N.GW_DIAL_NORM: (-9.0, 9.0)}.get(t, (-3.0, 3.0)))) for t, _ in DIALS]
+    if truncate:
+        x = np.concatenate([x, [np.inf, -np.inf]])
+    big = np.finfo(np.float64).max  # the clamp of a parameter without one
+    want = np.clip([[O.dial(t, d, v, v, truncate) for t, d in DIALS] for v in x], -big, big)
+    inside = np.array([[truncate or a <= v <= b for _, a, b in ends] for v in x])
+    tol = 16 * 2.0 ** -53 * 8 * np.where(inside, 1.0, 4.0 ** 3)
+    for k in (1, 4, 24, 64):
+        e = engine("fp64", k, layout, truncate=truncate)
+        for family in families(e, k):
+            got = []
+            for i in range(0, x.size, k):
+                pts = np.zeros((k, 3))
+                n = x[i:i + k].size
+                pts[:n, 1:] = x[i:i + k, None]
+                got.append(e.eval(pts)[0][:n])
+            got = np.concatenate(got)
+            for i in range(len(DIALS)):
+                err = np.abs(got[:, i] - want[:, i]) / tol[:, i]
+                assert err.max() <= 1.0, (k, family, DIALS[i][0], x[err.argmax()], err.max())
+        e.close()
