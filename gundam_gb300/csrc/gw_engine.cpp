@@ -804,6 +804,11 @@ int build_and_upload(gw_engine* e) {
   const int B = e->cfg.n_bins;
   const int64_t D = (int64_t)e->dials.size();
   const size_t tsz = sizeof(T);
+  // point columns per row: a batched pass covers up to 64 points; an engine of one
+  // point keeps one column, so that its parameters, clamps aside, fit a few L1
+  // lines (200 parameters 64 columns apart are 200 lines, more than the L1 that
+  // the K = 1 kernels' shared memory leaves: 171 against 146 us for 1M events)
+  e->kpad = e->cfg.k_max == 1 ? 1 : ((e->cfg.k_max + 63) / 64) * 64;
   // stored form of the uniform-knot splines (gw_config.flags).  Default:
   // knot values for FP32 K = 1 engines (bandwidth-bound); the grid form for
   // engines evaluating 32 or more points, where the lanes-over-points kernel
@@ -926,8 +931,7 @@ int build_and_upload(gw_engine* e) {
       });
     }
     for (auto& x : th) x.join();
-    const int64_t kpad_of = ((e->cfg.k_max + 63) / 64) * 64;
-    if (grid_if_small && (int64_t)grids.size() * kpad_of * (int64_t)sizeof(GridPoint<T>) > 32768) {
+    if (grid_if_small && (int64_t)grids.size() * e->kpad * (int64_t)sizeof(GridPoint<T>) > 32768) {
       form = form_small;
       grids.clear();
       grid_of.clear();
@@ -1177,11 +1181,6 @@ int build_and_upload(gw_engine* e) {
   GW_CUDA(e, cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, e->device));
   GW_CUDA(e, cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
   GW_CUDA(e, cudaEventCreateWithFlags(&e->chain_done, cudaEventDisableTiming));
-  // point columns per row: a batched pass covers up to 64 points; an engine of one
-  // point keeps one column, so that its parameters, clamps aside, fit a few L1
-  // lines (200 parameters 64 columns apart are 200 lines, more than the L1 that
-  // the K = 1 kernels' shared memory leaves: 171 against 146 us for 1M events)
-  e->kpad = e->cfg.k_max == 1 ? 1 : ((e->cfg.k_max + 63) / 64) * 64;
   const int P = e->cfg.n_params;
   const int kpad = e->kpad;
 
@@ -1214,7 +1213,6 @@ int build_and_upload(gw_engine* e) {
   v.n_tiles = (int)T_;
   v.kpad = kpad;
   v.llh_type = e->llh_type;
-  v.has_prior = e->has_prior ? 1 : 0;
   v.has_cap = e->has_cap ? 1 : 0;
   v.cap = e->cap;
   v.tile_payload_bytes = (int)(((cap_elems * tsz) + 127) & ~(int64_t)127);

@@ -23,7 +23,6 @@ struct DevView {
   int n_tiles;
   int kpad;             // parameter points per row of the [param][kpad] arrays
   int llh_type;
-  int has_prior;
   int has_cap;
   int n_tables;
   int n_table_fns;

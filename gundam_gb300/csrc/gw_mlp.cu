@@ -2198,7 +2198,6 @@ extern "C" int gwm_train_epochs(gwm_net* n, int32_t epochs, int32_t batch, float
   GWM_CUDA(n, cudaSetDevice(n->device));
   const int64_t N = n->train_n;
   const int64_t spe = N / batch, total = (int64_t)epochs * spe;
-  const int din = n->dims[0], nb = n->dims[n->n_layers];
   // permutations of all epochs, drawn on the host (splitmix64 + Fisher-Yates)
   std::vector<int32_t> perm((size_t)epochs * N);
   uint64_t st = seed;
@@ -2241,8 +2240,6 @@ extern "C" int gwm_train_epochs(gwm_net* n, int32_t epochs, int32_t batch, float
     if (!rc) rc = backward(n, batch);
     if (!rc) rc = adam_all(n, batch, lr);
   }
-  (void)din;
-  (void)nb;
   if (rc == GW_OK) rc = check_status(n);
   if (rc == GW_OK && losses &&
       cudaMemcpy(losses, d_loss, sizeof(float) * epochs, cudaMemcpyDeviceToHost) != cudaSuccess)
@@ -2422,7 +2419,7 @@ struct gwm_chain_state {
   int P = 0;
   bool prior = false;
   float *Lt = nullptr, *icov = nullptr;
-  double *m = nullptr, *phi = nullptr, *f = nullptr, *pen = nullptr;
+  double *m = nullptr, *phi = nullptr, *f = nullptr;
   int32_t* nacc = nullptr;
 };
 
@@ -2433,7 +2430,6 @@ static void chain_free(gwm_chain_state* s) {
   cudaFree(s->icov);
   cudaFree(s->phi);
   cudaFree(s->f);
-  cudaFree(s->pen);
   cudaFree(s->nacc);
   delete s;
 }
@@ -2473,7 +2469,6 @@ extern "C" int gwm_set_chain(gwm_net* n, const double* prop_chol, const double* 
               cudaMalloc(&s->icov, sizeof(float) * P * P) == cudaSuccess &&
               cudaMalloc(&s->phi, sizeof(double) * (size_t)Cm * P) == cudaSuccess &&
               cudaMalloc(&s->f, sizeof(double) * Cm) == cudaSuccess &&
-              cudaMalloc(&s->pen, sizeof(double) * Cm) == cudaSuccess &&
               cudaMalloc(&s->nacc, sizeof(int32_t) * Cm) == cudaSuccess;
     if (!ok) {
       cudaGetLastError();

@@ -15,11 +15,12 @@ chosen index is printed).
 
 train: the C2 surrogate network (200 -> 512 -> 512 -> 512 -> 3000, BF16)
 trained for `steps` (default 8) Adam steps of batch 2048 on a device-resident
-set of 8192 random points (the tcgen05 GEMMs k_gemm, the loss, Adam).
+set of 8192 random points (the tcgen05 products k_gemm, the last with the loss,
+and k_gemm_group, then k_adam).
 
 substeps: 64 surrogate sub-chains of n_sub (default 4) steps with an additive
-head fitted to a synthetic response (k_propose, the GEMMs, k_head_staged,
-k_penalty, k_accept).
+head fitted to a synthetic response (k_propose_stage, the products k_gemm,
+k_head_staged, k_finish_accept).
 
 Profile with e.g.
     ncu --set full --clock-control none -k regex:k_plain -s 2 -c 1 ...
