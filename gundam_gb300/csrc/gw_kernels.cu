@@ -531,6 +531,10 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
       for (int q = 0; q < A; ++q) part[sl + q * SL][bb][kk] = make_double2(s[q], s2[q]);
     } else {
       double s = 0.0, s2 = 0.0;
+      auto add = [](double& x, double& y, const double2& p) {
+        x += p.x;
+        y += p.y;
+      };
       if (n <= kRuns) {  // a slot per run at most: the runs in order are the slots in order
         int r = 0;
         for (; r + 3 < n; r += 4) {  // four rows in flight
@@ -538,34 +542,46 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
 #pragma unroll
           for (int q = 0; q < 4; ++q) p[q] = src[(size_t)(r + q) * v.kpad];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            s += p[q].x;
-            s2 += p[q].y;
-          }
+          for (int q = 0; q < 4; ++q) add(s, s2, p[q]);
         }
-        for (; r < n; ++r) {
-          const double2 p = src[(size_t)r * v.kpad];
-          s += p.x;
-          s2 += p.y;
-        }
+        for (; r < n; ++r) add(s, s2, src[(size_t)r * v.kpad]);
       } else {
-        for (int h = 0; h < kRuns; h += 4) {  // four runs at a time, a row of each in flight
-          double t[4] = {}, t2[4] = {};
-          for (int r = h; r < n; r += kRuns) {
+        // run h has n / 8 slots, the first n % 8 runs one more: unconditional
+        // additions, since even one that adds zero takes its 16 cycles
+        const int full = n / kRuns, rem = n % kRuns;
+        auto runs = [&](int h, int end, int m) {
+          for (; h < end; ++h) {
+            double t = 0.0, t2 = 0.0;
+            const double2* row = src + (size_t)h * v.kpad;
+            for (int i = 0; i < m; ++i, row += (size_t)kRuns * v.kpad) add(t, t2, *row);
+            s += t;
+            s2 += t2;
+          }
+        };
+        if (full == 1) {  // 9 to 15 slots: four of them in flight
+          int h = 0;
+          for (; h + 1 < rem; h += 2) {
             double2 p[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) p[q] = r + q < n ? src[(size_t)(r + q) * v.kpad] : make_double2(0.0, 0.0);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              t[q] += p[q].x;
-              t2[q] += p[q].y;
-            }
+            for (int q = 0; q < 4; ++q) p[q] = src[(size_t)(h + (q >> 1) + (q & 1) * kRuns) * v.kpad];
+            s += p[0].x + p[1].x;
+            s2 += p[0].y + p[1].y;
+            s += p[2].x + p[3].x;
+            s2 += p[2].y + p[3].y;
           }
+          runs(h, rem, 2);
+          h = rem;
+          for (; h + 3 < kRuns; h += 4) {
+            double2 p[4];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            s += t[q];
-            s2 += t2[q];
+            for (int q = 0; q < 4; ++q) p[q] = src[(size_t)(h + q) * v.kpad];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) add(s, s2, p[q]);
           }
+          for (; h < kRuns; ++h) add(s, s2, src[(size_t)h * v.kpad]);
+        } else {
+          runs(0, rem, full + 1);
+          runs(rem, kRuns, full);
         }
       }
       part[0][bb][kk] = make_double2(s, s2);
@@ -613,17 +629,42 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
   const int parts = (v.n_bins + kLlhBins - 1) / kLlhBins;
   double t = 0.0;
   for (int g = warp; g * 32 < parts; g += kLlhRuns) {
-    double x[KT];
+    // this thread's KT parts of the group, four on the way at a time; parts beyond
+    // the last are zeros
+    constexpr int C = KT < 4 ? KT : 4;
+    double x = 0.0, sum1 = 0.0, sum2 = 0.0, sum4 = 0.0;  // x, or of the first of two runs of C, 2 C, 4 C parts
+    const int i0 = g * 32 + sub * KT, n = min(parts - i0, KT);
+    const double* src = v.llh_blocks + (size_t)i0 * v.kpad + k;
+    int c = 0;
+#pragma unroll 1
+    for (; c * C < n; ++c, src += (size_t)C * v.kpad) {
+      double y[C];
 #pragma unroll
-    for (int j = 0; j < KT; ++j) {
-      const int i = g * 32 + sub * KT + j;
-      x[j] = i < parts && k < K ? __ldcg(&v.llh_blocks[(size_t)i * v.kpad + k]) : 0.0;
+      for (int j = 0; j < C; ++j) y[j] = c * C + j < n && k < K ? __ldcg(src + (size_t)j * v.kpad) : 0.0;
+#pragma unroll
+      for (int h = 1; h < C; h <<= 1)
+#pragma unroll
+        for (int j = 0; j < C; j += 2 * h) y[j] += y[j + h];
+      x = y[0];
+      if (c & 1) {
+        x = sum1 + x;
+        if (c & 2) {
+          x = sum2 + x;
+          if (c & 4) x = sum4 + x;
+          else sum4 = x;
+        } else {
+          sum2 = x;
+        }
+      } else {
+        sum1 = x;
+      }
     }
-#pragma unroll
-    for (int h = 1; h < KT; h <<= 1)
-#pragma unroll
-      for (int j = 0; j < KT; j += 2 * h) x[j] += x[j + h];
-    t += neighbour_tree<KT, 32>(x[0]);
+    if (c < KT / C) {  // the rest are zeros: what the tree has so far
+      x = c & 1 ? sum1 : 0.0;
+      if (c & 2) x = sum2 + x;
+      if (c & 4) x = sum4 + x;
+    }
+    t += neighbour_tree<KT, 32>(x);
   }
   if (sub == 0) red[warp * KT + kk] = t;
   __syncthreads();
