@@ -201,35 +201,57 @@ __device__ __forceinline__ void grid_values(uint32_t h, uint32_t pl, const GridP
   for (int j = 0; j < KR; ++j) val[j] = block_cubic(a + (uint32_t)r.g[j].jb * (uint32_t)sizeof(T), r.g[j].u);
 }
 
-// The same of the other dial types (h, hy: the header's two words).
+// Response clamp of a dial: the common [0, 1e20], a table's, a grid's, the
+// parameter's as given (norm dials) or within [-1e20, 1e20] (Calculate*.h).
+// The common one (the default lower bound of a dial collection, no upper bound)
+// is known from the header, so that nothing is loaded.  Checking the bits of an
+// event's responses instead of clamping each, and evaluating an event again
+// when one had left the range, saved three instructions a dial but cost more:
+// of 64 draws from the prior some parameter lies beyond its knots in most events.
 template <typename T, int KR>
-__device__ __forceinline__ void other_values(const DevView& v, uint32_t h, uint32_t hy, uint32_t pl, int k0, int kstep,
-                                             T (&val)[KR]) {
-  const int type = lhdr_type(h);
-  const uint32_t da = pl + lhdr_off(h);
-  const int n = lhdr_n(h);
-  const bool trunc = (h & kLhTrunc) != 0;
-  const T* d = reinterpret_cast<const T*>(__cvta_shared_to_generic(da));
-  if (type >= kTabulated) {
-    // Tabulated.h:27-28 and Kriged.cpp:14-21; per-point tables are laid out [entry][kpad]
-    const TableDesc td = v.tables[hy & 0xFFFFu];
-    const int64_t st = td.per_k ? v.kpad : 1;
-    const T* tab = (const T*)v.table_arena + td.offset;
+__device__ __forceinline__ void clamp_common(T (&val)[KR]) {
 #pragma unroll
-    for (int j = 0; j < KR; ++j) {
-      const int64_t kk = td.per_k ? (int64_t)(k0 + j * kstep) : 0;
-      if (type == kTabulated) {
-        const T f = d[0];
-        const int idx = (int)d[1];
-        val[j] = f * tab[idx * st + kk] + (T(1) - f) * tab[(idx + 1) * st + kk];
-      } else {
-        T a = T(0);
-        for (int q = 0; q < n; ++q) a += d[n + q] * tab[(int64_t)(int)d[q] * st + kk];
-        val[j] = a;
-      }
+  for (int j = 0; j < KR; ++j) val[j] = clamp_response(val[j], T(0.0f), T(1e20));
+}
+// The largest value of a type, the upper clamp of a parameter without one.
+template <typename T>
+__device__ __forceinline__ T open_bound() {
+  return sizeof(T) == 4 ? T(FLT_MAX) : T(DBL_MAX);
+}
+
+// Tabulated.h:27-28 and Kriged.cpp:14-21, clamped to the table's bounds (q: the
+// table; d, n: the dial's payload); per-point tables are laid out [entry][kpad].
+template <typename T, int KR>
+__device__ __forceinline__ void table_values(const DevView& v, int type, uint32_t q, const T* d, int n, int k0,
+                                             int kstep, T (&val)[KR]) {
+  const TableDesc td = v.tables[q];
+  const int64_t st = td.per_k ? v.kpad : 1;
+  const T* tab = (const T*)v.table_arena + td.offset;
+  const T lo = (T)td.lower, hi = (T)td.upper;
+#pragma unroll
+  for (int j = 0; j < KR; ++j) {
+    const int64_t kk = td.per_k ? (int64_t)(k0 + j * kstep) : 0;
+    if (type == kTabulated) {
+      const T f = d[0];
+      const int idx = (int)d[1];
+      val[j] = f * tab[idx * st + kk] + (T(1) - f) * tab[(idx + 1) * st + kk];
+    } else {
+      T a = T(0);
+      for (int i = 0; i < n; ++i) a += d[n + i] * tab[(int64_t)(int)d[i] * st + kk];
+      val[j] = a;
     }
-    return;
   }
+#pragma unroll
+  for (int j = 0; j < KR; ++j) val[j] = clamp_response(val[j], lo, hi);
+}
+
+// The responses of a parameter's dials, before the response clamp (da, d: the
+// dial's payload).
+template <typename T, int KR>
+__device__ __forceinline__ void parameter_values(const DevView& v, uint32_t h, uint32_t hy, uint32_t da, const T* d,
+                                                 int k0, int kstep, T (&val)[KR]) {
+  const int type = lhdr_type(h), n = lhdr_n(h);
+  const bool trunc = (h & kLhTrunc) != 0;
   T x[KR];
   points_of<T, KR>(v, hy & 0xFFFFu, k0, kstep, x);
   if (type == kGeneral) {
@@ -263,47 +285,64 @@ __device__ __forceinline__ void other_values(const DevView& v, uint32_t h, uint3
   }
 }
 
-// Response clamp of a dial: the common [0, 1e20], a table's, a grid's, the
-// parameter's as given (norm dials) or within [-1e20, 1e20] (Calculate*.h).
-// The common one (the default lower bound of a dial collection, no upper bound)
-// is known from the header, so that nothing is loaded.  Checking the bits of an
-// event's responses instead of clamping each, and evaluating an event again
-// when one had left the range, saved three instructions a dial but cost more:
-// of 64 draws from the prior some parameter lies beyond its knots in most events.
-template <typename T, int KR>
-__device__ __forceinline__ void clamp_common(T (&val)[KR]) {
-#pragma unroll
-  for (int j = 0; j < KR; ++j) val[j] = clamp_response(val[j], T(0.0f), T(1e20));
-}
-// The largest value of a type, the upper clamp of a parameter without one.
-template <typename T>
-__device__ __forceinline__ T open_bound() {
-  return sizeof(T) == 4 ? T(FLT_MAX) : T(DBL_MAX);
-}
-template <typename T, int KR>
-__device__ __forceinline__ void clamp_values(const DevView& v, uint32_t h, uint32_t hy, T (&val)[KR]) {
+// The clamped responses of the dials that the kernel has no shorter path for (h,
+// hy: the header's two words; pl, base: the tile's payload; g: a grid dial's
+// points, when `have_grid`).  A clamp that is not the common one is loaded before the
+// response is formed: one tile per SM and one point per lane is a chain of
+// latencies (7200 tabulated dials 28 -> 21 us, splines on grids 13.9 -> 12.5).  Two
+// 8-byte points per lane are short of registers and load it after (200k events in
+// FP64, 64 points: 1.74 against 1.76 ms).
+template <typename T, int KR, bool have_grid>
+__device__ __forceinline__ void other_values(const DevView& v, uint32_t h, uint32_t hy, uint32_t pl, const T* base,
+                                             int k0, int kstep, GridPoints<T, KR>& g, T (&val)[KR]) {
+  constexpr bool kEarly = sizeof(T) == 4 || KR == 1;
+  using V2 = typename Vec2<T>::type;
   const int type = lhdr_type(h);
-  if ((h & kLhCommonClamp) && type != kNorm) {
-    clamp_common<T, KR>(val);
-    return;
-  }
-  const uint32_t q = hy & 0xFFFFu;
-  T lo, hi;
-  if (type == kTabulated || type == kKriged) {
-    const TableDesc td = v.tables[q];
-    lo = (T)td.lower;
-    hi = (T)td.upper;
-  } else {
-    const typename Vec2<T>::type c = ((const typename Vec2<T>::type*)(type == kGrid ? v.grid_clamp : v.pclamp))[q];
-    lo = c.x;
-    hi = c.y;
-    if (type != kNorm) {
+  const uint32_t da = pl + lhdr_off(h), q = hy & 0xFFFFu;
+  const T* d = kEarly ? (const T*)((const unsigned char*)base + lhdr_off(h))
+                      : reinterpret_cast<const T*>(__cvta_shared_to_generic(da));
+  auto grid = [&]() {
+    if constexpr (!have_grid) grid_points<T, KR>(v, q, k0, kstep, g);
+    grid_values<T, KR>(h, pl, g, val);
+  };
+  auto clamp = [&](const V2& c) {
+    T lo = c.x, hi = c.y;
+    if (type != kNorm && type != kGrid) {
       if (lo < T(-1e20)) lo = T(-1e20);
       if (hi > T(1e20)) hi = T(1e20);
     }
-  }
 #pragma unroll
-  for (int j = 0; j < KR; ++j) val[j] = clamp_response(val[j], lo, hi);
+    for (int j = 0; j < KR; ++j) val[j] = clamp_response(val[j], lo, hi);
+  };
+  const bool common = (h & kLhCommonClamp) && type != kNorm;
+  if constexpr (kEarly) {
+    if (type >= kTabulated) {
+      if (type == kGrid) {
+        const V2 c = ((const V2*)v.grid_clamp)[q];
+        grid();
+        clamp(c);
+      } else {
+        table_values<T, KR>(v, type, q, d, lhdr_n(h), k0, kstep, val);
+      }
+      return;
+    }
+    V2 c;
+    if (!common) c = ((const V2*)v.pclamp)[q];
+    parameter_values<T, KR>(v, h, hy, da, d, k0, kstep, val);
+    if (common) clamp_common<T, KR>(val);
+    else clamp(c);
+  } else {
+    if (type == kGrid) {
+      grid();
+    } else if (type >= kTabulated) {
+      table_values<T, KR>(v, type, q, d, lhdr_n(h), k0, kstep, val);
+      return;
+    } else {
+      parameter_values<T, KR>(v, h, hy, da, d, k0, kstep, val);
+    }
+    if (common) clamp_common<T, KR>(val);
+    else clamp(((const V2*)(type == kGrid ? v.grid_clamp : v.pclamp))[q]);
+  }
 }
 
 }  // namespace

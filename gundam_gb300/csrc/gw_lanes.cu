@@ -164,13 +164,7 @@ __global__ void __launch_bounds__(NT, MB) k_batched(const DevView v, int K) {
 #pragma unroll
               for (int j = 0; j < KR; ++j) val[j] = clamp_response(val[j], T(0.0f), open_bound<T>());
             } else {
-              if (lhdr_type(h.x) == kGrid) {
-                if constexpr (!kAhead) grid_points<T, KR>(v, h.y & 0xFFFFu, k0, KC, g);
-                grid_values<T, KR>(h.x, pl, g, val);
-              } else {
-                other_values<T, KR>(v, h.x, h.y, pl, k0, KC, val);
-              }
-              clamp_values<T, KR>(v, h.x, h.y, val);
+              other_values<T, KR, kAhead>(v, h.x, h.y, pl, (const T*)stage, k0, KC, g, val);
             }
 #pragma unroll
             for (int j = 0; j < KR; ++j) w[j] *= val[j];
