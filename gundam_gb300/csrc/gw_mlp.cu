@@ -739,15 +739,20 @@ struct HeadOut {
   bf16* dy;
 };
 
-// Likelihood term of one (point m, bin) from the base `acc` and the log ratio
-// `racc`, with its optional outputs.
+// The network's output at (point m, bin), loaded before any output is stored.
+__device__ __forceinline__ float head_mlp(const Head& h, const float* mlp, int C, int m, int bin) {
+  return bin < h.nb && m < C ? mlp[(size_t)m * h.nb + bin] : 0.f;
+}
+
+// Likelihood term of one (point m, bin) from the base `acc`, the log ratio `racc`
+// and the network's output y, with its optional outputs.
 template <bool GRAD>
-__device__ __forceinline__ double head_term(const Head& h, const float* mlp, int C, int m, int bin,
+__device__ __forceinline__ double head_term(const Head& h, float y, int C, int m, int bin,
                                             const double* __restrict__ data, int llh_type, float acc, float racc,
                                             const HeadOut& out) {
   if (bin >= h.nb || m >= C) return 0.0;
   const size_t o = (size_t)m * h.nb + bin;
-  const float lr = acc + h.mu[bin] + h.sd[bin] * mlp[o];
+  const float lr = acc + h.mu[bin] + h.sd[bin] * y;
   const float mu = expf(lr), s2 = expf(lr + racc);
   if (out.sums) out.sums[o] = (double)mu;
   if (out.sums2) out.sums2[o] = (double)s2;
@@ -904,14 +909,19 @@ __global__ void __launch_bounds__(kHeadThreads, 3) k_head_staged(const __grid_co
     }
     if (tid == 0 && c + kHeadStages < nchunk) issue(c + kHeadStages);
   }
+  float y[2][2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) y[j][i] = head_mlp(h, mlp, C, mb + warp + 4 * j, bin + i);
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     float a0, a1, r0, r1;
     upk2(acc[j], a0, a1);
     upk2(racc[j], r0, r1);
     const int m = mb + warp + 4 * j;
-    const double t0 = head_term<GRAD>(h, mlp, C, m, bin, data, llh_type, a0, r0, out);
-    const double t1 = head_term<GRAD>(h, mlp, C, m, bin + 1, data, llh_type, a1, r1, out);
+    const double t0 = head_term<GRAD>(h, y[j][0], C, m, bin, data, llh_type, a0, r0, out);
+    const double t1 = head_term<GRAD>(h, y[j][1], C, m, bin + 1, data, llh_type, a1, r1, out);
     head_part(t0 + t1, C, m, out.part);
   }
 }
@@ -923,7 +933,11 @@ __global__ void __launch_bounds__(kHeadThreads, 3) k_head_staged(const __grid_co
 // table offset of the interpolation interval and its weight in shared memory;
 // the inner loop is then two coalesced table loads and two FMAs per point and
 // parameter, with the table lines of a bin shared through L1 across the
-// block's points.
+// block's points.  Four parameters' loads are issued before the first is used:
+// left to the compiler, the form without gradients came to 40 registers, fewer
+// loads in flight and a sixth block per SM that took the L1 from the others (200
+// parameters, 16 nodes, 3000 bins, 2048 points: a call 1312 us, 1077 with 48
+// registers, 998 now; 64 points 164 -> 130).
 template <int PPT, bool GRAD>
 __global__ void __launch_bounds__(256) k_head_llh(Head h, const float* x, const float* mlp, int C,
                                                   const double* __restrict__ data, int llh_type, HeadOut out) {
@@ -939,19 +953,27 @@ __global__ void __launch_bounds__(256) k_head_llh(Head h, const float* x, const 
   const int tid = threadIdx.y * 32 + threadIdx.x;
   const bool additive = h.nodes >= 2;
   const float inv_w = additive ? (float)(h.nodes - 1) / (2.f * h.lim) : 0.f;
-  for (int e = tid; e < NP * din; e += 256) {
-    const int ml = e / din, k = e - ml * din, m = mb + ml;
-    const float z = m < C ? x[(size_t)m * din + k] : 0.f;
-    s_z[e] = z;
-    if (additive) {
-      const float xc = fminf(fmaxf(z, -h.lim), h.lim);
-      const float u = (xc + h.lim) * inv_w;
-      const int i = min((int)u, h.nodes - 2);
-      s_t[e] = u - (float)i;
-      s_off[e] = (k * h.nodes + i) * h.nb;
-    } else {
-      s_t[e] = z;
-      s_off[e] = k * h.nb;
+  const float* xb = x + (size_t)mb * din;
+  const int rows = min(C - mb, NP) * din;
+  for (int e0 = tid; e0 < NP * din; e0 += 4 * 256) {
+    float z[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) z[q] = e0 + q * 256 < rows ? xb[e0 + q * 256] : 0.f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = e0 + q * 256, k = e % din;
+      if (e >= NP * din) break;
+      s_z[e] = z[q];
+      if (additive) {
+        const float xc = fminf(fmaxf(z[q], -h.lim), h.lim);
+        const float u = (xc + h.lim) * inv_w;
+        const int i = min((int)u, h.nodes - 2);
+        s_t[e] = u - (float)i;
+        s_off[e] = (k * h.nodes + i) * h.nb;
+      } else {
+        s_t[e] = z[q];
+        s_off[e] = k * h.nb;
+      }
     }
   }
   __syncthreads();
@@ -967,28 +989,39 @@ __global__ void __launch_bounds__(256) k_head_llh(Head h, const float* x, const 
     const float* __restrict__ tab = h.tab + bin;
     const float* __restrict__ rw = h.r_w ? h.r_w + bin : nullptr;
     const int nb = h.nb;
-#pragma unroll 4
-    for (int k = 0; k < din; ++k) {
-      const float w = rw ? __ldg(rw + (size_t)k * nb) : 0.f;
+    // four parameters' table rows on the way at a time (din is a multiple of 8)
+    constexpr int U = 4;
+    for (int k = 0; k < din; k += U) {
+      float w[U], lo[U][PPT], hi[U][PPT];
 #pragma unroll
-      for (int j = 0; j < PPT; ++j) {
-        const int e = (threadIdx.y + 8 * j) * din + k;
-        const int off = s_off[e];
-        const float t = s_t[e];
-        if (additive) {
-          const float lo = __ldg(tab + off), hi = __ldg(tab + off + nb);
-          acc[j] += fmaf(t, hi - lo, lo);
-        } else {
-          acc[j] = fmaf(t, __ldg(tab + off), acc[j]);
+      for (int u = 0; u < U; ++u) {
+        w[u] = rw ? __ldg(rw + (size_t)(k + u) * nb) : 0.f;
+#pragma unroll
+        for (int j = 0; j < PPT; ++j) {
+          const int off = s_off[(threadIdx.y + 8 * j) * din + k + u];
+          lo[u][j] = __ldg(tab + off);
+          hi[u][j] = additive ? __ldg(tab + off + nb) : 0.f;
         }
-        racc[j] = fmaf(s_z[e], w, racc[j]);
       }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < PPT; ++j) {
+          const int e = (threadIdx.y + 8 * j) * din + k + u;
+          const float t = s_t[e];
+          if (additive) acc[j] += fmaf(t, hi[u][j] - lo[u][j], lo[u][j]);
+          else acc[j] = fmaf(t, lo[u][j], acc[j]);
+          racc[j] = fmaf(s_z[e], w[u], racc[j]);
+        }
     }
   }
+  float y[PPT];
+#pragma unroll
+  for (int j = 0; j < PPT; ++j) y[j] = head_mlp(h, mlp, C, mb + threadIdx.y + 8 * j, bin);
 #pragma unroll
   for (int j = 0; j < PPT; ++j) {
     const int m = mb + threadIdx.y + 8 * j;
-    head_part(head_term<GRAD>(h, mlp, C, m, bin, data, llh_type, acc[j], racc[j], out), C, m, out.part);
+    head_part(head_term<GRAD>(h, y[j], C, m, bin, data, llh_type, acc[j], racc[j], out), C, m, out.part);
   }
 }
 
@@ -1021,9 +1054,21 @@ __global__ void __launch_bounds__(256) k_base_grad(Head h, const float* x, const
   float* g = shg;            // [nb]
   float* sg = shg + h.nb;    // [nb]
   const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int b = tid; b < h.nb; b += 256) {
-    g[b] = G[(size_t)m * h.nb + b];
-    sg[b] = S[(size_t)m * h.nb + b];
+  const float *Gm = G + (size_t)m * h.nb, *Sm = S + (size_t)m * h.nb;
+  for (int b0 = tid; b0 < h.nb; b0 += 4 * 256) {  // four of each on the way
+    float vg[4], vs[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int b = min(b0 + q * 256, h.nb - 1);
+      vg[q] = Gm[b];
+      vs[q] = Sm[b];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (b0 + q * 256 < h.nb) {
+        g[b0 + q * 256] = vg[q];
+        sg[b0 + q * 256] = vs[q];
+      }
   }
   __syncthreads();
   const bool additive = h.nodes >= 2;
