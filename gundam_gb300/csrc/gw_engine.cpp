@@ -1377,8 +1377,12 @@ int build_and_upload(gw_engine* e) {
   v.partials = (double2*)p;
   if ((rc = alloc(sizeof(double) * (size_t)kpad * ((B + kLlhBins - 1) / kLlhBins), &p))) return rc;
   v.llh_blocks = (double*)p;
-  if ((rc = alloc(sizeof(unsigned int) * kpad, &p))) return rc;
-  GW_CUDA(e, cudaMemset(p, 0, sizeof(unsigned int) * kpad));
+  const size_t groups = ((size_t)B + 255) / 256;
+  if ((rc = alloc(sizeof(double) * groups * kpad, &p))) return rc;
+  v.llh_groups = (double*)p;
+  const size_t counters = sizeof(unsigned int) * (1 + (size_t)kpad / 32) * (1 + groups);
+  if ((rc = alloc(counters, &p))) return rc;
+  GW_CUDA(e, cudaMemset(p, 0, counters));
   v.llh_counter = (unsigned int*)p;
   // evaluation I/O buffers
   if ((rc = alloc(sizeof(double) * (size_t)kpad * P, &e->d_params))) return rc;

@@ -70,7 +70,8 @@ struct DevView {
   double* penalty;            // [n_pen * kpad] parts of delta^T C^-1 delta, one row of points per block
   double2* partials;          // [n_slots * kpad]  (scratch)
   double* llh_blocks;         // [ceil(n_bins / kLlhBins) * kpad] (scratch)
-  unsigned int* llh_counter;  // [kpad]           (scratch)
+  double* llh_groups;         // [ceil(n_bins / 256) * kpad] sums of 256 bins' terms (scratch)
+  unsigned int* llh_counter;  // [(1 + kpad / 32) * (1 + ceil(n_bins / 256))] blocks done, per point tile (scratch)
   double* event_weights;      // [n_events] in result order, or nullptr
   uint32_t* status;
 };
@@ -123,6 +124,6 @@ int batched_blocks_per_sm(const DevView& v, const BatchedShape& b);
 
 constexpr int kPlainThreads = 256;
 constexpr int kPenRows = 8;  // rows of C^-1 per penalty block of k_params
-constexpr int kLlhBins = 8;  // bins per part of k_bins_llh's likelihood sum (its smallest block)
+constexpr int kLlhBins = 8;  // bins of k_bins_llh's smallest block
 
 }  // namespace gw

@@ -480,18 +480,22 @@ __global__ void __launch_bounds__(NEV + kWsRed, sizeof(T) == 4 ? 3 : 2) k_plain_
 //      runs are added in order, so that a point's sums do not depend on how many
 //      points share the call;
 //   2. thread (bin, point), bins fastest, writes the sums and evaluates the
-//      likelihood term; the terms of 8 bins of a point are added;
-//   3. the last block of a point tile adds these parts, in the order of
-//      kLlhGroup, and the penalty's: warp w run w, thread (point kk, sub) of it KT
-//      parts of each sum of 256 bins, all on the way at once.
-// A Barlow-Beeston term is ~80 FP64 operations and an SM issues one warp of
-// them every 16 cycles (pipe busy 84 % at 10000 bins, 100 points: 203 us, 232
-// with CUDA's logarithm, a third square root and FP64 compares; see
-// llh_bb_oa2021), so the terms are cut into many small blocks with full warps:
-// 256 bins per block left 140 SMs idle at K = 1 (19.2 us for 3000 bins, now
-// 13.5 us; the launch alone is 5 us).  The small KT give their threads to the
-// slots of a bin instead,
-// whose reads are a chain of L2 latencies.
+//      likelihood term; the BT terms of a point are added;
+//   3. these parts are added in the order of kLlhGroup, by the last block of the
+//      point tile, or, where that block would have more than kOneLevel of them per
+//      thread, by the last block of each group of 256 bins and then by the last of
+//      all, which adds the penalty's.
+// A Barlow-Beeston term is ~85 FP64 operations and an SM issues one warp of
+// them every 16 cycles (10000 bins, 100 points: 189 us, 232 with CUDA's logarithm, a
+// third square root and FP64 compares; see llh_bb_oa2021), so the terms are cut
+// into many small blocks with full warps: 256 bins per block left 140 SMs idle at
+// K = 1 (19.2 us for 3000 bins, now 12.5 us; the launch alone is 5 us).  The small
+// KT give their threads to the slots of a bin instead, whose reads are a chain of
+// L2 latencies.  Adding the parts in two levels takes a second arrival (1 us), in
+// one level the parts go through a single SM (10000 bins, 100 points: 208 us that
+// way; 100000 bins, 16 points: 140 us of 616), so the line lies where a thread of
+// the last block would wait for more than a few rounds of loads.
+constexpr int kOneLevel = 16;
 template <int KT, int BT>
 __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double* sums, double* sums2,
                                                   double* llh, double* llh_stat) {
@@ -500,6 +504,7 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
   constexpr int kRuns = 8, kParts = SL > 1 ? kRuns : 1;  // one thread per bin and point adds its runs itself
   static_assert(kRuns % SL == 0, "whole runs per slot lane");
   __shared__ double2 part[kParts][BT][KT + (KT > 1 ? 1 : 0)];
+  __shared__ int slots[BT];
   __shared__ double red[kLlhRuns * KT];
   __shared__ bool last;
   const int tid = threadIdx.x;
@@ -512,76 +517,104 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
     const int n = b < v.n_bins && k < K ? v.bin_slot[b + 1] - i0 : 0;
     const double2* src = v.partials + (size_t)i0 * v.kpad + k;
     if constexpr (SL > 1) {
-      constexpr int A = kRuns / SL, U = A < 4 ? 4 / A : 1;  // runs of this thread; four rows in flight
+      if (kk == 0 && sl == 0) slots[bb] = n;
+      constexpr int A = kRuns / SL, R = 4;  // runs of this thread, rows in flight
+      static_assert(R % A == 0, "whole periods");
       double s[A] = {}, s2[A] = {};
-      for (int r = sl; r < n; r += U * kRuns) {
-        double2 p[U][A];
+      int r = sl;
+      for (; r + (R - 1) * SL < n; r += R * SL) {
+        double2 p[R];
 #pragma unroll
-        for (int q = 0; q < U * A; ++q) {
-          const int i = r + q * SL;
-          p[q / A][q % A] = i < n ? src[(size_t)i * v.kpad] : make_double2(0.0, 0.0);
-        }
+        for (int q = 0; q < R; ++q) p[q] = src[(size_t)(r + q * SL) * v.kpad];
 #pragma unroll
-        for (int q = 0; q < U * A; ++q) {
-          s[q % A] += p[q / A][q % A].x;
-          s2[q % A] += p[q / A][q % A].y;
+        for (int q = 0; q < R; ++q) {
+          s[q % A] += p[q].x;
+          s2[q % A] += p[q].y;
         }
+      }
+      if constexpr (A == 1) {  // most lanes have no slot: nothing is issued for them
+        for (; r < n; r += SL) {
+          const double2 p = src[(size_t)r * v.kpad];
+          s[0] += p.x;
+          s2[0] += p.y;
+        }
+      } else {
+        double2 p[R - 1];
+#pragma unroll
+        for (int q = 0; q < R - 1; ++q)
+          if (r + q * SL < n) p[q] = src[(size_t)(r + q * SL) * v.kpad];
+#pragma unroll
+        for (int q = 0; q < R - 1; ++q)
+          if (r + q * SL < n) {
+            s[q % A] += p[q].x;
+            s2[q % A] += p[q].y;
+          }
       }
 #pragma unroll
       for (int q = 0; q < A; ++q) part[sl + q * SL][bb][kk] = make_double2(s[q], s2[q]);
     } else {
+      // additions of rows that are there only: even one that adds zero takes its 16
+      // cycles; four rows in flight
       double s = 0.0, s2 = 0.0;
+      auto row = [&](int i) { return src[(size_t)i * v.kpad]; };
       auto add = [](double& x, double& y, const double2& p) {
         x += p.x;
         y += p.y;
       };
       if (n <= kRuns) {  // a slot per run at most: the runs in order are the slots in order
         int r = 0;
-        for (; r + 3 < n; r += 4) {  // four rows in flight
+        for (; r + 3 < n; r += 4) {
           double2 p[4];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) p[q] = src[(size_t)(r + q) * v.kpad];
+          for (int q = 0; q < 4; ++q) p[q] = row(r + q);
 #pragma unroll
           for (int q = 0; q < 4; ++q) add(s, s2, p[q]);
         }
-        for (; r < n; ++r) add(s, s2, src[(size_t)r * v.kpad]);
+        for (; r < n; ++r) add(s, s2, row(r));
+      } else if (n < 2 * kRuns) {  // two slots in the first n - 8 runs, one in the others
+        const int two = n - kRuns;
+        int h = 0;
+        for (; h + 1 < two; h += 2) {
+          double2 p[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) p[q] = row(h + (q >> 1) + (q & 1) * kRuns);
+          s += p[0].x + p[1].x;
+          s2 += p[0].y + p[1].y;
+          s += p[2].x + p[3].x;
+          s2 += p[2].y + p[3].y;
+        }
+        if (h < two) {
+          const double2 p = row(h), q = row(h + kRuns);
+          s += p.x + q.x;
+          s2 += p.y + q.y;
+        }
+        h = two;
+        for (; h + 3 < kRuns; h += 4) {
+          double2 p[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) p[q] = row(h + q);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) add(s, s2, p[q]);
+        }
+        for (; h < kRuns; ++h) add(s, s2, row(h));
       } else {
-        // run h has n / 8 slots, the first n % 8 runs one more: unconditional
-        // additions, since even one that adds zero takes its 16 cycles
-        const int full = n / kRuns, rem = n % kRuns;
-        auto runs = [&](int h, int end, int m) {
-          for (; h < end; ++h) {
-            double t = 0.0, t2 = 0.0;
-            const double2* row = src + (size_t)h * v.kpad;
-            for (int i = 0; i < m; ++i, row += (size_t)kRuns * v.kpad) add(t, t2, *row);
-            s += t;
-            s2 += t2;
-          }
-        };
-        if (full == 1) {  // 9 to 15 slots: four of them in flight
-          int h = 0;
-          for (; h + 1 < rem; h += 2) {
+#pragma unroll 1
+        for (int h = 0; h < kRuns; h += 4) {  // four runs at a time, each a sum of its own
+          double2 t[4] = {};
+          int i = h;
+#pragma unroll 1
+          for (; i + 3 < n; i += kRuns) {
             double2 p[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) p[q] = src[(size_t)(h + (q >> 1) + (q & 1) * kRuns) * v.kpad];
-            s += p[0].x + p[1].x;
-            s2 += p[0].y + p[1].y;
-            s += p[2].x + p[3].x;
-            s2 += p[2].y + p[3].y;
-          }
-          runs(h, rem, 2);
-          h = rem;
-          for (; h + 3 < kRuns; h += 4) {
-            double2 p[4];
+            for (int q = 0; q < 4; ++q) p[q] = row(i + q);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) p[q] = src[(size_t)(h + q) * v.kpad];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) add(s, s2, p[q]);
+            for (int q = 0; q < 4; ++q) add(t[q].x, t[q].y, p[q]);
           }
-          for (; h < kRuns; ++h) add(s, s2, src[(size_t)h * v.kpad]);
-        } else {
-          runs(0, rem, full + 1);
-          runs(rem, kRuns, full);
+#pragma unroll
+          for (int q = 0; q < 3; ++q)
+            if (i + q < n) add(t[q].x, t[q].y, row(i + q));
+#pragma unroll
+          for (int q = 0; q < 4; ++q) add(s, s2, t[q]);
         }
       }
       part[0][bb][kk] = make_double2(s, s2);
@@ -596,12 +629,17 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
     double term = 0.0;
     if (in) {
       double s = 0.0, s2 = 0.0;
-#pragma unroll
-      for (int q = 0; q < kParts; ++q) {
-        const double2 p = part[q][bb][kk];
-        s = q ? s + p.x : p.x;
-        s2 = q ? s2 + p.y : p.y;
+      {
+        const double2 p = part[0][bb][kk];
+        s = p.x;
+        s2 = p.y;
       }
+      if constexpr (kParts > 1)
+        for (int q = 1; q < min(slots[bb], kParts); ++q) {  // the runs that have a slot
+          const double2 p = part[q][bb][kk];
+          s += p.x;
+          s2 += p.y;
+        }
       if (sums) sums[(size_t)k * v.n_bins + b] = s;
       if (sums2) sums2[(size_t)k * v.n_bins + b] = s2;
       if (want_llh) {
@@ -613,58 +651,95 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
     }
     if (want_llh) {
       // whole warps are in this branch (KT * BT is a multiple of 32)
-      term = neighbour_tree<1, kLlhBins>(term);
-      if (in && bb % kLlhBins == 0) v.llh_blocks[(size_t)(b / kLlhBins) * v.kpad + k] = term;
+      term = neighbour_tree<1, BT>(term);
+      if (in && bb == 0) v.llh_blocks[(size_t)blockIdx.x * v.kpad + k] = term;
     }
   }
   if (!want_llh) return;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) last = atomicAdd(&v.llh_counter[blockIdx.y], 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  static_assert(NT == 32 * kLlhRuns && kLlhGroup == 32 * kLlhBins && KT <= 32, "a warp per run");
+  static_assert(NT == 32 * kLlhRuns && kLlhGroup % BT == 0 && KT <= 32, "a warp per run, whole blocks per group");
+  constexpr int PG = kLlhGroup / BT;  // parts per group
   const int warp = tid >> 5, kk = tid % KT, sub = (tid & 31) / KT, k = kb + kk;
-  const int parts = (v.n_bins + kLlhBins - 1) / kLlhBins;
+  const int parts = gridDim.x, groups = (parts + PG - 1) / PG;
+  unsigned int* const counter = v.llh_counter + (size_t)blockIdx.y * (groups + 1);  // per group, and one for all
+  auto part_of = [&](int i) { return i < parts && k < K ? __ldcg(&v.llh_blocks[(size_t)i * v.kpad + k]) : 0.0; };
+  // whether this block is the last of `of` to arrive at counter c, its own results visible
+  auto last_of = [&](int c, int of) {
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+      last = atomicAdd(&counter[c], 1u) == (unsigned)of - 1;
+      if (last) counter[c] = 0u;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+  };
+  // one level: a warp, L lanes per point and group, X parts per lane, G groups at a time
+  constexpr int L = 32 / KT < PG ? 32 / KT : PG, X = PG / L, G = 32 / KT / L;
   double t = 0.0;
-  for (int g = warp; g * 32 < parts; g += kLlhRuns) {
-    // this thread's KT parts of the group, four on the way at a time; parts beyond
-    // the last are zeros
-    constexpr int C = KT < 4 ? KT : 4;
-    double x = 0.0, sum1 = 0.0, sum2 = 0.0, sum4 = 0.0;  // x, or of the first of two runs of C, 2 C, 4 C parts
-    const int i0 = g * 32 + sub * KT, n = min(parts - i0, KT);
-    const double* src = v.llh_blocks + (size_t)i0 * v.kpad + k;
-    int c = 0;
-#pragma unroll 1
-    for (; c * C < n; ++c, src += (size_t)C * v.kpad) {
-      double y[C];
+  if (X > kOneLevel || (groups + kLlhRuns * G - 1) / (kLlhRuns * G) * X > kOneLevel) {
+    // this block's group: P neighbouring parts per thread, T threads per point
+    constexpr int P = PG * KT > NT ? PG * KT / NT : 1, T = PG / P, W = T * KT > 32 ? T * KT / 32 : 1;
+    const int g = blockIdx.x / PG, j0 = tid / KT * P;
+    if (!last_of(g, min(parts - g * PG, PG))) return;
+    double y[P];
 #pragma unroll
-      for (int j = 0; j < C; ++j) y[j] = c * C + j < n && k < K ? __ldcg(src + (size_t)j * v.kpad) : 0.0;
+    for (int j = 0; j < P; ++j) y[j] = j0 < PG ? part_of(g * PG + j0 + j) : 0.0;
 #pragma unroll
-      for (int h = 1; h < C; h <<= 1)
+    for (int h = 1; h < P; h <<= 1)
 #pragma unroll
-        for (int j = 0; j < C; j += 2 * h) y[j] += y[j + h];
-      x = y[0];
-      if (c & 1) {
-        x = sum1 + x;
-        if (c & 2) {
-          x = sum2 + x;
-          if (c & 4) x = sum4 + x;
-          else sum4 = x;
-        } else {
-          sum2 = x;
-        }
-      } else {
-        sum1 = x;
+      for (int j = 0; j < P; j += 2 * h) y[j] += y[j + h];
+    t = neighbour_tree<KT, W == 1 ? T * KT : 32>(y[0]);
+    if (sub == 0) red[warp * KT + kk] = t;
+    __syncthreads();
+    if (tid < KT && k < K) {
+      double w[W];
+#pragma unroll
+      for (int i = 0; i < W; ++i) w[i] = red[i * KT + kk];
+#pragma unroll
+      for (int h = 1; h < W; h <<= 1)
+#pragma unroll
+        for (int i = 0; i < W; i += 2 * h) w[i] += w[i + h];
+      if (groups > 1) v.llh_groups[(size_t)g * v.kpad + k] = w[0];
+      t = w[0];
+    }
+    if (groups > 1) {
+      if (!last_of(groups, groups)) return;
+      t = 0.0;
+      // 32 / KT groups of the run at a time, added in order
+      constexpr int S = 32 / KT;
+#pragma unroll 4
+      for (int g0 = warp; g0 < groups; g0 += kLlhRuns * S) {
+        const int i = g0 + kLlhRuns * sub;
+        const double x = i < groups && k < K ? __ldcg(&v.llh_groups[(size_t)i * v.kpad + k]) : 0.0;
+#pragma unroll
+        for (int q = 0; q < S; ++q) t += S > 1 ? __shfl_sync(0xffffffffu, x, q * KT + kk) : x;
+      }
+    } else {
+      if (tid >= KT) t = 0.0;  // the one group is run 0, the others are empty
+      __syncthreads();
+    }
+  } else {
+    if (!last_of(groups, parts)) return;
+    constexpr int U = X < 4 ? 4 / X : 1;  // rounds in flight
+    for (int g0 = warp; g0 < groups; g0 += kLlhRuns * G * U) {
+      double y[U][X];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < X; ++j) y[u][j] = part_of((g0 + kLlhRuns * (u * G + sub / L)) * PG + sub % L * X + j);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (g0 + kLlhRuns * u * G >= groups) break;
+#pragma unroll
+        for (int h = 1; h < X; h <<= 1)
+#pragma unroll
+          for (int j = 0; j < X; j += 2 * h) y[u][j] += y[u][j + h];
+        const double x = neighbour_tree<KT, KT * L>(y[u][0]);
+#pragma unroll
+        for (int q = 0; q < G; ++q) t += G > 1 ? __shfl_sync(0xffffffffu, x, q * L * KT + kk) : x;
       }
     }
-    if (c < KT / C) {  // the rest are zeros: what the tree has so far
-      x = c & 1 ? sum1 : 0.0;
-      if (c & 2) x = sum2 + x;
-      if (c & 4) x = sum4 + x;
-    }
-    t += neighbour_tree<KT, 32>(x);
   }
   if (sub == 0) red[warp * KT + kk] = t;
   __syncthreads();
@@ -678,7 +753,6 @@ __global__ void __launch_bounds__(256) k_bins_llh(const DevView v, int K, double
     if (llh_stat) llh_stat[k] = t;
     if (llh) llh[k] = t + pen;
   }
-  if (tid == 0) v.llh_counter[blockIdx.y] = 0u;
 }
 
 // log(data) per bin, taken once when the data are set instead of per bin and
@@ -890,8 +964,8 @@ cudaError_t launch_bins_llh(const DevView& v, int K, double* sums, double* sums2
   auto grid = [&](int kt, int bt) { return dim3((v.n_bins + bt - 1) / bt, (K + kt - 1) / kt); };
   if (K == 1)
     return launch_dependent(k_bins_llh<1, 32>, grid(1, 32), 256, 0, s, v, K, sums, sums2, llh, llh_stat);
-  if (K <= 4)
-    k_bins_llh<4, 16><<<grid(4, 16), 256, 0, s>>>(v, K, sums, sums2, llh, llh_stat);
+  if (K <= 4)  // a warp of terms per point: of three points in one tile of four, a quarter was idle
+    k_bins_llh<2, 32><<<grid(2, 32), 256, 0, s>>>(v, K, sums, sums2, llh, llh_stat);
   else if (K <= 8)
     k_bins_llh<8, 16><<<grid(8, 16), 256, 0, s>>>(v, K, sums, sums2, llh, llh_stat);
   else if (K <= 16)

@@ -56,8 +56,9 @@ def test_sums_of_a_point_at_every_number_of_points():
     e.close()
 
 
-# bins: one part of 8, one group of 256 and a bin, more groups than runs
-@pytest.mark.parametrize("n_bins", [8, 257, 2500])
+# bins: one part of 8, one group of 256 and a bin, more groups than runs, and so many
+# that one point's parts are added in two levels as well
+@pytest.mark.parametrize("n_bins", [8, 257, 2500, 17000])
 @pytest.mark.parametrize("llh_type", [N.GW_LLH_POISSON, N.GW_LLH_BARLOW_BEESTON_OA2021])
 def test_likelihood_of_a_point_at_every_number_of_points(llh_type, n_bins):
     torch = pytest.importorskip("torch")
