@@ -405,7 +405,8 @@ __device__ __forceinline__ double log_data_of(double data) {
 // = -1, fractionalErrorLimit = 1e150, usePoissonLikelihood = false); root =
 // sqrt(mcuncert).  Its FP64 operations bound k_bins_llh, so the tests that
 // nearly always go one way look at the high words first, and the logarithm is
-// that of gw_log.cuh (10000 bins, 100 points: 232 -> 203 us with both).
+// that of gw_log.cuh (10000 bins, 100 points: 232 us without, 203 with both, of
+// which the logarithm's last half ulp costs 5).
 __device__ __forceinline__ double llh_bb_oa2021(double data, double log_data, double pred, double mcuncert,
                                                 double root) {
   if (__double2hiint(pred) < 0 && pred <= -1.0) {

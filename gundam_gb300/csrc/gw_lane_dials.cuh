@@ -3,8 +3,8 @@
 // headers (make_lane_header) and its payload by 32-bit shared-memory addresses.
 // The arithmetic is that of gw_dials.cuh; what differs is the index work around
 // it, which is most of a warp's instructions (64 points, warp instructions per
-// dial with the generic dial_values and now: grid dial 67 -> 50, general spline
-// 229 -> 193, graph 205 -> 140, bilinear surface 266 -> 217).
+// dial with the generic dial_values and now: grid dial 67 -> 47, general spline
+// 229 -> 197, graph 205 -> 144, bilinear surface 266 -> 222, norm 56 -> 26).
 #pragma once
 #include "gw_device.cuh"
 
