@@ -16,6 +16,7 @@
 // The reference needs ~1 + n_types + 2*(2 + log2 max bin occupancy) launches
 // for the same work (CacheWeights.cpp:153-183, CacheRecursiveSums.cpp:282-352).
 #include <algorithm>
+#include <mutex>
 
 #include "gw.h"
 #include "gw_device.cuh"
@@ -841,25 +842,23 @@ static const void* pick_plain(const DevView& v) {
   return v.precision ? plain_fn<float>(v.plain_kind) : plain_fn<double>(v.plain_kind);
 }
 
-// Raises the kernel's limit of dynamic shared memory on the current device to all
-// that a block may have there.  The limit is the kernel's, not an engine's: set to
-// the need of the engine built last, it would refuse the launches of an earlier
-// one with larger tiles or more parameters.
-static cudaError_t open_shared(const void* fn) {
-  int dev = 0, optin = 0;
+// Raises the kernel's limit of dynamic shared memory on the current device to
+// `smem`, and never lowers it: the limit is the kernel's, not an engine's, and set to
+// the need of the engine built last it would refuse the launches of an earlier one
+// with larger tiles or more parameters.
+static cudaError_t open_shared(const void* fn, size_t smem) {
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
   cudaFuncAttributes a;
-  cudaError_t r = cudaGetDevice(&dev);
-  if (r == cudaSuccess) r = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (r == cudaSuccess) r = cudaFuncGetAttributes(&a, fn);
-  if (r == cudaSuccess)
-    r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes);
-  return r;
+  const cudaError_t r = cudaFuncGetAttributes(&a, fn);
+  if (r != cudaSuccess || (size_t)a.maxDynamicSharedSizeBytes >= smem) return r;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
 // Resident blocks per SM, 0 when the kernel cannot run with that much shared memory.
 static int blocks_per_sm(const void* fn, int threads, size_t smem) {
   int n = 0;
-  if (open_shared(fn) != cudaSuccess ||
+  if (open_shared(fn, smem) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;
@@ -884,7 +883,8 @@ size_t params_smem_bytes(const DevView& v) { return (size_t)v.n_params * sizeof(
 cudaError_t prepare_params(const DevView& v) {
   return open_shared(v.precision == 2 ? (const void*)k_params<dfloat>
                      : v.precision   ? (const void*)k_params<float>
-                                     : (const void*)k_params<double>);
+                                     : (const void*)k_params<double>,
+                     params_smem_bytes(v));
 }
 
 cudaError_t launch_params(const DevView& v, const double* params, int K, cudaStream_t s) {

@@ -288,14 +288,10 @@ __device__ __forceinline__ void parameter_values(const DevView& v, uint32_t h, u
 // The clamped responses of the dials that the kernel has no shorter path for (h,
 // hy: the header's two words; pl, base: the tile's payload; g: a grid dial's
 // points, when `have_grid`).  A clamp that is not the common one is loaded before the
-// response is formed: one tile per SM and one point per lane is a chain of
-// latencies (7200 tabulated dials 28 -> 21 us, splines on grids 13.9 -> 12.5).  Two
-// 8-byte points per lane are short of registers and load it after (200k events in
-// FP64, 64 points: 1.74 against 1.76 ms).
-template <typename T, int KR, bool have_grid>
+// response is formed (kEarly) or after it, see k_batched.
+template <typename T, int KR, bool have_grid, bool kEarly>
 __device__ __forceinline__ void other_values(const DevView& v, uint32_t h, uint32_t hy, uint32_t pl, const T* base,
                                              int k0, int kstep, GridPoints<T, KR>& g, T (&val)[KR]) {
-  constexpr bool kEarly = sizeof(T) == 4 || KR == 1;
   using V2 = typename Vec2<T>::type;
   const int type = lhdr_type(h);
   const uint32_t da = pl + lhdr_off(h), q = hy & 0xFFFFu;

@@ -135,6 +135,15 @@ __global__ void __launch_bounds__(NT, MB) k_batched(const DevView v, int K) {
           // 9.79 ms); with two points per lane the extra live registers cost
           // more than the hidden latency (K = 64 on 1M: 1.18 against 1.11 ms)
           constexpr bool kAhead = KR >= 4;
+          // With one point per lane and few tiles a dial is a chain of latencies, so a
+          // clamp of its own is loaded before the response is formed (7200 tabulated
+          // dials at 32 points 28 -> 21 us, splines on grids 13.9 -> 12.5), as it is
+          // at four FP32 points per lane (300k events, K = 100: 871 -> 845 us) and in
+          // the 64-register shape (1M events, K = 64: 1.08 -> 1.06 ms); the other
+          // shapes have the registers for more in flight without it (100k events, K =
+          // 64, 128 threads: 67.8 us against 72.8; FP64, 200k events: 1.74 ms against
+          // 1.76).
+          constexpr bool kEarly = KR == 1 || (sizeof(T) == 4 && (KR >= 4 || MB == 4));
           uint2 hn = make_uint2(0u, 0u);
           GridPoints<T, KR> gn;
           if (kAhead && h0 < h1) {
@@ -164,7 +173,7 @@ __global__ void __launch_bounds__(NT, MB) k_batched(const DevView v, int K) {
 #pragma unroll
               for (int j = 0; j < KR; ++j) val[j] = clamp_response(val[j], T(0.0f), open_bound<T>());
             } else {
-              other_values<T, KR, kAhead>(v, h.x, h.y, pl, (const T*)stage, k0, KC, g, val);
+              other_values<T, KR, kAhead, kEarly>(v, h.x, h.y, pl, (const T*)stage, k0, KC, g, val);
             }
 #pragma unroll
             for (int j = 0; j < KR; ++j) w[j] *= val[j];

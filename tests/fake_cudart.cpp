@@ -137,9 +137,12 @@ cudaError_t cudaFuncSetAttribute(const void* fn, cudaFuncAttribute a, int v) {
   }
   return cudaSuccess;
 }
-cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void*) {
+cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void* fn) {
+  std::lock_guard<std::recursive_mutex> g(mu);
+  const auto it = limits.find({device, fn});
   memset(a, 0, sizeof *a);
   a->sharedSizeBytes = kStatic;
+  a->maxDynamicSharedSizeBytes = it == limits.end() ? 48 * 1024 : it->second;
   return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int, size_t smem) {
